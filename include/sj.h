@@ -287,7 +287,8 @@ int sj_synchronize(sj_sim* sim);
    march z segments of zseg in {8, 16, 32} planes (tile_y, ring ignored).
    TMA: tiles of 32 x tile_y cells, a TMA ring of `ring` planes
    ((tile_y, ring) in {(4,3), (8,3), (16,3), (4,4), (8,4)}), z segments of
-   zseg planes.  Applies to the schedule selected when it is called. */
+   zseg planes.  Applies to the schedule selected when it is called.  FUSED
+   steps with the tile kernels from then on, on small grids too. */
 int sj_set_tiling(sj_sim* sim, int32_t tile_y, int32_t ring, int32_t zseg);
 int sj_get_tiling(const sj_sim* sim, int32_t* tile_y, int32_t* ring, int32_t* zseg);
 /* FUSED: columns per thread in the tile kernels.  0 (default) = two where
@@ -316,10 +317,14 @@ int sj_autotune(sj_sim* sim, int32_t steps, int32_t* tile_y, int32_t* ring, int3
 /* ---------------------------------------------------------------- stepping */
 /* n_steps iterations of the loop body at src/disp.cpp:719-741: sample
    monitors when step % save_span == 0, accumulate DFTs, then fields.step().
-   Asynchronous on the sim's stream. */
+   Asynchronous on the sim's stream.  FUSED with its default launch settings
+   and without design regions: on small grids (all instances together at most
+   2^23 cells in FP32, 2^25 in FP64) a call of two or more steps is one
+   cooperative launch per 256 steps, with the tile launches' bits. */
 int sj_step(sj_sim* sim, int64_t n_steps);
 
-/* same, recorded once into a CUDA graph of `chunk` steps and replayed */
+/* same, recorded once into a CUDA graph of `chunk` steps and replayed (small
+   grids: as sj_step) */
 int sj_step_graph(sj_sim* sim, int64_t n_steps, int32_t chunk);
 
 /* ---------------------------------------------------------------- queries */
@@ -337,8 +342,9 @@ int sj_transfer_bytes(const sj_sim* sim, int64_t* h2d, int64_t* d2h);
 /* per-instance voxel count and algorithmic bytes per step (roofline model) */
 int64_t sj_voxels(const sj_sim* sim, int32_t inst);
 double sj_bytes_per_step(const sj_sim* sim, int32_t inst);
-/* kernel launches one sj_step step issues under the current schedule (GB300
-   query; the reference has no counterpart) */
+/* kernel launches a single step issues under the current schedule (GB300
+   query; the reference has no counterpart; runs of steps on small grids issue
+   fewer) */
 int32_t sj_launches_per_step(const sj_sim* sim);
 
 /* ---------------------------------------------------------------- read-back */

@@ -12,7 +12,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libsj_gb300.so")
 OBJ = os.path.join(HERE, "_build")
-SOURCES = ["sj_host.cu", "sj_step.cu", "sj_lean.cu", "sj_fused.cu", "sj_raster.cu", "sj_adjoint.cu", "sj_spectrum.cu",
+SOURCES = ["sj_host.cu", "sj_step.cu", "sj_lean.cu", "sj_resident.cu", "sj_fused.cu", "sj_raster.cu", "sj_adjoint.cu", "sj_spectrum.cu",
            "sj_diag.cu", "sj_phases.cu"]
 HEADERS = ["sj_internal.h", "sj_physics.cuh", os.path.join("..", "..", "include", "sj.h")]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -20,7 +20,7 @@ FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxe
 # the fused stepper writes every fused multiply-add explicitly (results must
 # not depend on which of its kernels updated a voxel); host tables and the
 # smoothing offsets are computed without contraction on every host CPU
-FILE_FLAGS = {"sj_lean.cu": ["-fmad=false"], "sj_host.cu": ["-Xcompiler", "-ffp-contract=off"]}
+FILE_FLAGS = {"sj_lean.cu": ["-fmad=false"], "sj_resident.cu": ["-fmad=false"], "sj_host.cu": ["-Xcompiler", "-ffp-contract=off"]}
 
 
 def _nvcc():

@@ -189,6 +189,10 @@ struct sj_sim {
     long long q_version = -1;          // table_version the queue tables were built from
     long long lists_version = 0;       // bumped whenever prepare_lean rebuilds the tile lists
     long long q_lists = -1;            // lists_version the queue items were built from
+    // small grids: runs of steps in one cooperative launch (sj_resident.cu)
+    int r_blocks = -1;                 // resident blocks the device holds (-1: not asked yet, 0: cannot run)
+    bool tiles_asked = false;          // a tile-kernel setting was made by the caller
+    unsigned* d_bar = nullptr;         // the grid barrier's counter
     // dump_raw snapshots (per instance) and the stream their host copies run on
     std::vector<Snapshots> snaps;
     cudaStream_t copy_stream = nullptr;
@@ -763,6 +767,7 @@ void build_instance(sj_sim* sim, const sj_instance_desc& d, HostInst<real>& H, I
         const sj_probe_desc& pd = d.probes[p];
         if (pd.component < 0 || pd.component > 5) fail(SJ_E_INVALID, "probe component out of range");
         pcomp[p] = pd.component;
+        I.n_hprobe += pd.component >= 3;
         if (pd.flags & SJ_PROBE_MONITOR) pmon[p] = H.n_mon++;
         if (pd.flags & SJ_PROBE_DFT) {
             pdft[p] = H.n_dft++;
@@ -1330,22 +1335,72 @@ void take_snapshot_async(sj_sim* sim, int q) {
     sim->d2h += (long long)(row * H.ny * H.nz);
 }
 
+// Most cells (all instances) that run through the resident kernel.  Measured,
+// us per step, resident against tile launches (zseg 16): FP32 64^3 9.1 / 72,
+// 128^3 44 / 119, 192^3 157 / 184, 4 x 128^3 (2^23) 208 / 244, 256 x 256 x
+// 192 272 / 254 (the two-pass traffic leaves L2); FP64, whose bound is the
+// FP64 pipe and which gains from the missing halo work, 64^3 27 / 124, 192^3
+// 540 / 684, 256 x 256 x 192 879 / 1005, 384 x 384 x 288 (42M) 2936 / 2956.
+template <typename real>
+constexpr long long res_max_voxels() { return sizeof(real) == 4 ? 1LL << 23 : 1LL << 25; }
+constexpr int RES_CHUNK = 256;                                // steps per launch
+constexpr unsigned long long RES_WAIT_NS = 4000000000ull;     // limit of a wait at the grid barrier
+
+// Do runs of steps go through the resident kernel?
+template <typename real>
+bool resident(sj_sim* sim) {
+    if (sim->schedule != SJ_SCHED_FUSED || sim->tiles_asked || sim->l_one_column || sim->l_launch != SJ_LAUNCH_GROUPED ||
+        sim->n_inst > RES_MAX_INST || sim->r_blocks == 0)
+        return false;
+    long long cells = 0;
+    for (const InstDev<real>& I : devv<real>(sim)) {
+        if (I.dinv || 2 * I.vol >= (1LL << 32)) return false;
+        cells += (long long)I.nx * I.ny * I.nz;
+    }
+    if (cells > res_max_voxels<real>()) return false;
+    if (sim->r_blocks < 0) {
+        sim->r_blocks = resident_grid<real>(sim->n_inst);
+        if (sim->r_blocks > 0) sim->d_bar = (unsigned*)sim->dalloc(sizeof(unsigned));
+    }
+    return sim->r_blocks > 0;
+}
+
+// n steps with no save point inside: one cooperative launch per RES_CHUNK
+// steps on small grids, else a step's launches n times
+template <typename real>
+void run_steps(sj_sim* sim, long long n) {
+    if (n >= 2 && resident<real>(sim)) {
+        const InstDev<real>* d = reinterpret_cast<const InstDev<real>*>(sim->d_table);
+        while (n > 0) {
+            const int m = (int)std::min<long long>(n, RES_CHUNK);
+            ck(launch_resident<real>(devv<real>(sim).data(), d, sim->n_inst, sim->cur, m, sim->r_blocks, sim->d_bar,
+                                     RES_WAIT_NS, sim->d_state, sim->stream),
+               "resident launch");
+            sim->t += m;
+            n -= m;
+        }
+        return;
+    }
+    for (; n > 0; --n) {
+        ck(launch_one<real>(sim), "step launch");
+        sim->t += 1;
+    }
+}
+
 template <typename real>
 void do_steps(sj_sim* sim, long long n) {
     ensure_capacity<real>(sim, sim->t + n);
-    if (!sim->any_snapshots()) {
-        for (long long q = 0; q < n; ++q) ck(launch_one<real>(sim), "step launch");
-        sim->t += n;
-        return;
-    }
-    // with snapshots: step by step, the counter current at every save point
-    for (long long q = 0; q < n; ++q) {
+    while (n > 0) {
+        // up to the next save point, the counter current there
+        long long m = n;
         for (int i = 0; i < sim->n_inst; ++i) {
             const Snapshots& S = sim->snaps[i];
-            if (S.every > 0 && sim->t % S.every == 0) take_snapshot_async<real>(sim, i);
+            if (S.every <= 0) continue;
+            if (sim->t % S.every == 0) take_snapshot_async<real>(sim, i);
+            m = std::min<long long>(m, S.every - sim->t % S.every);
         }
-        ck(launch_one<real>(sim), "step launch");
-        sim->t += 1;
+        run_steps<real>(sim, m);
+        n -= m;
     }
 }
 
@@ -1356,6 +1411,7 @@ template <typename real>
 void do_steps_graph(sj_sim* sim, long long n, int chunk) {
     if (chunk < 1) fail(SJ_E_INVALID, "chunk must be >= 1");
     if (sim->any_snapshots()) return do_steps<real>(sim, n);  // save points fall inside chunks
+    if (resident<real>(sim)) return do_steps<real>(sim, n);   // one launch per run of steps already
     ensure_capacity<real>(sim, sim->t + n);
     // everything that allocates or copies happens before the capture
     prepare_schedule<real>(sim);
@@ -1991,6 +2047,7 @@ int sj_set_tiling(sj_sim* sim, int32_t tile_y, int32_t ring, int32_t zseg) {
         if (zseg != 8 && zseg != 16 && zseg != 32)
             return finish(sim, SJ_E_INVALID, "fused schedule: zseg must be 8, 16 or 32");
         sim->l_zb = zseg;
+        sim->tiles_asked = true;
         sim->drop_graphs();
         return SJ_OK;
     }

@@ -74,6 +74,7 @@ struct InstDev {
 
     // probes (monitors and DFT points)
     int n_probe, n_mon, n_dft, n_freq, save_span;
+    int n_hprobe;               // probes of H components
     const int* probe_comp;      // [n_probe]
     const long long* probe_idx; // [n_probe][8] element offsets, -1 = outside
     const double* probe_w;      // [n_probe][8]
@@ -230,6 +231,17 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
                              int n_groups, const LeanGen& gen, const LeanFix& fix, int n_inst, int zb, int dry,
                              int cur, DevState* st, const LeanStreams& ls, int one_column = 0,
                              const LeanQueue<real>* queue = nullptr);
+// Small grids (sj_resident.cu): n_steps steps in one cooperative launch of at
+// most max_blocks resident blocks, in place in buffer `cur`.  resident_grid:
+// the blocks of the kernel that fit the device at once (0: it cannot run).
+// d_bar: the barrier's counter, zeroed by the launch.
+constexpr int RES_MAX_INST = 32;  // instances of one resident launch
+template <typename real>
+int resident_grid(int n_inst);
+template <typename real>
+cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d_insts, int n_inst, int cur,
+                            int n_steps, int max_blocks, unsigned* d_bar, unsigned long long limit_ns, DevState* st,
+                            cudaStream_t s);
 template <typename real>
 int fused_box_width();          // TMA box width in elements (x)
 template <typename real>

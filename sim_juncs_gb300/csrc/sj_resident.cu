@@ -1,0 +1,617 @@
+// Small grids: many steps of the fused schedule in one cooperative launch.
+//
+// A 64^3 step is 262k cells, a few microseconds of work from L2, but as tile
+// launches it costs ten launches on forked streams, and its 64 tiles of 16
+// planes are a serial march on 64 of the 152 SMs.  Here a grid of resident
+// blocks (one per SM) runs a whole run of steps: per step an H phase
+// and an E phase over every cell of every instance, in place, with a grid
+// barrier after each.  In the E phase a cell's sources and polarisations
+// follow its curl directly (they are separate passes after the tile kernels).
+// The cell's arithmetic is the tile kernels', operation for operation, so
+// the bits are theirs (this file too is compiled with contraction off).
+//
+// FP32 is bound by latency up to about 64^3 (36^3 8.5 us per step, 64^3 9.1: two
+// L2 round trips and two barriers; 72 us as tile launches) and by L2 above.
+// FP64 is bound by the FP64 pipe (19 cycles per warp instruction and SM):
+// 64^3 27 us per step (124 as tile launches), of which 17 are its 35 FP64
+// operations per cell.
+//
+// Cells are dealt out by their linear index over nx*ny*nz, so odd rows leave
+// no idle lanes.  Probes have blocks of their own: E probes of step n are
+// read during its H phase, which does not write E, and H probes of step n
+// (H^{n-1/2}) during the E phase of step n-1, which does not write H.
+#include <algorithm>
+
+#include "sj_physics.cuh"
+
+namespace sj {
+
+namespace {
+
+constexpr int RES_MAXF = 256;
+#ifndef SJ_RES_THREADS32
+#define SJ_RES_THREADS32 1024
+#endif
+#ifndef SJ_RES_CHUNK32
+#define SJ_RES_CHUNK32 1024
+#endif
+#ifndef SJ_RES_CHUNK64
+#define SJ_RES_CHUNK64 32
+#endif
+
+// FP32: 1024 threads of 64 registers hide latency better than 512 of 96
+// (96^3 18.4 us per step against 23.7; 36^3 8.6 against 9.7 is the price)
+template <typename real>
+constexpr int res_threads() { return sizeof(real) == 4 ? SJ_RES_THREADS32 : 512; }
+
+// A block takes its cells in chunks of this many consecutive ones, dealt out
+// over the blocks in turn.  FP64 is bound by the FP64 pipe of each SM, so its
+// chunks are one warp's (the SMs' shares differ by one: 64^3 27.3 us per step,
+// 29.9 with 256); FP32's are the block's, whose rows share L1 lines.
+template <typename real>
+constexpr int res_chunk() { return sizeof(real) == 4 ? SJ_RES_CHUNK32 : SJ_RES_CHUNK64; }
+
+// q = t / d for t < 2^31 by multiplication (Granlund and Montgomery, "Division
+// by invariant integers using multiplication", 1994)
+struct Div {
+    unsigned d, m, s;
+    __device__ __forceinline__ void set(unsigned dd) {
+        d = dd;
+        s = dd > 1 ? 32 - __clz(dd - 1) : 0;
+        m = (unsigned)((((1ull << 32) * ((1ull << s) - dd)) / dd) + 1);
+    }
+    __device__ __forceinline__ unsigned div(unsigned t) const { return (__umulhi(t, m) + t) >> s; }
+};
+
+// What a block knows of one instance besides its descriptor.  FP64 deals the
+// columns between the x slabs first and the slabs' columns after them: a
+// warp then seldom mixes the two, and only the slabs' warps pay for the x
+// terms (all warps of a 64-cell row would).
+struct ResGrid {
+    Div dx, dxs, dy;             // columns between the x slabs (FP32: all), columns of the slabs, rows
+    unsigned inner, cells;       // cells of the former, of all
+    unsigned start;              // this block's first cell
+    int lo;                      // first column between the slabs
+    int hsrc, esrc;              // any H / E source
+};
+
+struct Cell {
+    int i, j, k;
+};
+template <typename real>
+__device__ __forceinline__ Cell res_cell(const ResGrid& G, unsigned t) {
+    Cell c;
+    if (sizeof(real) == 4) {
+        const unsigned q = G.dx.div(t), kk = G.dy.div(q);
+        c.i = (int)(t - q * G.dx.d), c.j = (int)(q - kk * G.dy.d), c.k = (int)kk;
+        return c;
+    }
+    const bool in = t < G.inner;
+    const Div& D = in ? G.dx : G.dxs;
+    t -= in ? 0u : G.inner;
+    const unsigned q = D.div(t), kk = G.dy.div(q);
+    c.i = (int)(t - q * D.d), c.j = (int)(q - kk * G.dy.d), c.k = (int)kk;
+    c.i += in ? G.lo : (c.i >= G.lo ? (int)G.dx.d : 0);
+    return c;
+}
+
+// Grid barrier: every block arrives with release, waits for `target`
+// arrivals with acquire.  A wait that does not end within `limit` ns records
+// SJ_E_TIMEOUT and ends the launch (false, block-uniform).
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, unsigned long long limit, DevState* st) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ok = 1;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        unsigned long long t0 = 0;
+        for (unsigned spin = 0;; ++spin) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if (v >= target) break;
+            if ((spin & 1023u) == 1023u) {
+                unsigned long long t;
+                asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+                if (!t0) t0 = t;
+                if (t - t0 > limit) {
+                    st->status = SJ_E_TIMEOUT;
+                    ok = 0;
+                    break;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// Does this lane run the terms of an axis its cell lies (on) or not in the
+// slab of?  FP64: when some lane of the warp does, by select (a branch per
+// lane has the compiler emit the common FP64 work once for each side).
+template <typename real>
+__device__ __forceinline__ bool res_any(bool on) {
+    return sizeof(real) == 8 ? __any_sync(__activemask(), on) : on;
+}
+
+// One CPML term: psi = fma(b, psi, c d), added to or subtracted from the curl
+// where the cell is in the slab; any: some lane of the warp is
+template <bool ADD, typename real>
+__device__ __forceinline__ void res_term(real& cv, bool any, bool on, real b, real c, real d, real po, real* p) {
+    if (!any) return;
+    const real ps = fma(b, po, c * d);
+    if (on) *p = ps;
+    cv = ADD ? cv + (on ? ps : real(-0.0)) : cv - (on ? ps : real(0));
+}
+
+template <typename real>
+__device__ __forceinline__ bool src_hit(const SrcDev<real>& s, int i, int j, int k) {
+    return (unsigned)(i - s.lo[0]) < (unsigned)s.n[0] && (unsigned)(j - s.lo[1]) < (unsigned)s.n[1] &&
+           (unsigned)(k - s.lo[2]) < (unsigned)s.n[2];
+}
+
+// dt J of the H sources of component comp at the cell
+template <typename real>
+__device__ __forceinline__ real res_hsrc(const InstDev<real>& I, int comp, int i, int j, int k, long long n, real h) {
+    real acc = 0;
+    bool hit = false;
+    for (int s = 0; s < I.n_src; ++s) {
+        const SrcDev<real>& v = I.src[s];
+        if (v.comp != comp || !src_hit(v, i, j, k)) continue;
+        acc += (real)v.tab[n] * v.w[0][i - v.lo[0]] * v.w[1][j - v.lo[1]] * v.w[2][k - v.lo[2]];
+        hit = true;
+    }
+    return hit ? h - acc : h;
+}
+
+// H^{n+1/2} of one cell, in place
+template <typename real>
+__device__ __forceinline__ void res_h(const InstDev<real>& I, const ResGrid& G, int cur, unsigned t, long long n) {
+    const Cell c3 = res_cell<real>(G, t);
+    const int i = c3.i, j = c3.j, k = c3.k;
+    const int nx = I.nx, ny = I.ny, nz = I.nz;
+    const unsigned px = (unsigned)I.px, plane = (unsigned)I.plane, vol = (unsigned)I.vol;
+    const unsigned o = (unsigned)k * plane + (unsigned)j * px + (unsigned)i;
+    const real* eX = I.F[cur][0];
+    const real* eY = I.F[cur][1];
+    const real* eZ = I.F[cur][2];
+    real* const hX = I.F[cur][3] + o;
+    real* const hY = I.F[cur][4] + o;
+    real* const hZ = I.F[cur][5] + o;
+    const bool xp = i + 1 < nx, yp = j + 1 < ny, zp = k + 1 < nz;
+    const bool xo = in_slab(I, 0, i), yo = in_slab(I, 1, j), zo = in_slab(I, 2, k);
+    const real ex = eX[o], ey = eY[o], ez = eZ[o];
+    const real ex_y = yp ? eX[o + px] : real(0), ex_z = zp ? eX[o + plane] : real(0);
+    const real ey_x = xp ? eY[o + 1] : real(0), ey_z = zp ? eY[o + plane] : real(0);
+    const real ez_x = xp ? eZ[o + 1] : real(0), ez_y = yp ? eZ[o + px] : real(0);
+    const real hx0 = *hX, hy0 = *hY, hz0 = *hZ;
+    const bool ax = res_any<real>(xo), ay = res_any<real>(yo), az = res_any<real>(zo);
+    real *pX = nullptr, *pY = nullptr, *pZ = nullptr;
+    real qx0 = 0, qx1 = 0, qy0 = 0, qy1 = 0, qz0 = 0, qz1 = 0;
+    real bx = 1, cx = 0, by = 1, cy = 0, bz = 1, cz = 0;
+    if (xo) {
+        pX = I.psiH[cur][0] + o;
+        qx0 = pX[0], qx1 = pX[vol];
+        bx = __ldg(I.prof[0] + 2 * nx + i), cx = __ldg(I.prof[0] + 3 * nx + i);
+    }
+    if (yo) {
+        pY = I.psiH[cur][1] + o;
+        qy0 = pY[0], qy1 = pY[vol];
+        by = __ldg(I.prof[1] + 2 * ny + j), cy = __ldg(I.prof[1] + 3 * ny + j);
+    }
+    if (zo) {
+        pZ = I.psiH[cur][2] + o;
+        qz0 = pZ[0], qz1 = pZ[vol];
+        bz = __ldg(I.prof[2] + 2 * nz + k), cz = __ldg(I.prof[2] + 3 * nz + k);
+    }
+    real hx, hy, hz;
+    {
+        const real d1 = ez_y - ez, d2 = ey_z - ey;
+        real cv = d1 - d2;
+        res_term<true>(cv, ay, yo, by, cy, d1, qy0, pY);
+        res_term<false>(cv, az, zo, bz, cz, d2, qz0, pZ);
+        hx = fma(-I.S, cv, hx0);
+    }
+    {
+        const real d1 = ex_z - ex, d2 = ez_x - ez;
+        real cv = d1 - d2;
+        res_term<true>(cv, az, zo, bz, cz, d1, qz1, pZ + vol);
+        res_term<false>(cv, ax, xo, bx, cx, d2, qx0, pX);
+        hy = fma(-I.S, cv, hy0);
+    }
+    {
+        const real d1 = ey_x - ey, d2 = ex_y - ex;
+        real cv = d1 - d2;
+        res_term<true>(cv, ax, xo, bx, cx, d1, qx1, pX + vol);
+        res_term<false>(cv, ay, yo, by, cy, d2, qy1, pY + vol);
+        hz = fma(-I.S, cv, hz0);
+    }
+    if (G.hsrc) {
+        hx = res_hsrc(I, 3, i, j, k, n, hx);
+        hy = res_hsrc(I, 4, i, j, k, n, hy);
+        hz = res_hsrc(I, 5, i, j, k, n, hz);
+    }
+    *hX = hx;
+    *hY = hy;
+    *hZ = hz;
+}
+
+// E^{n+1} of one cell, in place: curl, then the E sources in order, then the
+// polarisations of the cell's material
+template <typename real>
+__device__ __forceinline__ void res_e(const InstDev<real>& I, const ResGrid& G, int cur, unsigned t, long long n) {
+    const Cell c3 = res_cell<real>(G, t);
+    const int i = c3.i, j = c3.j, k = c3.k;
+    const int nx = I.nx, ny = I.ny, nz = I.nz;
+    const unsigned px = (unsigned)I.px, plane = (unsigned)I.plane, vol = (unsigned)I.vol;
+    const unsigned o = (unsigned)k * plane + (unsigned)j * px + (unsigned)i;
+    const real* hX = I.F[cur][3];
+    const real* hY = I.F[cur][4];
+    const real* hZ = I.F[cur][5];
+    const int cb = __ldg(I.combo + o);
+    const unsigned mask = __ldg(I.pmask + cb);
+    const real* cf = I.coef + cb * I.ncoef;
+    const real* sv = cf + I.ncoef - 3;
+    const bool xm = i > 0, ym = j > 0, zm = k > 0;
+    const bool xo = in_slab(I, 0, i), yo = in_slab(I, 1, j), zo = in_slab(I, 2, k);
+    const real hx = hX[o], hy = hY[o], hz = hZ[o];
+    const real hx_y = ym ? hX[o - px] : real(0), hx_z = zm ? hX[o - plane] : real(0);
+    const real hy_x = xm ? hY[o - 1] : real(0), hy_z = zm ? hY[o - plane] : real(0);
+    const real hz_x = xm ? hZ[o - 1] : real(0), hz_y = ym ? hZ[o - px] : real(0);
+    real* const E[3] = {I.F[cur][0] + o, I.F[cur][1] + o, I.F[cur][2] + o};
+    const real e0[3] = {*E[0], *E[1], *E[2]};
+    const bool ax = res_any<real>(xo), ay = res_any<real>(yo), az = res_any<real>(zo);
+    real *pX = nullptr, *pY = nullptr, *pZ = nullptr;
+    real qx0 = 0, qx1 = 0, qy0 = 0, qy1 = 0, qz0 = 0, qz1 = 0;
+    real bx = 1, cx = 0, by = 1, cy = 0, bz = 1, cz = 0;
+    if (xo) {
+        pX = I.psiE[0] + o;
+        qx0 = pX[0], qx1 = pX[vol];
+        bx = __ldg(I.prof[0] + i), cx = __ldg(I.prof[0] + nx + i);
+    }
+    if (yo) {
+        pY = I.psiE[1] + o;
+        qy0 = pY[0], qy1 = pY[vol];
+        by = __ldg(I.prof[1] + j), cy = __ldg(I.prof[1] + ny + j);
+    }
+    if (zo) {
+        pZ = I.psiE[2] + o;
+        qz0 = pZ[0], qz1 = pZ[vol];
+        bz = __ldg(I.prof[2] + k), cz = __ldg(I.prof[2] + nz + k);
+    }
+    real e[3];
+    {
+        const real d1 = hz - hz_y, d2 = hy - hy_z;
+        real cv = d1 - d2;
+        res_term<true>(cv, ay, yo, by, cy, d1, qy0, pY);
+        res_term<false>(cv, az, zo, bz, cz, d2, qz0, pZ);
+        e[0] = fma(__ldg(sv), cv, e0[0]);
+    }
+    {
+        const real d1 = hx - hx_z, d2 = hz - hz_x;
+        real cv = d1 - d2;
+        res_term<true>(cv, az, zo, bz, cz, d1, qz1, pZ + vol);
+        res_term<false>(cv, ax, xo, bx, cx, d2, qx0, pX);
+        e[1] = fma(__ldg(sv + 1), cv, e0[1]);
+    }
+    {
+        const real d1 = hy - hy_x, d2 = hx - hx_y;
+        real cv = d1 - d2;
+        res_term<true>(cv, ax, xo, bx, cx, d1, qx1, pX + vol);
+        res_term<false>(cv, ay, yo, by, cy, d2, qy1, pY + vol);
+        e[2] = fma(__ldg(sv + 2), cv, e0[2]);
+    }
+    if (G.esrc)
+        for (int s = 0; s < I.n_src; ++s) {
+            const SrcDev<real>& v = I.src[s];
+            if (v.comp >= 3 || !src_hit(v, i, j, k)) continue;
+            const real J = (real)v.tab[n] * v.w[0][i - v.lo[0]] * v.w[1][j - v.lo[1]] * v.w[2][k - v.lo[2]];
+            const real c = __ldg(cf + v.comp);
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                if (a == v.comp) e[a] = fma(-c, J, e[a]);
+        }
+    if (mask) {
+        const unsigned u = ((unsigned)(k - I.dlo[2]) * (unsigned)I.dn[1] + (unsigned)(j - I.dlo[1])) *
+                               (unsigned)I.dn[0] + (unsigned)(i - I.dlo[0]);
+        const long long lv = 3 * I.dvol;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const unsigned mc = (mask >> (8 * c)) & 255u;
+            if (!mc) continue;
+            real corr = 0;
+            for (unsigned m = mc; m; m &= m - 1) {
+                const int p = __ffs(m) - 1;
+                real* pp = I.P + ((long long)p * 6 + c) * I.dvol + u;
+                const real pn = *pp, pq = pp[lv];
+                const real pnew = I.A[p] * pn + I.B[p] * pq + __ldg(cf + 3 + 3 * p + c) * e0[c];
+                corr += pnew - pn;
+                pp[lv] = pn;
+                *pp = pnew;
+            }
+            e[c] = fma(-__ldg(cf + c), corr, e[c]);
+        }
+    }
+    *E[0] = e[0];
+    *E[1] = e[1];
+    *E[2] = e[2];
+}
+
+// dt e^{i 2 pi f t} of every DFT frequency for the E (h = 0) or H (h = 1)
+// probes of step n
+template <typename real>
+__device__ __forceinline__ void res_phases(const InstDev<real>& I, long long n, int h, double2* ph) {
+    const double tt = h ? ((double)n - 0.5) * I.dt : (double)n * I.dt;
+    for (int f = threadIdx.x; f < I.n_freq; f += blockDim.x) {
+        double s, c;
+        sincospi(2.0 * I.freqs[f] * tt, &s, &c);
+        ph[f] = make_double2(c * I.dt, s * I.dt);
+    }
+}
+
+// What a thread keeps of a probe through a run of steps.
+template <typename real>
+struct Probe {
+    const real* F[8];   // stencil points, null outside the grid
+    double w[8];
+    double2* row;       // DFT sums, null without
+    int comp, mon;
+};
+template <typename real>
+__device__ __forceinline__ Probe<real> res_probe(const InstDev<real>& I, int cur, int p) {
+    Probe<real> r;
+    r.comp = I.probe_comp[p];
+    r.mon = I.probe_mon[p];
+    const int ds = I.probe_dft[p];
+    r.row = ds >= 0 ? I.dft + (long long)ds * I.n_freq : nullptr;
+    const real* F = I.F[cur][r.comp];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        const long long idx = I.probe_idx[8 * p + m];
+        r.F[m] = idx >= 0 ? F + idx : nullptr;
+        r.w[m] = I.probe_w[8 * p + m];
+    }
+    return r;
+}
+
+// Sample a probe at step n: its monitor value (at save points) and its DFT
+// sums, as the tile path's probe blocks form them.
+template <typename real>
+__device__ __forceinline__ void res_sample(const InstDev<real>& I, const Probe<real>& r, long long n, bool save,
+                                           int n_freq, DevState* st, const double2* ph) {
+    const bool mon = r.mon >= 0 && save;
+    if (!mon && !r.row) return;
+    double2 a[4];
+    if (r.row)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (u < n_freq) a[u] = r.row[u];
+    double v = 0.0;
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+        if (r.F[m]) v += r.w[m] * (double)*r.F[m];
+    if (mon) monitor_store(I, n, r.mon, v, st);
+    if (!r.row) return;
+    for (int f0 = 0; f0 < n_freq; f0 += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (f0 && f0 + u < n_freq) a[u] = r.row[f0 + u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (f0 + u < n_freq) {
+                a[u].x += v * ph[f0 + u].x;
+                a[u].y += v * ph[f0 + u].y;
+                r.row[f0 + u] = a[u];
+            }
+    }
+}
+
+// The E or H probes (h) of every instance at step n.  Block b of nb takes
+// every nb-th chunk of blockDim.x probes.
+template <typename real>
+__device__ __forceinline__ void res_probes(const InstDev<real>* tab, int n_inst, int cur, long long n, int h, int b,
+                                           int nb, DevState* st, double2* ph) {
+    int item = 0;
+    for (int q = 0; q < n_inst; ++q) {
+        const InstDev<real>& I = tab[q];
+        const bool save = n % I.save_span == 0;
+        const int chunks = (I.n_probe + (int)blockDim.x - 1) / (int)blockDim.x;
+        if (!chunks || (!save && !I.n_dft)) {
+            item += chunks;
+            continue;
+        }
+        bool have = false;
+        for (int c = 0; c < chunks; ++c, ++item) {
+            if (item % nb != b) continue;
+            if (!have && I.n_dft) {
+                __syncthreads();
+                res_phases(I, n, h, ph);
+                __syncthreads();
+            }
+            have = true;
+            const int p = c * blockDim.x + threadIdx.x;
+            if (p >= I.n_probe || (I.probe_comp[p] >= 3) != (h != 0)) continue;
+            res_sample(I, res_probe(I, cur, p), n, save, I.n_freq, st, ph);
+        }
+    }
+}
+
+// A probe block's run of steps.  one_chunk: every block has at most one
+// chunk, so a thread keeps its probe, and the phases of its next samples are
+// formed while the cells of the phase before are updated.
+template <typename real>
+__device__ __noinline__ void res_probe_block(const InstDev<real>* tab, int n_inst, int cur, long long n0, int n_steps,
+                                             int b, int nb, int h_probes, int one_chunk, unsigned* bar,
+                                             unsigned long long limit, DevState* st) {
+    __shared__ double2 ph[2][RES_MAXF];
+    unsigned target = 0;
+    if (!one_chunk) {
+        if (h_probes) {
+            res_probes<real>(tab, n_inst, cur, n0, 1, b, nb, st, ph[1]);
+            if (!grid_barrier(bar, target += gridDim.x, limit, st)) return;
+        }
+        for (int s = 0; s < n_steps; ++s) {
+            const bool more = s + 1 < n_steps;
+            res_probes<real>(tab, n_inst, cur, n0 + s, 0, b, nb, st, ph[0]);
+            if (!grid_barrier(bar, target += gridDim.x, limit, st)) return;
+            if (h_probes && more) res_probes<real>(tab, n_inst, cur, n0 + s + 1, 1, b, nb, st, ph[1]);
+            if (more && !grid_barrier(bar, target += gridDim.x, limit, st)) return;
+        }
+        return;
+    }
+    int item = 0, q = 0, chunk = 0;
+    for (; q < n_inst; ++q) {
+        const int chunks = (tab[q].n_probe + (int)blockDim.x - 1) / (int)blockDim.x;
+        chunk = b - item;
+        item += chunks;
+        if (b < item) break;
+    }
+    const InstDev<real>& I = tab[q];
+    const int p = chunk * (int)blockDim.x + (int)threadIdx.x, n_freq = I.n_freq;
+    Probe<real> r;
+    r.comp = -1;
+    if (p < I.n_probe) r = res_probe(I, cur, p);
+    const int kind = r.comp < 0 ? -1 : r.comp >= 3;  // 0: an E probe, 1: an H probe
+    const bool dft = I.n_dft > 0;
+    long long until = n0 % I.save_span;              // steps to the next save point
+    until = until ? I.save_span - until : 0;
+    if (dft) {
+        res_phases(I, n0, 0, ph[0]);
+        res_phases(I, n0, 1, ph[1]);
+    }
+    __syncthreads();
+    if (h_probes) {
+        if (kind == 1) res_sample(I, r, n0, until == 0, n_freq, st, ph[1]);
+        if (!grid_barrier(bar, target += gridDim.x, limit, st)) return;
+    }
+    for (int s = 0; s < n_steps; ++s) {
+        const long long n = n0 + s;
+        const bool more = s + 1 < n_steps;
+        if (kind == 0) res_sample(I, r, n, until == 0, n_freq, st, ph[0]);
+        until = until ? until - 1 : I.save_span - 1;
+        if (dft && h_probes) res_phases(I, n + 1, 1, ph[1]);
+        if (!grid_barrier(bar, target += gridDim.x, limit, st)) return;
+        if (dft) res_phases(I, n + 1, 0, ph[0]);
+        if (kind == 1 && more) res_sample(I, r, n + 1, until == 0, n_freq, st, ph[1]);
+        if (more && !grid_barrier(bar, target += gridDim.x, limit, st)) return;
+    }
+}
+
+// ONE: a single instance, its descriptor in the parameter space; else the
+// descriptors are copied to shared memory.  The fields' buffer `cur` is
+// stepped in place.
+template <typename real, bool ONE>
+__global__ void __launch_bounds__(res_threads<real>(), 1)
+k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __restrict__ tab, int n_inst, int cur,
+           int n_steps, int workers, int h_probes, int one_chunk, unsigned* bar, unsigned long long limit,
+           DevState* st) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ ResGrid grids[RES_MAX_INST];
+    constexpr unsigned CH = res_chunk<real>(), SLOTS = res_threads<real>() / CH;
+    const long long n0 = st->step;
+    if ((int)blockIdx.x >= workers) {
+        res_probe_block<real>(tab, n_inst, cur, n0, n_steps, (int)blockIdx.x - workers, (int)gridDim.x - workers,
+                              h_probes, one_chunk, bar, limit, st);
+        return;
+    }
+    InstDev<real>* sh = reinterpret_cast<InstDev<real>*>(smem);
+    if (!ONE) {
+        const int* s = reinterpret_cast<const int*>(tab);
+        int* d = reinterpret_cast<int*>(sh);
+        const int nw = n_inst * (int)(sizeof(InstDev<real>) / sizeof(int));
+        for (int w = threadIdx.x; w < nw; w += blockDim.x) d[w] = s[w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        unsigned first = 0;
+        for (int q = 0; q < n_inst; ++q) {
+            const InstDev<real>& I = ONE ? one : sh[q];
+            ResGrid& g = grids[q];
+            const unsigned rows = (unsigned)I.ny * (unsigned)I.nz;
+            const unsigned ws = sizeof(real) == 8 ? (unsigned)(I.pl[0] + I.ph[0]) : 0u;
+            g.dx.set(max(1u, (unsigned)I.nx - ws));
+            g.dxs.set(max(1u, ws));
+            g.dy.set((unsigned)I.ny);
+            g.inner = ((unsigned)I.nx - ws) * rows;
+            g.cells = (unsigned)I.nx * rows;
+            g.lo = ws ? I.pl[0] : 0;
+            // this block's first cell: chunks go to the blocks in turn, instance after instance
+            g.start = (blockIdx.x + (unsigned)workers - first) % (unsigned)workers * CH;
+            first = (first + (g.cells + CH - 1) / CH) % (unsigned)workers;
+            g.hsrc = g.esrc = 0;
+            for (int s = 0; s < I.n_src; ++s) (I.src[s].comp >= 3 ? g.hsrc : g.esrc) = 1;
+        }
+    }
+    __syncthreads();
+    const unsigned at = threadIdx.x / CH * ((unsigned)workers * CH) + threadIdx.x % CH;
+    const unsigned stride = (unsigned)workers * CH * SLOTS;
+    unsigned target = 0;
+    if (h_probes && !grid_barrier(bar, target += gridDim.x, limit, st)) return;
+    for (int s = 0; s < n_steps; ++s) {
+        const long long n = n0 + s;
+        for (int q = 0; q < n_inst; ++q) {
+            const ResGrid& G = grids[q];
+            for (unsigned t = G.start + at; t < G.cells; t += stride) res_h<real>(ONE ? one : sh[q], G, cur, t, n);
+        }
+        if (!grid_barrier(bar, target += gridDim.x, limit, st)) return;
+        for (int q = 0; q < n_inst; ++q) {
+            const ResGrid& G = grids[q];
+            for (unsigned t = G.start + at; t < G.cells; t += stride) res_e<real>(ONE ? one : sh[q], G, cur, t, n);
+        }
+        if (s + 1 < n_steps && !grid_barrier(bar, target += gridDim.x, limit, st)) return;
+    }
+    // every block read st->step before the first barrier
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->step = n0 + n_steps;
+}
+
+}  // namespace
+
+template <typename real>
+int resident_grid(int n_inst) {
+    int dev = 0, sms = 0, coop = 0, nb = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (!coop) return 0;
+    const size_t smem = n_inst > 1 ? (size_t)n_inst * sizeof(InstDev<real>) : 0;
+    cudaError_t e = n_inst > 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_resident<real, false>,
+                                                                              res_threads<real>(), smem)
+                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_resident<real, true>,
+                                                                              res_threads<real>(), smem);
+    return e == cudaSuccess ? nb * sms : 0;
+}
+
+template <typename real>
+cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d_insts, int n_inst, int cur,
+                            int n_steps, int max_blocks, unsigned* d_bar, unsigned long long limit_ns, DevState* st,
+                            cudaStream_t s) {
+    long long cells = 0, chunks = 0;
+    int h_probes = 0;
+    const int T = res_threads<real>();
+    for (int q = 0; q < n_inst; ++q) {
+        const InstDev<real>& I = h_insts[q];
+        cells += (long long)I.nx * I.ny * I.nz;
+        chunks += (I.n_probe + T - 1) / T;
+        h_probes |= I.n_hprobe > 0;
+    }
+    // probe blocks: each takes one chunk a phase where that leaves most of the grid to the cells
+    const int probe = (int)std::min<long long>(chunks, std::max(1, max_blocks / 8));
+    const int workers = (int)std::min<long long>((cells + T - 1) / T, max_blocks - probe);
+    if (workers < 1) return cudaErrorInvalidValue;
+    cudaError_t e = cudaMemsetAsync(d_bar, 0, sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    InstDev<real> one = h_insts[0];
+    int w = workers, one_chunk = chunks <= probe;
+    void* args[] = {&one, &d_insts, &n_inst, &cur, &n_steps, &w, &h_probes, &one_chunk, &d_bar, &limit_ns, &st};
+    const size_t smem = n_inst > 1 ? (size_t)n_inst * sizeof(InstDev<real>) : 0;
+    const void* f = n_inst > 1 ? (const void*)k_resident<real, false> : (const void*)k_resident<real, true>;
+    return cudaLaunchCooperativeKernel(f, dim3(workers + probe), dim3(T), args, smem, s);
+}
+
+template int resident_grid<float>(int);
+template int resident_grid<double>(int);
+template cudaError_t launch_resident<float>(const InstDev<float>*, const InstDev<float>*, int, int, int, int, unsigned*,
+                                            unsigned long long, DevState*, cudaStream_t);
+template cudaError_t launch_resident<double>(const InstDev<double>*, const InstDev<double>*, int, int, int, int,
+                                             unsigned*, unsigned long long, DevState*, cudaStream_t);
+
+}  // namespace sj

@@ -1,0 +1,67 @@
+"""Small grids step through one cooperative launch per run of steps; the tile
+kernels (which an explicit set_tiling asks for, and which single steps use)
+must give the same bits: same arithmetic per cell, other work split."""
+import numpy as np
+import pytest
+
+from sim_juncs_gb300 import _abi
+from sim_juncs_gb300.configs import inverse_design_case, junction_instance
+from sim_juncs_gb300.fields import Fields
+from sim_juncs_gb300.spec import PML, Grid, Probe
+
+pytestmark = pytest.mark.gpu
+
+
+def odd_box():
+    """Odd, unequal sides; slabs on some faces only; an Hy sheet; H and E probes sampled every 3 steps."""
+    inst = junction_instance(n=45, res=14.0, probe_components=("Ex", "Hy", "Hz"), component=_abi.HY, save_span=3)
+    inst.grid = Grid(37, 45, 29, inst.grid.dx, inst.grid.dt)
+    inst.pml = PML([[0.3, 0.0], [0.0, 0.4], [0.25, 0.25]])
+    return [inst]
+
+
+def whole_slab():
+    """Every column in an x slab, one plane of cells in z, no probes."""
+    inst = junction_instance(n=20, res=14.0)
+    inst.grid = Grid(8, 20, 1, inst.grid.dx, inst.grid.dt)
+    inst.pml = PML([[4 / 14.0, 4 / 14.0], [0.0, 0.0], [0.0, 0.0]])
+    inst.probes, inst.freqs = [], []
+    return [inst]
+
+
+def many_probes():
+    """More probes than the probe blocks hold one each (several chunks per block), on two of three grids."""
+    a, b = junction_instance(n=32, res=10.0), junction_instance(n=33, res=10.5, probe_components=("Ez",), dft=False)
+    a.probes = [Probe(c, (0.3 + 0.0003 * q, 1.6, 1.6), dft=c != _abi.EZ) for c in (0, 2, 4) for q in range(3800)]
+    return [a, junction_instance(n=24, res=7.5, probe_components=(), dft=False), b]
+
+
+def batch():
+    return [junction_instance(n=n, res=r, phase=ph, amplitude=am) for n, r, ph, am in
+            ((64, 20.0, 0.3, 2.0), (40, 12.5, 1.7, 0.5), (64, 20.0, 4.0, 1.0))]
+
+
+CASES = {"odd_box": odd_box, "whole_slab": whole_slab, "many_probes": many_probes, "batch": batch,
+         "quartz": lambda: [inverse_design_case(0, n=72)[0]], "junction65": lambda: [junction_instance(n=65, res=20.0)]}
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("case", CASES)
+def test_resident_runs_equal_tile_launches(lib, case, precision):
+    insts = CASES[case]()
+    a, b = Fields(insts, precision), Fields(insts, precision)
+    b.set_tiling(8, 0, 8)
+    for n in (3, 1, 290, 2):  # odd parities, a single (tile) step between runs, a run longer than one launch
+        a.step(n)
+    a.step_graph(7, chunk=2)
+    b.step(303)
+    assert a.steps_done == b.steps_done == 303
+    a.synchronize()
+    for q in range(len(insts)):
+        for c in range(6):
+            np.testing.assert_array_equal(a.get_array(c, q), b.get_array(c, q), err_msg=f"instance {q} component {c}")
+        np.testing.assert_array_equal(a.monitors(q), b.monitors(q))
+        np.testing.assert_array_equal(a.dft(q), b.dft(q))
+    assert case == "whole_slab" or max(float(np.max(np.abs(a.get_array(c)))) for c in range(6)) > 0
+    a.close()
+    b.close()
