@@ -1630,8 +1630,8 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
     prepare_schedule<real>(sim);
     cudaStream_t st = sim->stream;
     std::vector<void*> temps;  // freed at the end
-    auto tmp = [&](size_t bytes) {
-        void* p = sim->dalloc(bytes);
+    auto tmp = [&](size_t bytes, bool zero) {
+        void* p = sim->dalloc(bytes, zero);
         temps.push_back(p);
         return p;
     };
@@ -1668,8 +1668,12 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
             fail(SJ_E_NOMEM, buf);
         }
     }
-    char* arena = (char*)tmp((size_t)(nseg + 1) * sbytes);
-    std::vector<int> slot_cur(nseg + 1, 0);  // the parity each checkpoint was taken at
+    // the last segment is recorded as the forward pass reaches it and never
+    // re-run; the segments before it need their first state, and the state
+    // after N steps has to be kept only where they overwrite it
+    const long long keep = backward && nseg > 1 ? nseg : 0;  // slots: segments 0 .. nseg-2, then the final state
+    char* arena = keep ? (char*)tmp((size_t)keep * sbytes, false) : nullptr;
+    std::vector<int> slot_cur(keep, 0);  // the parity each checkpoint was taken at
     auto save = [&](long long slot) {
         size_t off = (size_t)slot * sbytes;
         for (const Arr& a : state_of(sim->cur)) {
@@ -1687,35 +1691,54 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
         }
     };
     // ---- objective cells and DFT sums
-    std::vector<int*> d_cells(ni, nullptr);
-    std::vector<double2*> d_D(ni, nullptr);
+    std::vector<ObjDev<real>> O(ni);
     for (int q = 0; q < ni; ++q) {
-        const int nc = objs[q].n_cells;
-        if (nc == 0) continue;
-        d_cells[q] = (int*)tmp((size_t)nc * 3 * sizeof(int));
-        ck(cudaMemcpyAsync(d_cells[q], objs[q].cells, (size_t)nc * 3 * sizeof(int), cudaMemcpyHostToDevice, st),
-           "cells");
-        d_D[q] = (double2*)tmp((size_t)nc * 3 * sizeof(double2));
+        const InstDev<real>& I = dv[q];
+        ObjDev<real>& o = O[q];
+        memset(&o, 0, sizeof(o));
+        for (int b = 0; b < 2; ++b)
+            for (int c = 0; c < 3; ++c) o.E[b][c] = I.F[b][c];
+        o.plane = I.plane, o.px = I.px, o.dt = I.dt;
+        o.n_cells = objs[q].n_cells, o.comp_mask = objs[q].comp_mask, o.freq = objs[q].frequency;
+        if (o.n_cells == 0) continue;
+        int* dc = (int*)tmp((size_t)o.n_cells * 3 * sizeof(int), false);
+        ck(cudaMemcpyAsync(dc, objs[q].cells, (size_t)o.n_cells * 3 * sizeof(int), cudaMemcpyHostToDevice, st), "cells");
+        o.cells = dc;
+        o.D = (double2*)tmp((size_t)o.n_cells * 3 * sizeof(double2), true);
     }
-    // ---- forward from rest, keeping the state every K steps and at the end
+    // ---- records of the E-update bracket at the design points, one segment long
+    std::vector<real*> rec(ni, nullptr);
+    if (backward)
+        for (int q = 0; q < ni; ++q)
+            if (!hv[q].des_eps.empty()) rec[q] = (real*)tmp((size_t)K * hv[q].des_eps.size() * 3 * sizeof(real), true);
+    auto record = [&](long long t0, long long len) {  // len = 0: off
+        if (!backward || total_d == 0) return;
+        for (int q = 0; q < ni; ++q) dv[q].rec_acc = len ? rec[q] : nullptr, dv[q].rec_t0 = t0, dv[q].rec_len = len;
+        upload_table<real>(sim);
+    };
+    // ---- forward from rest
     for (const Arr& a : state_of(sim->cur)) ck(cudaMemsetAsync(a.p, 0, a.bytes, st), "reset");
     for (int q = 0; q < ni; ++q)
         if (dv[q].dft) ck(cudaMemsetAsync(dv[q].dft, 0, (size_t)hv[q].n_dft * hv[q].n_freq * sizeof(double2), st), "reset");
     sim->t = 0;
     set_dev_step<real>(sim, 0);
-    for (long long n = 0; n < N; ++n) {
-        if (n % K == 0) save(n / K);
-        for (int q = 0; q < ni; ++q)
-            ck(launch_objective<real>(dv[q], sim->cur, d_cells[q], objs[q].n_cells, objs[q].comp_mask,
-                                      objs[q].frequency, d_D[q], n, true, nullptr, st),
-               "objective");
-        ck(launch_one<real>(sim), "step launch");
+    for (long long seg = 0; seg < nseg; ++seg) {
+        const long long t0 = seg * K, t1 = std::min(N, t0 + K);
+        if (seg < nseg - 1)
+            save(seg);
+        else
+            record(t0, t1 - t0);
+        for (long long n = t0; n < t1; ++n) {
+            ck(launch_objective<real>(O.data(), ni, sim->cur, n, st), "objective");
+            ck(launch_one<real>(sim), "step launch");
+        }
     }
-    save(nseg);
+    record(0, 0);
+    if (keep) save(nseg - 1);
     std::vector<std::vector<double2>> dft_keep(ni);
     ck(cudaStreamSynchronize(st), "sync");
     for (int q = 0; q < ni; ++q) {
-        if (dv[q].dft) {
+        if (keep && dv[q].dft) {
             dft_keep[q].resize((size_t)hv[q].n_dft * hv[q].n_freq);
             ck(cudaMemcpy(dft_keep[q].data(), dv[q].dft, dft_keep[q].size() * sizeof(double2), cudaMemcpyDeviceToHost),
                "dft");
@@ -1723,7 +1746,7 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
         double F = 0;
         if (objs[q].n_cells) {
             std::vector<double2> D((size_t)objs[q].n_cells * 3);
-            ck(cudaMemcpy(D.data(), d_D[q], D.size() * sizeof(double2), cudaMemcpyDeviceToHost), "objective");
+            ck(cudaMemcpy(D.data(), O[q].D, D.size() * sizeof(double2), cudaMemcpyDeviceToHost), "objective");
             for (const double2& v : D) F += v.x * v.x + v.y * v.y;
         }
         objv[q] = F;
@@ -1742,53 +1765,49 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
         a.I = I;
         const size_t vb = (size_t)I.vol * sizeof(real);
         for (int c = 0; c < 3; ++c) {
-            a.eb[c] = (real*)tmp(vb);
-            a.hb[c] = (real*)tmp(vb);
-            a.t1[c] = (real*)tmp(vb);
-            a.t2[c] = (real*)tmp(vb);
-            a.t3[c] = (real*)tmp(vb);
-            a.t4[c] = (real*)tmp(vb);
+            a.eb[c] = (real*)tmp(vb, true);
+            a.hb[c] = (real*)tmp(vb, true);
+            a.cv[c] = (real*)tmp(vb, false);
         }
         for (int ax = 0; ax < 3; ++ax)
-            if (I.psiE[ax]) a.psEb[ax] = (real*)tmp(2 * vb), a.psHb[ax] = (real*)tmp(2 * vb);
-        if (I.P) a.pb = (real*)tmp((size_t)I.n_poles * 6 * I.dvol * sizeof(real));
+            if (I.psiE[ax]) a.psEb[ax] = (real*)tmp(2 * vb, true), a.psHb[ax] = (real*)tmp(2 * vb, true);
+        if (I.P) a.pb = (real*)tmp((size_t)I.n_poles * 6 * I.dvol * sizeof(real), true);
         const long long nd = (long long)hv[q].des_eps.size();
         if (nd) {
-            a.rec = (const real*)tmp((size_t)K * nd * 3 * sizeof(real));
-            a.g = (double*)tmp((size_t)nd * 3 * sizeof(double));
+            a.rec = rec[q];
+            a.g = (double*)tmp((size_t)nd * 3 * sizeof(double), true);
         }
+        a.cells = O[q].cells, a.D = O[q].D;
+        a.n_cells = O[q].n_cells, a.comp_mask = O[q].comp_mask, a.freq = O[q].freq;
     }
-    // ---- backwards, one segment at a time: re-run it forward recording acc
-    // at the design points, then its transposed steps in reverse
-    bool first = true;  // the sweep's first transposed step has no gather to fold in
+    // ---- backwards, one segment at a time: run it forward once more to record
+    // acc at the design points (the last is recorded already), then its
+    // transposed steps in reverse
     for (long long seg = nseg - 1; seg >= 0; --seg) {
         const long long t0 = seg * K, t1 = std::min(N, t0 + K);
-        restore(seg);
-        sim->t = t0;
-        set_dev_step<real>(sim, t0);
-        for (int q = 0; q < ni; ++q)
-            if (A[q].rec) dv[q].rec_acc = const_cast<real*>(A[q].rec), dv[q].rec_t0 = t0, dv[q].rec_len = t1 - t0;
-        upload_table<real>(sim);
-        for (long long n = t0; n < t1; ++n) ck(launch_one<real>(sim), "step launch");
-        for (int q = 0; q < ni; ++q) dv[q].rec_acc = nullptr, dv[q].rec_len = 0;
-        upload_table<real>(sim);
-        for (long long n = t1 - 1; n >= t0; --n, first = false)
-            for (int q = 0; q < ni; ++q) {
-                A[q].rec_t0 = t0;
-                ck(launch_adjoint_step<real>(A[q], n, first, st), "adjoint step");
-                ck(launch_objective<real>(dv[q], sim->cur, d_cells[q], objs[q].n_cells, objs[q].comp_mask,
-                                          objs[q].frequency, d_D[q], n, false, A[q].eb, st),
-                   "adjoint source");
-            }
+        if (seg < nseg - 1) {
+            restore(seg);
+            sim->t = t0;
+            set_dev_step<real>(sim, t0);
+            record(t0, t1 - t0);
+            for (long long n = t0; n < t1; ++n) ck(launch_one<real>(sim), "step launch");
+            record(0, 0);
+        }
+        for (auto& a : A) a.rec_t0 = t0;
+        for (long long n = t1 - 1; n >= t0; --n)
+            for (const auto& a : A) ck(launch_adjoint_step<real>(a, n, st), "adjoint step");
     }
     // ---- back to the state after N steps
-    restore(nseg);
     sim->t = N;
-    set_dev_step<real>(sim, N);
-    for (int q = 0; q < ni; ++q)
-        if (dv[q].dft)
-            ck(cudaMemcpy(dv[q].dft, dft_keep[q].data(), dft_keep[q].size() * sizeof(double2), cudaMemcpyHostToDevice),
-               "dft");
+    if (keep) {
+        restore(nseg - 1);
+        set_dev_step<real>(sim, N);
+        for (int q = 0; q < ni; ++q)
+            if (dv[q].dft)
+                ck(cudaMemcpy(dv[q].dft, dft_keep[q].data(), dft_keep[q].size() * sizeof(double2), cudaMemcpyHostToDevice),
+                   "dft");
+    }
+    ck(cudaStreamSynchronize(st), "sync");
     // ---- dF/d(eps) = -eps^{-2} sum_c dF/d(inverse eps at the voxel's E_c point)
     long long off = 0;
     for (int q = 0; q < ni; ++q) {

@@ -260,26 +260,37 @@ struct AdjDev {
     InstDev<real> I;            // coefficients, geometry, design region
     real* eb[3];                // dF/dE
     real* hb[3];                // dF/dH
-    real* t1[3];                // per component: adjoint of its first difference (E update)
-    real* t2[3];                // ... and of its second
-    real* t3[3];                // the same for the H update's differences
-    real* t4[3];
-    real* psEb[3];              // [axis] -> [2 slots][vol] (null where the axis has no slab)
-    real* psHb[3];
+    real* cv[3];                // S eps^{-1} dF/dE: the adjoint of the E update's curls
+    real* psEb[3];              // [axis] -> [2 slots][vol] (null where the axis has no slab): psi adjoints
+    real* psHb[3];              // before their factor b
     real* pb;                   // polarisation layout: level 0 = dF/dP^n, level 1 = dF/dP^{n-1}
     const real* rec;            // E-update acc at the design points, [step - rec_t0][d][3]
     long long rec_t0;
     double* g;                  // dF/d(inverse eps) at the design points [d][3]
+    // objective: its cells, E components, frequency and DFT sums [cell][3]
+    const int* cells;
+    int n_cells, comp_mask;
+    double freq;
+    const double2* D;
 };
-// Adjoint step n: the E update's transpose (first = false: with step n+1's
-// gather into dF/dE folded in) and the H update's.
+// Adjoint step n: the E update's transpose (step n+1's gather into dF/dE
+// folded in), the H update's, and the objective's dF/dE^n.
 template <typename real>
-cudaError_t launch_adjoint_step(const AdjDev<real>& a, long long n, bool first, cudaStream_t s);
-// Objective DFT of one instance: D[q][c] += dt E_c^n(cell q) e^{i 2 pi f n dt}
-// (sample = true, from buffer cur) or dF/dE^n source into eb (sample = false).
+cudaError_t launch_adjoint_step(const AdjDev<real>& a, long long n, cudaStream_t s);
+// Objective DFT of an instance: D[q][c] += dt E_c^n(cell q) e^{i 2 pi f n dt},
+// read from buffer cur.
 template <typename real>
-cudaError_t launch_objective(const InstDev<real>& I, int cur, const int* d_cells, int n_cells, int comp_mask,
-                             double freq, double2* d_D, long long n, bool sample, real* const* eb, cudaStream_t s);
+struct ObjDev {
+    const real* E[2][3];
+    long long plane;
+    int px, n_cells, comp_mask;
+    double dt, freq;
+    const int* cells;
+    double2* D;
+};
+constexpr int OBJ_MAX = 32;     // instances of one launch
+template <typename real>
+cudaError_t launch_objective(const ObjDev<real>* o, int n_inst, int cur, long long n, cudaStream_t s);
 
 // Diagnostics (sj_diag.cu): the discrete energy (scale * sum, partial sums in
 // d_partial[energy_partials()]) and the flux spectrum of DFT-probe rows.
