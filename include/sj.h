@@ -317,10 +317,11 @@ int sj_autotune(sj_sim* sim, int32_t steps, int32_t* tile_y, int32_t* ring, int3
 /* ---------------------------------------------------------------- stepping */
 /* n_steps iterations of the loop body at src/disp.cpp:719-741: sample
    monitors when step % save_span == 0, accumulate DFTs, then fields.step().
-   Asynchronous on the sim's stream.  FUSED with its default launch settings
-   and without design regions: on small grids (all instances together at most
-   2^23 cells in FP32, 2^25 in FP64) a call of two or more steps is one
-   cooperative launch per 256 steps, with the tile launches' bits. */
+   Asynchronous on the sim's stream.  FUSED with its default launch settings:
+   on small grids (all instances together at most 2^23 cells in FP32, 2^25 in
+   FP64) a call of two or more steps is one cooperative launch per 256 steps,
+   with the tile launches' bits; sj_adjoint_gradient and sj_objective run
+   forward the same way. */
 int sj_step(sj_sim* sim, int64_t n_steps);
 
 /* same, recorded once into a CUDA graph of `chunk` steps and replayed (small

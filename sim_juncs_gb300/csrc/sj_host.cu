@@ -1354,7 +1354,7 @@ bool resident(sj_sim* sim) {
         return false;
     long long cells = 0;
     for (const InstDev<real>& I : devv<real>(sim)) {
-        if (I.dinv || 2 * I.vol >= (1LL << 32)) return false;
+        if (2 * I.vol >= (1LL << 32)) return false;
         cells += (long long)I.nx * I.ny * I.nz;
     }
     if (cells > res_max_voxels<real>()) return false;
@@ -1365,20 +1365,24 @@ bool resident(sj_sim* sim) {
     return sim->r_blocks > 0;
 }
 
+// n steps in cooperative launches of up to RES_CHUNK; the caller's step mirror
+// is its own affair
+template <typename real>
+void run_resident(sj_sim* sim, long long n, const ObjDev<real>* d_obj = nullptr, int obj_blocks = 0) {
+    const InstDev<real>* d = reinterpret_cast<const InstDev<real>*>(sim->d_table);
+    for (; n > 0; n -= RES_CHUNK)
+        ck(launch_resident<real>(devv<real>(sim).data(), d, sim->n_inst, sim->cur, (int)std::min<long long>(n, RES_CHUNK),
+                                 sim->r_blocks, d_obj, obj_blocks, sim->d_bar, RES_WAIT_NS, sim->d_state, sim->stream),
+           "resident launch");
+}
+
 // n steps with no save point inside: one cooperative launch per RES_CHUNK
 // steps on small grids, else a step's launches n times
 template <typename real>
 void run_steps(sj_sim* sim, long long n) {
     if (n >= 2 && resident<real>(sim)) {
-        const InstDev<real>* d = reinterpret_cast<const InstDev<real>*>(sim->d_table);
-        while (n > 0) {
-            const int m = (int)std::min<long long>(n, RES_CHUNK);
-            ck(launch_resident<real>(devv<real>(sim).data(), d, sim->n_inst, sim->cur, m, sim->r_blocks, sim->d_bar,
-                                     RES_WAIT_NS, sim->d_state, sim->stream),
-               "resident launch");
-            sim->t += m;
-            n -= m;
-        }
+        run_resident<real>(sim, n);
+        sim->t += n;
         return;
     }
     for (; n > 0; --n) {
@@ -1706,6 +1710,14 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
         o.cells = dc;
         o.D = (double2*)tmp((size_t)o.n_cells * 3 * sizeof(double2), true);
     }
+    // small grids run forward through the resident kernel, the objective's sums in blocks of its own
+    const int obj_blocks = resident_objective_blocks<real>(O.data(), ni);
+    const bool res = resident<real>(sim) && obj_blocks <= sim->r_blocks / 4;
+    ObjDev<real>* d_obj = nullptr;
+    if (res) {
+        d_obj = (ObjDev<real>*)tmp(ni * sizeof(ObjDev<real>), false);
+        ck(cudaMemcpyAsync(d_obj, O.data(), ni * sizeof(ObjDev<real>), cudaMemcpyHostToDevice, st), "objectives");
+    }
     // ---- records of the E-update bracket at the design points, one segment long
     std::vector<real*> rec(ni, nullptr);
     if (backward)
@@ -1728,6 +1740,10 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
             save(seg);
         else
             record(t0, t1 - t0);
+        if (res) {
+            run_resident<real>(sim, t1 - t0, d_obj, obj_blocks);
+            continue;
+        }
         for (long long n = t0; n < t1; ++n) {
             ck(launch_objective<real>(O.data(), ni, sim->cur, n, st), "objective");
             ck(launch_one<real>(sim), "step launch");
@@ -1790,7 +1806,10 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
             sim->t = t0;
             set_dev_step<real>(sim, t0);
             record(t0, t1 - t0);
-            for (long long n = t0; n < t1; ++n) ck(launch_one<real>(sim), "step launch");
+            if (res)
+                run_resident<real>(sim, t1 - t0);
+            else
+                for (long long n = t0; n < t1; ++n) ck(launch_one<real>(sim), "step launch");
             record(0, 0);
         }
         for (auto& a : A) a.rec_t0 = t0;

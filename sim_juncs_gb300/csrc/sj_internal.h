@@ -231,17 +231,6 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
                              int n_groups, const LeanGen& gen, const LeanFix& fix, int n_inst, int zb, int dry,
                              int cur, DevState* st, const LeanStreams& ls, int one_column = 0,
                              const LeanQueue<real>* queue = nullptr);
-// Small grids (sj_resident.cu): n_steps steps in one cooperative launch of at
-// most max_blocks resident blocks, in place in buffer `cur`.  resident_grid:
-// the blocks of the kernel that fit the device at once (0: it cannot run).
-// d_bar: the barrier's counter, zeroed by the launch.
-constexpr int RES_MAX_INST = 32;  // instances of one resident launch
-template <typename real>
-int resident_grid(int n_inst);
-template <typename real>
-cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d_insts, int n_inst, int cur,
-                            int n_steps, int max_blocks, unsigned* d_bar, unsigned long long limit_ns, DevState* st,
-                            cudaStream_t s);
 template <typename real>
 int fused_box_width();          // TMA box width in elements (x)
 template <typename real>
@@ -291,6 +280,22 @@ struct ObjDev {
 constexpr int OBJ_MAX = 32;     // instances of one launch
 template <typename real>
 cudaError_t launch_objective(const ObjDev<real>* o, int n_inst, int cur, long long n, cudaStream_t s);
+
+// Small grids (sj_resident.cu): n_steps steps in one cooperative launch of at
+// most max_blocks resident blocks, in place in buffer `cur`.  resident_grid:
+// the blocks of the kernel that fit the device at once (0: it cannot run).
+// d_obj (or null): objectives whose DFT sums the launch keeps, obj_blocks =
+// resident_objective_blocks of them.  d_bar: the barrier's counter, zeroed by
+// the launch.
+constexpr int RES_MAX_INST = 32;  // instances of one resident launch
+template <typename real>
+int resident_grid(int n_inst);
+template <typename real>
+int resident_objective_blocks(const ObjDev<real>* o, int n_inst);
+template <typename real>
+cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d_insts, int n_inst, int cur,
+                            int n_steps, int max_blocks, const ObjDev<real>* d_obj, int obj_blocks, unsigned* d_bar,
+                            unsigned long long limit_ns, DevState* st, cudaStream_t s);
 
 // Diagnostics (sj_diag.cu): the discrete energy (scale * sum, partial sums in
 // d_partial[energy_partials()]) and the flux spectrum of DFT-probe rows.

@@ -21,6 +21,7 @@
 // read during its H phase, which does not write E, and H probes of step n
 // (H^{n-1/2}) during the E phase of step n-1, which does not write H.
 #include <algorithm>
+#include <climits>
 
 #include "sj_physics.cuh"
 
@@ -236,8 +237,10 @@ __device__ __forceinline__ void res_h(const InstDev<real>& I, const ResGrid& G, 
 }
 
 // E^{n+1} of one cell, in place: curl, then the E sources in order, then the
-// polarisations of the cell's material
-template <typename real>
+// polarisations of the cell's material.  DES: a cell of the design region
+// scales by its own eps^-1 and, while a segment is recorded, its bracket
+// S curl H - dt J - dP is stored.
+template <bool DES, typename real>
 __device__ __forceinline__ void res_e(const InstDev<real>& I, const ResGrid& G, int cur, unsigned t, long long n) {
     const Cell c3 = res_cell<real>(G, t);
     const int i = c3.i, j = c3.j, k = c3.k;
@@ -278,37 +281,54 @@ __device__ __forceinline__ void res_e(const InstDev<real>& I, const ResGrid& G, 
         qz0 = pZ[0], qz1 = pZ[vol];
         bz = __ldg(I.prof[2] + k), cz = __ldg(I.prof[2] + nz + k);
     }
+    real sinv[3] = {__ldg(sv), __ldg(sv + 1), __ldg(sv + 2)}, dinv = 0, acc[3];
+    long long d = -1;
+    if (DES && I.dinv) {
+        const int u = i - I.des_lo[0], v = j - I.des_lo[1], w = k - I.des_lo[2];
+        if ((unsigned)u < (unsigned)I.des_n[0] && (unsigned)v < (unsigned)I.des_n[1] &&
+            (unsigned)w < (unsigned)I.des_n[2]) {
+            d = ((long long)w * I.des_n[1] + v) * I.des_n[0] + u;
+            dinv = I.dinv[d];
+            sinv[0] = sinv[1] = sinv[2] = I.S * dinv;
+        }
+    }
     real e[3];
     {
         const real d1 = hz - hz_y, d2 = hy - hy_z;
         real cv = d1 - d2;
         res_term<true>(cv, ay, yo, by, cy, d1, qy0, pY);
         res_term<false>(cv, az, zo, bz, cz, d2, qz0, pZ);
-        e[0] = fma(__ldg(sv), cv, e0[0]);
+        e[0] = fma(sinv[0], cv, e0[0]);
+        if (DES) acc[0] = I.S * cv;
     }
     {
         const real d1 = hx - hx_z, d2 = hz - hz_x;
         real cv = d1 - d2;
         res_term<true>(cv, az, zo, bz, cz, d1, qz1, pZ + vol);
         res_term<false>(cv, ax, xo, bx, cx, d2, qx0, pX);
-        e[1] = fma(__ldg(sv + 1), cv, e0[1]);
+        e[1] = fma(sinv[1], cv, e0[1]);
+        if (DES) acc[1] = I.S * cv;
     }
     {
         const real d1 = hy - hy_x, d2 = hx - hx_y;
         real cv = d1 - d2;
         res_term<true>(cv, ax, xo, bx, cx, d1, qx1, pX + vol);
         res_term<false>(cv, ay, yo, by, cy, d2, qy1, pY + vol);
-        e[2] = fma(__ldg(sv + 2), cv, e0[2]);
+        e[2] = fma(sinv[2], cv, e0[2]);
+        if (DES) acc[2] = I.S * cv;
     }
     if (G.esrc)
         for (int s = 0; s < I.n_src; ++s) {
             const SrcDev<real>& v = I.src[s];
             if (v.comp >= 3 || !src_hit(v, i, j, k)) continue;
             const real J = (real)v.tab[n] * v.w[0][i - v.lo[0]] * v.w[1][j - v.lo[1]] * v.w[2][k - v.lo[2]];
-            const real c = __ldg(cf + v.comp);
+            const real c = DES && d >= 0 ? dinv : __ldg(cf + v.comp);
 #pragma unroll
             for (int a = 0; a < 3; ++a)
-                if (a == v.comp) e[a] = fma(-c, J, e[a]);
+                if (a == v.comp) {
+                    e[a] = fma(-c, J, e[a]);
+                    if (DES) acc[a] -= J;
+                }
         }
     if (mask) {
         const unsigned u = ((unsigned)(k - I.dlo[2]) * (unsigned)I.dn[1] + (unsigned)(j - I.dlo[1])) *
@@ -328,8 +348,14 @@ __device__ __forceinline__ void res_e(const InstDev<real>& I, const ResGrid& G, 
                 pp[lv] = pn;
                 *pp = pnew;
             }
-            e[c] = fma(-__ldg(cf + c), corr, e[c]);
+            e[c] = fma(-(DES && d >= 0 ? dinv : __ldg(cf + c)), corr, e[c]);
+            if (DES) acc[c] -= corr;
         }
+    }
+    if (DES && d >= 0 && I.rec_acc && n >= I.rec_t0 && n < I.rec_t0 + I.rec_len) {
+        const long long nd = (long long)I.des_n[0] * I.des_n[1] * I.des_n[2];
+        real* r = I.rec_acc + ((n - I.rec_t0) * nd + d) * 3;
+        r[0] = acc[0], r[1] = acc[1], r[2] = acc[2];
     }
     *E[0] = e[0];
     *E[1] = e[1];
@@ -435,6 +461,43 @@ __device__ __forceinline__ void res_probes(const InstDev<real>* tab, int n_inst,
     }
 }
 
+// A block that keeps the objective's DFT sums of an instance (one chunk of its
+// cells and components) through a run of steps, sampling E^n during the H phase.
+template <typename real>
+__device__ __noinline__ void res_objective_block(const ObjDev<real>& O, int cur, int chunk, long long n0, int n_steps,
+                                                 int h_probes, unsigned* bar, unsigned long long limit, DevState* st) {
+    __shared__ double2 ph;
+    const int t = chunk * (int)blockDim.x + (int)threadIdx.x, q = t / 3, c = t % 3;
+    const bool on = q < O.n_cells && ((O.comp_mask >> c) & 1);
+    const real* E = nullptr;
+    double2 v = make_double2(0.0, 0.0);
+    if (on) {
+        const int* x = O.cells + 3 * q;
+        E = O.E[cur][c] + ((long long)x[2] * O.plane + (long long)x[1] * O.px + x[0]);
+        v = O.D[t];
+    }
+    const double dt = O.dt;
+    auto phase = [&](long long n) {
+        if (threadIdx.x == 0) sincospi(2.0 * O.freq * ((double)n * dt), &ph.y, &ph.x);
+    };
+    unsigned target = 0;
+    phase(n0);
+    __syncthreads();
+    if (h_probes && !grid_barrier(bar, target += gridDim.x, limit, st)) return;
+    for (int s = 0; s < n_steps; ++s) {
+        const bool more = s + 1 < n_steps;
+        if (on) {
+            const double e = (double)*E * dt;
+            v.x = fma(e, ph.x, v.x);
+            v.y = fma(e, ph.y, v.y);
+        }
+        if (!grid_barrier(bar, target += gridDim.x, limit, st)) return;
+        phase(n0 + s + 1);
+        if (more && !grid_barrier(bar, target += gridDim.x, limit, st)) return;
+    }
+    if (on) O.D[t] = v;
+}
+
 // A probe block's run of steps.  one_chunk: every block has at most one
 // chunk, so a thread keeps its probe, and the phases of its next samples are
 // formed while the cells of the phase before are updated.
@@ -499,18 +562,31 @@ __device__ __noinline__ void res_probe_block(const InstDev<real>* tab, int n_ins
 // ONE: a single instance, its descriptor in the parameter space; else the
 // descriptors are copied to shared memory.  The fields' buffer `cur` is
 // stepped in place.
-template <typename real, bool ONE>
+template <typename real, bool ONE, bool DES>
 __global__ void __launch_bounds__(res_threads<real>(), 1)
 k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __restrict__ tab, int n_inst, int cur,
-           int n_steps, int workers, int h_probes, int one_chunk, unsigned* bar, unsigned long long limit,
-           DevState* st) {
+           int n_steps, int workers, int probe_blocks, int h_probes, int one_chunk, const ObjDev<real>* __restrict__ obj,
+           unsigned* bar, unsigned long long limit, DevState* st) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ ResGrid grids[RES_MAX_INST];
     constexpr unsigned CH = res_chunk<real>(), SLOTS = res_threads<real>() / CH;
     const long long n0 = st->step;
     if ((int)blockIdx.x >= workers) {
-        res_probe_block<real>(tab, n_inst, cur, n0, n_steps, (int)blockIdx.x - workers, (int)gridDim.x - workers,
-                              h_probes, one_chunk, bar, limit, st);
+        int b = (int)blockIdx.x - workers;
+        if (b < probe_blocks) {
+            res_probe_block<real>(tab, n_inst, cur, n0, n_steps, b, probe_blocks, h_probes, one_chunk, bar, limit, st);
+            return;
+        }
+        if constexpr (DES) {
+            b -= probe_blocks;
+            int q = 0;
+            for (;; ++q) {
+                const int c = (3 * obj[q].n_cells + (int)blockDim.x - 1) / (int)blockDim.x;
+                if (b < c) break;
+                b -= c;
+            }
+            res_objective_block<real>(obj[q], cur, b, n0, n_steps, h_probes, bar, limit, st);
+        }
         return;
     }
     InstDev<real>* sh = reinterpret_cast<InstDev<real>*>(smem);
@@ -555,7 +631,7 @@ k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __res
         if (!grid_barrier(bar, target += gridDim.x, limit, st)) return;
         for (int q = 0; q < n_inst; ++q) {
             const ResGrid& G = grids[q];
-            for (unsigned t = G.start + at; t < G.cells; t += stride) res_e<real>(ONE ? one : sh[q], G, cur, t, n);
+            for (unsigned t = G.start + at; t < G.cells; t += stride) res_e<DES>(ONE ? one : sh[q], G, cur, t, n);
         }
         if (s + 1 < n_steps && !grid_barrier(bar, target += gridDim.x, limit, st)) return;
     }
@@ -565,53 +641,77 @@ k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __res
 
 }  // namespace
 
+namespace {
+template <typename real>
+const void* res_kernel(int n_inst, bool des) {
+    if (n_inst > 1) return des ? (const void*)k_resident<real, false, true> : (const void*)k_resident<real, false, false>;
+    return des ? (const void*)k_resident<real, true, true> : (const void*)k_resident<real, true, false>;
+}
+}  // namespace
+
 template <typename real>
 int resident_grid(int n_inst) {
-    int dev = 0, sms = 0, coop = 0, nb = 0;
+    int dev = 0, sms = 0, coop = 0, least = INT_MAX;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (!coop) return 0;
     const size_t smem = n_inst > 1 ? (size_t)n_inst * sizeof(InstDev<real>) : 0;
-    cudaError_t e = n_inst > 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_resident<real, false>,
-                                                                              res_threads<real>(), smem)
-                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_resident<real, true>,
-                                                                              res_threads<real>(), smem);
-    return e == cudaSuccess ? nb * sms : 0;
+    for (int des = 0; des < 2; ++des) {
+        int nb = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, res_kernel<real>(n_inst, des), res_threads<real>(), smem) !=
+            cudaSuccess)
+            return 0;
+        least = std::min(least, nb);
+    }
+    return least * sms;
+}
+
+template <typename real>
+int resident_objective_blocks(const ObjDev<real>* o, int n_inst) {
+    int b = 0;
+    for (int q = 0; q < n_inst; ++q) b += (3 * o[q].n_cells + res_threads<real>() - 1) / res_threads<real>();
+    return b;
 }
 
 template <typename real>
 cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d_insts, int n_inst, int cur,
-                            int n_steps, int max_blocks, unsigned* d_bar, unsigned long long limit_ns, DevState* st,
-                            cudaStream_t s) {
+                            int n_steps, int max_blocks, const ObjDev<real>* d_obj, int obj_blocks, unsigned* d_bar,
+                            unsigned long long limit_ns, DevState* st, cudaStream_t s) {
     long long cells = 0, chunks = 0;
     int h_probes = 0;
+    bool des = d_obj != nullptr;
     const int T = res_threads<real>();
     for (int q = 0; q < n_inst; ++q) {
         const InstDev<real>& I = h_insts[q];
         cells += (long long)I.nx * I.ny * I.nz;
         chunks += (I.n_probe + T - 1) / T;
         h_probes |= I.n_hprobe > 0;
+        des |= I.dinv != nullptr;
     }
     // probe blocks: each takes one chunk a phase where that leaves most of the grid to the cells
-    const int probe = (int)std::min<long long>(chunks, std::max(1, max_blocks / 8));
-    const int workers = (int)std::min<long long>((cells + T - 1) / T, max_blocks - probe);
-    if (workers < 1) return cudaErrorInvalidValue;
+    int probe = (int)std::min<long long>(chunks, std::max(1, max_blocks / 8));
+    int w = (int)std::min<long long>((cells + T - 1) / T, max_blocks - probe - obj_blocks);
+    if (w < 1) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(d_bar, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     InstDev<real> one = h_insts[0];
-    int w = workers, one_chunk = chunks <= probe;
-    void* args[] = {&one, &d_insts, &n_inst, &cur, &n_steps, &w, &h_probes, &one_chunk, &d_bar, &limit_ns, &st};
+    int one_chunk = chunks <= probe;
+    void* args[] = {&one,      &d_insts,   &n_inst, &cur,   &n_steps,  &w, &probe,
+                    &h_probes, &one_chunk, &d_obj,  &d_bar, &limit_ns, &st};
     const size_t smem = n_inst > 1 ? (size_t)n_inst * sizeof(InstDev<real>) : 0;
-    const void* f = n_inst > 1 ? (const void*)k_resident<real, false> : (const void*)k_resident<real, true>;
-    return cudaLaunchCooperativeKernel(f, dim3(workers + probe), dim3(T), args, smem, s);
+    return cudaLaunchCooperativeKernel(res_kernel<real>(n_inst, des), dim3(w + probe + obj_blocks), dim3(T), args, smem, s);
 }
 
 template int resident_grid<float>(int);
 template int resident_grid<double>(int);
-template cudaError_t launch_resident<float>(const InstDev<float>*, const InstDev<float>*, int, int, int, int, unsigned*,
-                                            unsigned long long, DevState*, cudaStream_t);
+template int resident_objective_blocks<float>(const ObjDev<float>*, int);
+template int resident_objective_blocks<double>(const ObjDev<double>*, int);
+template cudaError_t launch_resident<float>(const InstDev<float>*, const InstDev<float>*, int, int, int, int,
+                                            const ObjDev<float>*, int, unsigned*, unsigned long long, DevState*,
+                                            cudaStream_t);
 template cudaError_t launch_resident<double>(const InstDev<double>*, const InstDev<double>*, int, int, int, int,
-                                             unsigned*, unsigned long long, DevState*, cudaStream_t);
+                                             const ObjDev<double>*, int, unsigned*, unsigned long long, DevState*,
+                                             cudaStream_t);
 
 }  // namespace sj

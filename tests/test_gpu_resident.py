@@ -65,3 +65,32 @@ def test_resident_runs_equal_tile_launches(lib, case, precision):
     assert case == "whole_slab" or max(float(np.max(np.abs(a.get_array(c)))) for c in range(6)) > 0
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+def test_design_and_objective_through_both_paths(lib, precision):
+    """Design cells, their recorded brackets (one and several segments) and the objective's sums, two designs of
+    which one has more objective cells than a block has threads."""
+    cases = [inverse_design_case(q, n=72, design_um=(0.4, 0.3, 0.1), patch=p) for q, p in ((0, 5), (1, 19))]
+    for inst, _, _ in cases:
+        inst.sources[0].start_time, inst.sources[0].end_time = -9.0, 11.0
+    out = []
+    for tiles in (False, True):
+        f = Fields([c[0] for c in cases], precision)
+        if tiles:
+            f.set_tiling(8, 0, 16)
+        for q, c in enumerate(cases):
+            f.set_design(c[1], q)
+        f.step(60)
+        grads = [f.adjoint_gradient([c[2] for c in cases], 61, checkpoint_every=k) for k in (20, 61)]
+        out.append((f.objective([c[2] for c in cases], 40), grads, [f.get_array(c, q) for q in (0, 1) for c in range(6)]))
+        f.close()
+    assert out[0][0].min() > 0
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    for (Fa, ga), (Fb, gb) in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(Fa, Fb)
+        for x, y in zip(ga, gb):
+            assert np.max(np.abs(x)) > 0
+            np.testing.assert_array_equal(x, y)
+    for x, y in zip(out[0][2], out[1][2]):
+        np.testing.assert_array_equal(x, y)
