@@ -1051,7 +1051,7 @@ void prepare_lean(sj_sim* sim) {
     sim->lgen.blk = reinterpret_cast<const int4*>(sim->d_gen);
     // correction passes (independent of the tiling)
     std::vector<int2> passes[LEAN_FIX_PASSES];
-    lean_fix_blocks<real>(dv.data(), sim->n_inst, passes);
+    lean_fix_blocks<real>(dv.data(), sim->n_inst, passes, sim->lfix.per);
     std::vector<int2> fall;
     long long foff[LEAN_FIX_PASSES];
     for (int p = 0; p < LEAN_FIX_PASSES; ++p) {
@@ -2267,9 +2267,9 @@ int32_t sj_launches_per_step(const sj_sim* sim) {
             for (int c = 0; c < LEAN_CLASSES; ++c) lt[q].count[c] = (long long)lists[c].size();
         }
         if (sim->precision == SJ_F64)
-            lean_fix_blocks(sim->h64.data(), sim->n_inst, passes);
+            lean_fix_blocks(sim->h64.data(), sim->n_inst, passes, fx.per);
         else
-            lean_fix_blocks(sim->h32.data(), sim->n_inst, passes);
+            lean_fix_blocks(sim->h32.data(), sim->n_inst, passes, fx.per);
         for (int p = 0; p < LEAN_FIX_PASSES; ++p) fx.count[p] = (long long)passes[p].size();
         const LeanGroup* lg = sim->lgroups.data();
         const int ng = (int)sim->lgroups.size();

@@ -1372,19 +1372,16 @@ k_lean_general(const InstDev<real>* __restrict__ parity_tab, const int4* __restr
 // After the tile kernels of a step, on the caller's stream and in this
 // order: one k_lean_esrc launch per source slot s (the instances whose
 // source s is an E source), then one k_lean_disp launch (the instances with
-// dispersive voxels).  Block b takes FIX_THREADS cells of one instance's box:
-// blk[b] = (instance, first cell / FIX_THREADS).  Descriptors come from the
+// dispersive voxels).  Block b takes per * FIX_THREADS cells of one instance's
+// box: blk[b] = (instance, block of that instance).  Descriptors come from the
 // device table; `cur` is the step's parity.
 
 // E^{n+1} = fma(-eps_inf^{-1}, dt J_s, E^{n+1}) over source s's box
-// ESRC_R cells of the box per thread, in turn (fewer, longer blocks pay
-// less for the step counter's fence and atomic at the end of each block);
-// box coordinates in 32 bits.
-constexpr int ESRC_R = 8;
-constexpr int ESRC_CELLS = ESRC_R * FIX_THREADS;
+// `per` cells of the box per thread, in turn (fix_per); box coordinates in 32
+// bits.
 template <typename real>
 __global__ void __launch_bounds__(FIX_THREADS)
-k_lean_esrc(const InstDev<real>* __restrict__ insts, const int2* __restrict__ blk, int slot, int cur,
+k_lean_esrc(const InstDev<real>* __restrict__ insts, const int2* __restrict__ blk, int per, int slot, int cur,
             unsigned step_blocks, int dry, DevState* st) {
     const long long n = st->step;
     const int2 e = __ldg(blk + blockIdx.x);
@@ -1395,8 +1392,8 @@ k_lean_esrc(const InstDev<real>* __restrict__ insts, const int2* __restrict__ bl
     const int lo0 = sv.lo[0], lo1 = sv.lo[1], lo2 = sv.lo[2], comp = sv.comp;
     const real tn = (real)sv.tab[n];
     real* const E = I.F[cur ^ 1][comp];
-    for (int r = 0; r < ESRC_R; ++r) {
-        const unsigned cell = (unsigned)e.y * ESRC_CELLS + r * FIX_THREADS + threadIdx.x;
+    for (int r = 0; r < per; ++r) {
+        const unsigned cell = ((unsigned)e.y * (unsigned)per + r) * FIX_THREADS + threadIdx.x;
         if (cell >= cells) break;
         const unsigned q = cell / n0, dk = q / n1;
         const int di = (int)(cell - q * n0), dj = (int)(q - dk * n1);
@@ -1416,109 +1413,115 @@ k_lean_esrc(const InstDev<real>* __restrict__ insts, const int2* __restrict__ bl
 // E point (pmask), and E^{n+1} = fma(-eps_inf^{-1}, sum_p (P^{n+1} - P^n),
 // E^{n+1}).  A pole the material does not have at the E point keeps P = 0
 // and would add +0: it is neither read nor written, and neither is a
-// component without poles.  One thread per voxel (its three components), a
-// block per DISP_VOXELS voxels of the box (DISP_R per thread, in turn): per
-// voxel the combo first, then E and P of the first two poles of every
-// component together (a third and later pole of a component, which no
-// material here has, follows in order).  Sixteen voxels per thread and four
-// blocks per SM (64 registers): every block ends with the step counter's
-// fence and atomic, so fewer, longer blocks pay less for it (16 x 192^3 Au on
-// quartz, forward step: 4 voxels, 3 blocks per SM 3.21 ms; 4, 4: 2.99; 8, 4:
-// 2.89; 16, 4: 2.85; 32, 4: 2.85).
-#ifndef SJ_DISP_R
-#define SJ_DISP_R 16
-#endif
+// component without poles.  One thread per voxel (its three components), `per`
+// voxels per thread in turn.  A voxel's combo and poles are fetched while the
+// one before is updated; then E and the first pole of every component are
+// loaded together (with TWO, in warps where some voxel's component has more
+// than one pole, the second too; further poles follow in order).  A and B
+// wait in shared memory and the index arithmetic divides by multiplication: the
+// pass spent 467 instructions per voxel, mostly on those and on the second
+// pole that quartz does not have.
+template <typename real>
+struct DispVoxel {
+    int i, j, k, cb;
+    unsigned u, o, mask;  // place in the box, field offset, poles (0: none, or beyond the box)
+};
+template <typename real, bool TWO>
+__device__ __forceinline__ void disp_voxel(const InstDev<real>& I, const DispVoxel<real>& v, const real* sA,
+                                           const real* sB, real* const* Eo, real* const* En, long long n, bool des,
+                                           int dry) {
+    const real* cf = I.coef + v.cb * I.ncoef;
+    const size_t dvol = (size_t)I.dvol;
+    const unsigned o = v.o;
+    real eo[3], ec[3], pn1[3], pq1[3], pn2[3], pq2[3];
+    real* P1[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const unsigned m = (v.mask >> (8 * c)) & 255u;
+        P1[c] = I.P + (size_t)((m ? __ffs(m) - 1 : 0) * 6 + c) * dvol + v.u;
+        eo[c] = m ? Eo[c][o] : real(0), ec[c] = m ? En[c][o] : real(0);
+        pn1[c] = m ? P1[c][0] : real(0), pq1[c] = m ? P1[c][3 * dvol] : real(0);
+        if (TWO) {
+            const unsigned m2 = m & (m - 1);
+            const real* P2 = I.P + (size_t)((m2 ? __ffs(m2) - 1 : 0) * 6 + c) * dvol + v.u;
+            pn2[c] = m2 ? P2[0] : real(0), pq2[c] = m2 ? P2[3 * dvol] : real(0);
+        }
+    }
+    const long long d = des ? design_index(I, v.i, v.j, v.k) : -1;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        unsigned m = (v.mask >> (8 * c)) & 255u;
+        if (!m) continue;
+        real corr = 0;
+        auto pole = [&](int p, real* pp, real pn, real pq) {
+            const real pnew = sA[p] * pn + sB[p] * pq + ldg(cf, 3 + 3 * p + c) * eo[c];
+            corr += pnew - pn;
+            if (!dry) {
+                pp[3 * dvol] = pn;
+                *pp = pnew;
+            }
+        };
+        pole(__ffs(m) - 1, P1[c], pn1[c], pq1[c]);
+        if (TWO) {
+            m &= m - 1;
+            if (m) pole(__ffs(m) - 1, I.P + (size_t)((__ffs(m) - 1) * 6 + c) * dvol + v.u, pn2[c], pq2[c]);
+            for (m &= m - 1; m; m &= m - 1) {
+                real* pp = I.P + (size_t)((__ffs(m) - 1) * 6 + c) * dvol + v.u;
+                pole(__ffs(m) - 1, pp, pp[0], pp[3 * dvol]);
+            }
+        }
+        En[c][o] = fma(-(d >= 0 ? I.dinv[d] : ldg(cf, c)), corr, ec[c]);
+        if (!dry && d >= 0)
+            if (real* rr = design_rec(I, d, n, c)) *rr -= corr;
+    }
+}
+
 #ifndef SJ_DISP_MINB
 #define SJ_DISP_MINB 4
 #endif
-constexpr int DISP_R = SJ_DISP_R;
-constexpr int DISP_VOXELS = DISP_R * FIX_THREADS;
 template <typename real>
 __global__ void __launch_bounds__(FIX_THREADS, sizeof(real) == 4 ? SJ_DISP_MINB : 2)
-k_lean_disp(const InstDev<real>* __restrict__ insts, const int2* __restrict__ blk, int cur, unsigned step_blocks,
-            int dry, DevState* st) {
+k_lean_disp(const InstDev<real>* __restrict__ insts, const int2* __restrict__ blk, int per, int cur,
+            unsigned step_blocks, int dry, DevState* st) {
+    __shared__ Div s_div[2];
+    __shared__ real sA[MAXP], sB[MAXP];
     const long long n = st->step;
     const int2 e = __ldg(blk + blockIdx.x);
     const InstDev<real>& I = insts[e.x];
+    if (threadIdx.x < 2) s_div[threadIdx.x].set((unsigned)I.dn[threadIdx.x]);
+    if (threadIdx.x < MAXP) sA[threadIdx.x] = I.A[threadIdx.x], sB[threadIdx.x] = I.B[threadIdx.x];
+    __syncthreads();
     // the descriptor's fields, read once (offsets within an instance fit 32 bits)
     const unsigned dvol = (unsigned)I.dvol, d0 = (unsigned)I.dn[0], d1 = (unsigned)I.dn[1];
     const int lo0 = I.dlo[0], lo1 = I.dlo[1], lo2 = I.dlo[2];
     const unsigned plane = (unsigned)I.plane, px = (unsigned)I.px;
     const uint8_t* combo = I.combo;
     const uint32_t* pmask = I.pmask;
-    const real* coef = I.coef;
-    const int ncoef = I.ncoef;
-    real* const P = I.P;
-    const real* Eo[3] = {I.F[cur][0], I.F[cur][1], I.F[cur][2]};
+    real* const Eo[3] = {I.F[cur][0], I.F[cur][1], I.F[cur][2]};
     real* const En[3] = {I.F[cur ^ 1][0], I.F[cur ^ 1][1], I.F[cur ^ 1][2]};
-    const long long lv = 3 * (long long)dvol;  // from level n to level n-1 of a pole
-    const unsigned base = (unsigned)e.y * DISP_VOXELS + threadIdx.x;
-    for (int r = 0; r < DISP_R; ++r) {
-        const unsigned u = base + r * FIX_THREADS;
-        if (u >= dvol) break;
-        const unsigned q = u / d0, kk = q / d1;
-        const int i = lo0 + (int)(u - q * d0), j = lo1 + (int)(q - kk * d1), k = lo2 + (int)kk;
-        const unsigned o = (unsigned)k * plane + (unsigned)j * px + (unsigned)i;
-        const int cb = combo[o];
-        const unsigned mask = pmask[cb];
-        if (!mask) continue;
-        const real* cf = coef + cb * ncoef;
-        real eo[3], ec[3], pn1[3], pq1[3], pn2[3], pq2[3], c1[3], c2[3];
-        int pa[3], pb[3];
-        unsigned rest[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const unsigned m = (mask >> (8 * c)) & 255u;
-            const unsigned m2 = m & (m - 1);
-            pa[c] = m ? __ffs(m) - 1 : -1;
-            pb[c] = m2 ? __ffs(m2) - 1 : -1;
-            rest[c] = m2 & (m2 - 1);
-            eo[c] = m ? Eo[c][o] : real(0);
-            ec[c] = m ? En[c][o] : real(0);
-            const long long a1 = ((long long)pa[c] * 6 + c) * dvol + u, a2 = ((long long)pb[c] * 6 + c) * dvol + u;
-            c1[c] = m ? cf[3 + 3 * pa[c] + c] : real(0);
-            c2[c] = m2 ? cf[3 + 3 * pb[c] + c] : real(0);
-            pn1[c] = m ? P[a1] : real(0), pq1[c] = m ? P[a1 + lv] : real(0);
-            pn2[c] = m2 ? P[a2] : real(0), pq2[c] = m2 ? P[a2 + lv] : real(0);
-        }
-        const long long d = design_index(I, i, j, k);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            if (pa[c] < 0) continue;
-            real corr = 0;
-            {
-                const real pnew = I.A[pa[c]] * pn1[c] + I.B[pa[c]] * pq1[c] + c1[c] * eo[c];
-                corr += pnew - pn1[c];
-                if (!dry) {
-                    real* pp = P + ((long long)pa[c] * 6 + c) * dvol + u;
-                    pp[lv] = pn1[c];
-                    *pp = pnew;
-                }
-            }
-            if (pb[c] >= 0) {
-                const real pnew = I.A[pb[c]] * pn2[c] + I.B[pb[c]] * pq2[c] + c2[c] * eo[c];
-                corr += pnew - pn2[c];
-                if (!dry) {
-                    real* pp = P + ((long long)pb[c] * 6 + c) * dvol + u;
-                    pp[lv] = pn2[c];
-                    *pp = pnew;
-                }
-            }
-            for (unsigned m = rest[c]; m; m &= m - 1) {
-                const int p = __ffs(m) - 1;
-                real* pp = P + ((long long)p * 6 + c) * dvol + u;
-                const real pn = *pp, pq = pp[lv];
-                const real pnew = I.A[p] * pn + I.B[p] * pq + cf[3 + 3 * p + c] * eo[c];
-                corr += pnew - pn;
-                if (!dry) {
-                    pp[lv] = pn;
-                    *pp = pnew;
-                }
-            }
-            En[c][o] = fma(-(d >= 0 ? I.dinv[d] : cf[c]), corr, ec[c]);
-            if (!dry)
-                if (real* rr = design_rec(I, d, n, c)) *rr -= corr;
-        }
+    const bool des = I.dinv != nullptr;
+    const Div D0 = s_div[0], D1 = s_div[1];
+    auto voxel = [&](unsigned u) {
+        DispVoxel<real> v;
+        v.u = u;
+        const unsigned q = D0.div(u), kk = D1.div(q);
+        v.i = lo0 + (int)(u - q * d0), v.j = lo1 + (int)(q - kk * d1), v.k = lo2 + (int)kk;
+        v.o = (unsigned)v.k * plane + (unsigned)v.j * px + (unsigned)v.i;
+        v.cb = u < dvol ? __ldg(combo + v.o) : 0;
+        v.mask = u < dvol ? __ldg(pmask + v.cb) : 0u;
+        return v;
+    };
+    const unsigned base = (unsigned)e.y * (unsigned)per * FIX_THREADS + threadIdx.x;
+    DispVoxel<real> next = voxel(base);
+    for (int r = 0; r < per; ++r) {
+        const DispVoxel<real> v = next;
+        if (v.u >= dvol) break;
+        if (r + 1 < per) next = voxel(v.u + FIX_THREADS);
+        const unsigned two = (v.mask & (v.mask - 0x010101u)) & 0xffffffu;  // nonzero where a byte may hold two bits
+        if (__any_sync(__activemask(), two != 0))
+            disp_voxel<real, true>(I, v, sA, sB, Eo, En, n, des, dry);
+        else if (v.mask)
+            disp_voxel<real, false>(I, v, sA, sB, Eo, En, n, des, dry);
     }
     finish_block(step_blocks, dry, st);
 }
@@ -1586,23 +1589,37 @@ template void lean_gen_blocks<float>(const InstDev<float>*, const std::vector<un
 template void lean_gen_blocks<double>(const InstDev<double>*, const std::vector<unsigned>*, int,
                                       std::vector<int4>&, long long&);
 
+// Cells per thread of a correction pass: every block ends with the step
+// counter's fence and atomic, so few long blocks are cheaper where they fill
+// the device (16 x 192^3 on quartz, polarisation pass: 4 / 8 / 16 per thread
+// 2.99 / 2.89 / 2.85 ms a step), but a pass is the tail of its step, and on
+// a few thousand cells long blocks are a serial chain on a few SMs (4 members
+// of each sweep size: 16 / 8 per thread 779 / 758 us a step).
+int fix_per(long long cells, int most) {
+    int per = most;
+    while (per > 1 && cells < 1216LL * FIX_THREADS * per) per >>= 1;
+    return per;
+}
+
 template <typename real>
-void lean_fix_blocks(const InstDev<real>* h_insts, int n_inst, std::vector<int2>* passes) {
-    for (int p = 0; p < LEAN_FIX_PASSES; ++p) passes[p].clear();
-    for (int q = 0; q < n_inst; ++q) {
+void lean_fix_blocks(const InstDev<real>* h_insts, int n_inst, std::vector<int2>* passes, int* per) {
+    auto cells_of = [&](int q, int p) -> long long {  // cells of pass p in instance q
         const InstDev<real>& I = h_insts[q];
-        for (int s = 0; s < I.n_src; ++s) {
-            if (I.src[s].comp >= 3) continue;
-            const long long cells = (long long)I.src[s].n[0] * I.src[s].n[1] * I.src[s].n[2];
-            for (long long b = 0; b * ESRC_CELLS < cells; ++b) passes[s].push_back(make_int2(q, (int)b));
-        }
-        if (I.n_poles > 0 && I.dvol > 0)
-            for (long long b = 0; b * DISP_VOXELS < I.dvol; ++b)
-                passes[SJ_MAX_SOURCES].push_back(make_int2(q, (int)b));
+        if (p == SJ_MAX_SOURCES) return I.n_poles > 0 ? I.dvol : 0;
+        if (p >= I.n_src || I.src[p].comp >= 3) return 0;
+        return (long long)I.src[p].n[0] * I.src[p].n[1] * I.src[p].n[2];
+    };
+    for (int p = 0; p < LEAN_FIX_PASSES; ++p) {
+        passes[p].clear();
+        long long total = 0;
+        for (int q = 0; q < n_inst; ++q) total += cells_of(q, p);
+        per[p] = fix_per(total, p == SJ_MAX_SOURCES ? 16 : 8);
+        for (int q = 0; q < n_inst; ++q)
+            for (long long b = 0; b * per[p] * FIX_THREADS < cells_of(q, p); ++b) passes[p].push_back(make_int2(q, (int)b));
     }
 }
-template void lean_fix_blocks<float>(const InstDev<float>*, int, std::vector<int2>*);
-template void lean_fix_blocks<double>(const InstDev<double>*, int, std::vector<int2>*);
+template void lean_fix_blocks<float>(const InstDev<float>*, int, std::vector<int2>*, int*);
+template void lean_fix_blocks<double>(const InstDev<double>*, int, std::vector<int2>*, int*);
 
 // Each class of instance q goes to its own stream of set q % LEAN_SETS: the
 // kernels of a step overlap and fill each other's tails.  Only as many sets
@@ -1737,9 +1754,10 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
         if (!fix.count[p]) continue;
         const unsigned nb = (unsigned)fix.count[p];
         if (p < SJ_MAX_SOURCES)
-            k_lean_esrc<real><<<nb, FIX_THREADS, 0, ls.main>>>(d_insts, fix.blk[p], p, cur, (unsigned)gtotal, dry, st);
+            k_lean_esrc<real><<<nb, FIX_THREADS, 0, ls.main>>>(d_insts, fix.blk[p], fix.per[p], p, cur, (unsigned)gtotal,
+                                                               dry, st);
         else
-            k_lean_disp<real><<<nb, FIX_THREADS, 0, ls.main>>>(d_insts, fix.blk[p], cur, (unsigned)gtotal, dry, st);
+            k_lean_disp<real><<<nb, FIX_THREADS, 0, ls.main>>>(d_insts, fix.blk[p], fix.per[p], cur, (unsigned)gtotal, dry, st);
         e = cudaGetLastError();
     }
     return e;

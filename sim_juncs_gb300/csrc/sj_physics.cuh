@@ -9,6 +9,18 @@
 
 namespace sj {
 
+// q = t / d for t < 2^31 by multiplication (Granlund and Montgomery, "Division
+// by invariant integers using multiplication", 1994)
+struct Div {
+    unsigned d, m, s;
+    __device__ __forceinline__ void set(unsigned dd) {
+        d = dd;
+        s = dd > 1 ? 32 - __clz(dd - 1) : 0;
+        m = (unsigned)((((1ull << 32) * ((1ull << s) - dd)) / dd) + 1);
+    }
+    __device__ __forceinline__ unsigned div(unsigned t) const { return (__umulhi(t, m) + t) >> s; }
+};
+
 // Store monitor sample v of monitor column ms taken before step n, and apply
 // the divergence guard (bound_geom::run flags samples above 1000,
 // src/disp.cpp:727-729): the first sample of the sim with |v| above the bound,

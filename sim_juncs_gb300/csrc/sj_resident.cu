@@ -52,18 +52,6 @@ constexpr int res_threads() { return sizeof(real) == 4 ? SJ_RES_THREADS32 : 512;
 template <typename real>
 constexpr int res_chunk() { return sizeof(real) == 4 ? SJ_RES_CHUNK32 : SJ_RES_CHUNK64; }
 
-// q = t / d for t < 2^31 by multiplication (Granlund and Montgomery, "Division
-// by invariant integers using multiplication", 1994)
-struct Div {
-    unsigned d, m, s;
-    __device__ __forceinline__ void set(unsigned dd) {
-        d = dd;
-        s = dd > 1 ? 32 - __clz(dd - 1) : 0;
-        m = (unsigned)((((1ull << 32) * ((1ull << s) - dd)) / dd) + 1);
-    }
-    __device__ __forceinline__ unsigned div(unsigned t) const { return (__umulhi(t, m) + t) >> s; }
-};
-
 // What a block knows of one instance besides its descriptor.  FP64 deals the
 // columns between the x slabs first and the slabs' columns after them: a
 // warp then seldom mixes the two, and only the slabs' warps pay for the x
