@@ -334,6 +334,20 @@ __device__ __forceinline__ void pml_term_v(real& cv, bool on, real b, real c, re
     if (on && store) pout[x] = ps;
     cv = ADD ? cv + (on ? ps : real(-0.0)) : cv - (on ? ps : real(0));
 }
+// The same for a pair of columns with one store: the pair's psi goes out as one
+// vector (two scalar stores leave each 32-byte sector to two half-written
+// requests).  st: the pair's sectors hold a slab cell; a cell outside the
+// slab has psi 0 and b = 1, c = 0, so 0 is stored there, which nothing reads.
+template <bool AX, bool ADD, typename real>
+__device__ __forceinline__ void pml_pair(real& cv0, real& cv1, bool on0, bool on1, bool st, real b0, real b1, real c0,
+                                         real c1, real d0, real d1, real p0, real p1, real* pout, unsigned x) {
+    if (!AX) return;
+    if (sizeof(real) == 8 && !__any_sync(__activemask(), on0 || on1 || st)) return;
+    const real s0 = fma(b0, p0, c0 * d0), s1 = fma(b1, p1, c1 * d1);
+    if (st) st2(pout, x, s0, s1);
+    cv0 = ADD ? cv0 + (on0 ? s0 : real(-0.0)) : cv0 - (on0 ? s0 : real(0));
+    cv1 = ADD ? cv1 + (on1 ? s1 : real(-0.0)) : cv1 - (on1 ? s1 : real(0));
+}
 // old psi of a cell in the slab (predicated load), 0 elsewhere
 template <bool AX, bool NC, typename real>
 __device__ __forceinline__ real psi_old(bool on, const real* pin, unsigned x) {
@@ -917,6 +931,10 @@ __device__ __forceinline__ void tile_pair_halo(const InstDev<real>& I, int tx, i
     const bool xm = !EDGE || i0 > 0, ym = !EDGE || j0 > 0;
     const bool xo0 = SX && in_slab(I, 0, i), xo1 = SX && in_slab(I, 0, i + 1), xo = xo0 || xo1;
     const bool yo = SY && in_slab(I, 1, j);
+    // the pair's 32-byte sector of a row holds a cell of an x slab: x psi is
+    // stored in whole sectors (a partly written one costs a read in memory)
+    constexpr int SEC = 32 / (int)sizeof(real);
+    const bool xst = SX && (in_slab(I, 0, i & ~(SEC - 1)) || in_slab(I, 0, i | (SEC - 1)));
     real bxi0 = 1, cxi0 = 0, bxh0 = 1, cxh0 = 0, bxi1 = 1, cxi1 = 0, bxh1 = 1, cxh1 = 0;
     real byi = 1, cyi = 0, byh = 1, cyh = 0;
     if (SX) {
@@ -976,36 +994,34 @@ __device__ __forceinline__ void tile_pair_halo(const InstDev<real>& I, int tx, i
         const bool sp = store && !dry && own && act;
 
         // H^{n+1/2} at the thread's two cells
+        const bool spx = sp && xst, spy = sp && yo, spz = sp && zo;
         V2 hx, hy, hz;
         {
-            real d1 = c.ez_yp.x - c.ez.x, d2 = c.ey_n.x - ey_c.x, cv = d1 - d2;
-            pml_term_v<SY, true>(cv, yo, byh, cyh, d1, c.qy0.x, hoY, op, sp);
-            pml_term_v<SZ, false>(cv, zo, bzh, czh, d2, c.qz0.x, hoZ, op, sp);
+            const real d1 = c.ez_yp.x - c.ez.x, d2 = c.ey_n.x - ey_c.x;
+            const real f1 = c.ez_yp.y - c.ez.y, f2 = c.ey_n.y - ey_c.y;
+            real cv = d1 - d2, cw = f1 - f2;
+            pml_pair<SY, true>(cv, cw, yo, yo, spy, byh, byh, cyh, cyh, d1, f1, c.qy0.x, c.qy0.y, hoY, op);
+            pml_pair<SZ, false>(cv, cw, zo, zo, spz, bzh, bzh, czh, czh, d2, f2, c.qz0.x, c.qz0.y, hoZ, op);
             hx.x = fma(-S, cv, c.hx.x);
-            d1 = c.ez_yp.y - c.ez.y, d2 = c.ey_n.y - ey_c.y, cv = d1 - d2;
-            pml_term_v<SY, true>(cv, yo, byh, cyh, d1, c.qy0.y, hoY, op + 1, sp);
-            pml_term_v<SZ, false>(cv, zo, bzh, czh, d2, c.qz0.y, hoZ, op + 1, sp);
-            hx.y = fma(-S, cv, c.hx.y);
+            hx.y = fma(-S, cw, c.hx.y);
         }
         {
-            real d1 = c.ex_n.x - ex_c.x, d2 = c.ez.y - c.ez.x, cv = d1 - d2;
-            pml_term_v<SZ, true>(cv, zo, bzh, czh, d1, c.qz1.x, hoZ + vol, op, sp);
-            pml_term_v<SX, false>(cv, xo0, bxh0, cxh0, d2, c.qx0.x, hoX, op, sp);
+            const real d1 = c.ex_n.x - ex_c.x, d2 = c.ez.y - c.ez.x;
+            const real f1 = c.ex_n.y - ex_c.y, f2 = c.ez_x2 - c.ez.y;
+            real cv = d1 - d2, cw = f1 - f2;
+            pml_pair<SZ, true>(cv, cw, zo, zo, spz, bzh, bzh, czh, czh, d1, f1, c.qz1.x, c.qz1.y, hoZ + vol, op);
+            pml_pair<SX, false>(cv, cw, xo0, xo1, spx, bxh0, bxh1, cxh0, cxh1, d2, f2, c.qx0.x, c.qx0.y, hoX, op);
             hy.x = fma(-S, cv, c.hy.x);
-            d1 = c.ex_n.y - ex_c.y, d2 = c.ez_x2 - c.ez.y, cv = d1 - d2;
-            pml_term_v<SZ, true>(cv, zo, bzh, czh, d1, c.qz1.y, hoZ + vol, op + 1, sp);
-            pml_term_v<SX, false>(cv, xo1, bxh1, cxh1, d2, c.qx0.y, hoX, op + 1, sp);
-            hy.y = fma(-S, cv, c.hy.y);
+            hy.y = fma(-S, cw, c.hy.y);
         }
         {
-            real d1 = ey_c.y - ey_c.x, d2 = c.ex_yp.x - ex_c.x, cv = d1 - d2;
-            pml_term_v<SX, true>(cv, xo0, bxh0, cxh0, d1, c.qx1.x, hoX + vol, op, sp);
-            pml_term_v<SY, false>(cv, yo, byh, cyh, d2, c.qy1.x, hoY + vol, op, sp);
+            const real d1 = ey_c.y - ey_c.x, d2 = c.ex_yp.x - ex_c.x;
+            const real f1 = c.ey_x2 - ey_c.y, f2 = c.ex_yp.y - ex_c.y;
+            real cv = d1 - d2, cw = f1 - f2;
+            pml_pair<SX, true>(cv, cw, xo0, xo1, spx, bxh0, bxh1, cxh0, cxh1, d1, f1, c.qx1.x, c.qx1.y, hoX + vol, op);
+            pml_pair<SY, false>(cv, cw, yo, yo, spy, byh, byh, cyh, cyh, d2, f2, c.qy1.x, c.qy1.y, hoY + vol, op);
             hz.x = fma(-S, cv, c.hz.x);
-            d1 = c.ey_x2 - ey_c.y, d2 = c.ex_yp.y - ex_c.y, cv = d1 - d2;
-            pml_term_v<SX, true>(cv, xo1, bxh1, cxh1, d1, c.qx1.y, hoX + vol, op + 1, sp);
-            pml_term_v<SY, false>(cv, yo, byh, cyh, d2, c.qy1.y, hoY + vol, op + 1, sp);
-            hz.y = fma(-S, cv, c.hz.y);
+            hz.y = fma(-S, cw, c.hz.y);
         }
         if (store) {
             // the E update's loads ahead of the barrier: S eps_inf^-1 of both
@@ -1042,37 +1058,34 @@ __device__ __forceinline__ void tile_pair_halo(const InstDev<real>& I, int tx, i
                     st2(oHX, o, hx.x, hx.y);
                     st2(oHY, o, hy.x, hy.y);
                     st2(oHZ, o, hz.x, hz.y);
-                    const bool si = !dry;
+                    const bool six = !dry && xst, siy = !dry && yo, siz = !dry && zo;
                     V2 ex, ey, ezn;
                     {
-                        real d1 = hz.x - hz_ym.x, d2 = hy.x - hyp.x, cv = d1 - d2;
-                        pml_term_v<SY, true>(cv, yo, byi, cyi, d1, pY0.x, peY, op, si);
-                        pml_term_v<SZ, false>(cv, zo, bzi, czi, d2, pZ0.x, peZ, op, si);
+                        const real d1 = hz.x - hz_ym.x, d2 = hy.x - hyp.x;
+                        const real f1 = hz.y - hz_ym.y, f2 = hy.y - hyp.y;
+                        real cv = d1 - d2, cw = f1 - f2;
+                        pml_pair<SY, true>(cv, cw, yo, yo, siy, byi, byi, cyi, cyi, d1, f1, pY0.x, pY0.y, peY, op);
+                        pml_pair<SZ, false>(cv, cw, zo, zo, siz, bzi, bzi, czi, czi, d2, f2, pZ0.x, pZ0.y, peZ, op);
                         ex.x = e_new_v(a0, ex_c.x, cv);
-                        d1 = hz.y - hz_ym.y, d2 = hy.y - hyp.y, cv = d1 - d2;
-                        pml_term_v<SY, true>(cv, yo, byi, cyi, d1, pY0.y, peY, op + 1, si);
-                        pml_term_v<SZ, false>(cv, zo, bzi, czi, d2, pZ0.y, peZ, op + 1, si);
-                        ex.y = e_new_v(b0, ex_c.y, cv);
+                        ex.y = e_new_v(b0, ex_c.y, cw);
                     }
                     {
-                        real d1 = hx.x - hxp.x, d2 = hz.x - hz_m, cv = d1 - d2;
-                        pml_term_v<SZ, true>(cv, zo, bzi, czi, d1, pZ1.x, peZ + vol, op, si);
-                        pml_term_v<SX, false>(cv, xo0, bxi0, cxi0, d2, pX0.x, peX, op, si);
+                        const real d1 = hx.x - hxp.x, d2 = hz.x - hz_m;
+                        const real f1 = hx.y - hxp.y, f2 = hz.y - hz.x;
+                        real cv = d1 - d2, cw = f1 - f2;
+                        pml_pair<SZ, true>(cv, cw, zo, zo, siz, bzi, bzi, czi, czi, d1, f1, pZ1.x, pZ1.y, peZ + vol, op);
+                        pml_pair<SX, false>(cv, cw, xo0, xo1, six, bxi0, bxi1, cxi0, cxi1, d2, f2, pX0.x, pX0.y, peX, op);
                         ey.x = e_new_v(a1, ey_c.x, cv);
-                        d1 = hx.y - hxp.y, d2 = hz.y - hz.x, cv = d1 - d2;
-                        pml_term_v<SZ, true>(cv, zo, bzi, czi, d1, pZ1.y, peZ + vol, op + 1, si);
-                        pml_term_v<SX, false>(cv, xo1, bxi1, cxi1, d2, pX0.y, peX, op + 1, si);
-                        ey.y = e_new_v(b1, ey_c.y, cv);
+                        ey.y = e_new_v(b1, ey_c.y, cw);
                     }
                     {
-                        real d1 = hy.x - hy_m, d2 = hx.x - hx_ym.x, cv = d1 - d2;
-                        pml_term_v<SX, true>(cv, xo0, bxi0, cxi0, d1, pX1.x, peX + vol, op, si);
-                        pml_term_v<SY, false>(cv, yo, byi, cyi, d2, pY1.x, peY + vol, op, si);
+                        const real d1 = hy.x - hy_m, d2 = hx.x - hx_ym.x;
+                        const real f1 = hy.y - hy.x, f2 = hx.y - hx_ym.y;
+                        real cv = d1 - d2, cw = f1 - f2;
+                        pml_pair<SX, true>(cv, cw, xo0, xo1, six, bxi0, bxi1, cxi0, cxi1, d1, f1, pX1.x, pX1.y, peX + vol, op);
+                        pml_pair<SY, false>(cv, cw, yo, yo, siy, byi, byi, cyi, cyi, d2, f2, pY1.x, pY1.y, peY + vol, op);
                         ezn.x = e_new_v(a2, c.ez.x, cv);
-                        d1 = hy.y - hy.x, d2 = hx.y - hx_ym.y, cv = d1 - d2;
-                        pml_term_v<SX, true>(cv, xo1, bxi1, cxi1, d1, pX1.y, peX + vol, op + 1, si);
-                        pml_term_v<SY, false>(cv, yo, byi, cyi, d2, pY1.y, peY + vol, op + 1, si);
-                        ezn.y = e_new_v(b2, c.ez.y, cv);
+                        ezn.y = e_new_v(b2, c.ez.y, cw);
                     }
                     st2(oEX, o, ex.x, ex.y);
                     st2(oEY, o, ey.x, ey.y);
@@ -1235,11 +1248,14 @@ k_lean_multi(const __grid_constant__ LeanTable<real> tab) {
 }
 
 // Single- and multi-slab tiles with two columns per thread (instances whose
-// nx is a multiple of 32), 5 warps per tile.  The single-slab body fits 64
-// registers without spilling (6 blocks per SM); the multi-slab body spills a
-// little at 5 blocks per SM and still runs faster there than at 4 or 6.
+// nx is a multiple of 32), 5 warps per tile.  The single-slab body takes 72
+// registers (5 blocks per SM; at 6, with 64, the sweep's 96^3 group is 2%
+// slower); the multi-slab body spills a little at 5 blocks per SM and runs as
+// fast there as at 4, faster than at 6.  With each pair's psi stored as one
+// vector in whole sectors the 32 x 96^3 group takes 597 us per step (631
+// before), 32 x 128^3 1220 (1250), 32 x 192^3 3790 (3857: 4.9 TB/s).
 #ifndef SJ_LEAN_SLAB2_MINB
-#define SJ_LEAN_SLAB2_MINB 6
+#define SJ_LEAN_SLAB2_MINB 5
 #endif
 #ifndef SJ_LEAN_MULTI2_MINB
 #define SJ_LEAN_MULTI2_MINB 5
