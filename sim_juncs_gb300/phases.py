@@ -12,13 +12,11 @@ FIELDS = ("f0", "phi", "t0_corr", "t0", "mu", "sig", "skew", "f0_ind", "band_lo"
           "lowpass_steps", "status")
 
 
-def _to_dicts(res):
-    out = []
-    for r in res:
-        d = {k: getattr(r, k) for k in FIELDS}
-        d["amp"] = complex(r.amp[0], r.amp[1])
-        out.append(d)
-    return out
+def _to_dicts(res, n):
+    a = np.frombuffer(res, dtype=np.dtype(_abi.PhaseResult), count=n)
+    cols = [a[k].tolist() for k in FIELDS] + [a["amp"].view(np.complex128)[..., 0].tolist() if n else []]
+    names = FIELDS + ("amp",)
+    return [dict(zip(names, row)) for row in zip(*cols)]
 
 
 def extract_phases(t, v, lowpass_inc=1.0):
@@ -34,7 +32,7 @@ def extract_phases(t, v, lowpass_inc=1.0):
     res = (_abi.PhaseResult * max(n, 1))()
     _abi.check(lib, lib.sj_extract_phases(n, m, t.ctypes.data_as(C.POINTER(C.c_double)),
                                           v.ctypes.data_as(C.POINTER(C.c_double)), float(lowpass_inc), res))
-    return _to_dicts(res[:n])
+    return _to_dicts(res, n)
 
 
 def monitor_phases(fields, lowpass_inc=1.0):
@@ -45,7 +43,7 @@ def monitor_phases(fields, lowpass_inc=1.0):
     total = sum(counts)
     res = (_abi.PhaseResult * max(total, 1))()
     fields._ck(lib.sj_extract_monitor_phases(fields.handle, float(lowpass_inc), res, total))
-    flat = _to_dicts(res[:total])
+    flat = _to_dicts(res, total)
     out, off = [], 0
     for c in counts:
         out.append(flat[off:off + c])
