@@ -2314,8 +2314,9 @@ int sj_monitor_spectrum(sj_sim* sim, int32_t inst, double* out, size_t cap) {
     const long long n = sj_n_samples(sim, inst), np = sj_monitor_spectrum_length(sim, inst);
     if ((size_t)nm * np * 2 > cap) fail(SJ_E_RANGE, "out too small: n_monitors * length * 2 doubles");
     if (nm > 0 && np > 0) {
-        double* d_out = (double*)sim->dalloc((size_t)nm * np * 2 * sizeof(double), false);
-        cudaError_t e = launch_spectrum(dm, nm, n, np, d_out, sim->stream);
+        const size_t vals = (size_t)nm * np * 2;  // then the phase table
+        double* d_out = (double*)sim->dalloc(vals * sizeof(double) + (size_t)n * sizeof(double2), false);
+        cudaError_t e = launch_spectrum(dm, nm, n, np, reinterpret_cast<double2*>(d_out + vals), d_out, sim->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(sim->stream);
         if (e == cudaSuccess)
             e = cudaMemcpy(out, d_out, (size_t)nm * np * 2 * sizeof(double), cudaMemcpyDeviceToHost);

@@ -315,8 +315,10 @@ cudaError_t launch_phases(const double* d_v, long long s_series, long long s_sam
                           cudaStream_t s);
 
 // Monitor spectra (sj_spectrum.cu): out[monitor][np][re, im] from the
-// monitor buffer mon[sample][n_mon] (n samples, np = 2^floor(log2 n)).
-cudaError_t launch_spectrum(const double* d_mon, int n_mon, long long n, long long np, double* d_out, cudaStream_t s);
+// monitor buffer mon[sample][n_mon] (n < 2^31 samples, np = 2^floor(log2 n));
+// d_table: n entries of scratch.
+cudaError_t launch_spectrum(const double* d_mon, int n_mon, long long n, long long np, double2* d_table, double* d_out,
+                            cudaStream_t s);
 
 // Launch helpers implemented in sj_raster.cu.
 cudaError_t launch_rasterize(const sj_csg_node* d_nodes, const int* d_region_start,

@@ -233,7 +233,7 @@ class Fields:
         out = np.zeros((nm, max(npts, 0), 2), dtype=np.float64)
         self._ck(self.lib.sj_monitor_spectrum(self.handle, inst, out.ctypes.data_as(C.POINTER(C.c_double)),
                                               out.size))
-        return out[..., 0] + 1j * out[..., 1]
+        return out.view(np.complex128)[..., 0]
 
     def dft(self, inst=0):
         """Running DFT sums: complex [dft_probe][freq]."""
@@ -242,7 +242,7 @@ class Fields:
         out = np.zeros((nd, nf, 2), dtype=np.float64)
         self._ck(self.lib.sj_read_dft(self.handle, inst,
                                       out.ctypes.data_as(C.POINTER(C.c_double)), out.size))
-        return out[..., 0] + 1j * out[..., 1]
+        return out.view(np.complex128)[..., 0]
 
     def get_array(self, component, inst=0):
         """Full component array [nz][ny][nx] as float64 (dump_raw)."""
