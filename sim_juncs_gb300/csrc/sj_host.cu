@@ -168,6 +168,7 @@ struct sj_sim {
     int l_zb = 16;
     int l_one_column = 0;              // 1: one column per thread in every tile kernel
     int lean_zb = -1;                  // z-segment length the tile lists were built for
+    int lean_one = 0;                  // l_one_column they were built for
     void* d_tiles = nullptr;           // tile lists of all instances and classes
     std::vector<LeanTiles> ltiles;     // per instance
     std::vector<LeanGroup> lgroups;    // instances sharing tile launches (every instance in one)
@@ -990,7 +991,7 @@ void prepare_fused(sj_sim* sim) {
 // instance's tiles by class, in one device buffer.
 template <typename real>
 void prepare_lean(sj_sim* sim) {
-    if (sim->lean_zb == sim->l_zb && sim->d_tiles) return;
+    if (sim->lean_zb == sim->l_zb && sim->lean_one == sim->l_one_column && sim->d_tiles) return;
     auto& dv = devv<real>(sim);
     std::vector<unsigned> all;
     std::vector<long long> off((size_t)sim->n_inst * LEAN_CLASSES);
@@ -1000,7 +1001,7 @@ void prepare_lean(sj_sim* sim) {
     for (int q = 0; q < sim->n_inst; ++q) {
         if (2 * dv[q].vol >= (1LL << 32))
             fail(SJ_E_INVALID, "grid too large for the fused schedule's 32-bit offsets (use split or tma)");
-        if (lean_classify<real>(dv[q], sim->l_zb, lists) != 0)
+        if (lean_classify<real>(dv[q], sim->l_zb, !sim->l_one_column, lists, sim->ltiles[q].merged) != 0)
             fail(SJ_E_INVALID, "grid too large for the fused schedule's tile codes");
         for (int c = 0; c < LEAN_CLASSES; ++c) {
             off[(size_t)q * LEAN_CLASSES + c] = (long long)all.size();
@@ -1064,6 +1065,7 @@ void prepare_lean(sj_sim* sim) {
     for (int p = 0; p < LEAN_FIX_PASSES; ++p)
         sim->lfix.blk[p] = reinterpret_cast<const int2*>(sim->d_fix) + foff[p];
     sim->lean_zb = sim->l_zb;
+    sim->lean_one = sim->l_one_column;
 }
 
 // Can the fused schedule's tiles run as one queued launch?  FP32, two
@@ -1108,7 +1110,7 @@ const LeanQueue<real>* prepare_queue(sj_sim* sim) {
         sim->queue.tabs = tabs.data();
         sim->q_version = sim->table_version;
         if (sim->q_lists == sim->lists_version) return &sim->queue;  // the items still hold
-        // items: multi-slab tiles of every group, then single-slab, then plain;
+        // items: multi-slab tiles of every group (merged groups: all tiles), then single-slab, then plain;
         // groups of larger grids first, members in order
         std::vector<int> order(ng);
         for (int g = 0; g < ng; ++g) order[g] = g;
@@ -2261,8 +2263,10 @@ int32_t sj_launches_per_step(const sj_sim* sim) {
         std::vector<int2> passes[LEAN_FIX_PASSES];
         LeanFix fx{};
         for (int q = 0; q < sim->n_inst; ++q) {
-            const int r = sim->precision == SJ_F64 ? lean_classify(sim->h64[q], sim->l_zb, lists)
-                                                   : lean_classify(sim->h32[q], sim->l_zb, lists);
+            bool merged;
+            const int r = sim->precision == SJ_F64
+                              ? lean_classify(sim->h64[q], sim->l_zb, !sim->l_one_column, lists, merged)
+                              : lean_classify(sim->h32[q], sim->l_zb, !sim->l_one_column, lists, merged);
             if (r != 0) return -1;
             for (int c = 0; c < LEAN_CLASSES; ++c) lt[q].count[c] = (long long)lists[c].size();
         }

@@ -143,7 +143,7 @@ cudaError_t launch_fused_step(const InstDev<real>* d_insts, int n_inst, DevState
 // of one axis (slab) or of several (multi), or an H source (general).  E
 // sources and polarisations are corrections applied after the tiles.  The
 // plain, slab and multi tiles of a group of instances (LeanGroup) run as one
-// launch per class, blockIdx.y = member; general tiles as one launch per
+// launch per class, or one for all three (LeanTiles::merged), blockIdx.y = member; general tiles as one launch per
 // instance.  A launch carries its descriptor as a kernel parameter.
 enum { LEAN_PLAIN = 0, LEAN_SLAB = 1, LEAN_MULTI = 2, LEAN_GENERAL = 3, LEAN_CLASSES = 4 };
 template <typename real>
@@ -168,10 +168,12 @@ struct LeanGroup {
 struct LeanTiles {
     const unsigned* list[LEAN_CLASSES];
     long long count[LEAN_CLASSES];
+    bool merged;  // the plain and slab tiles are in the multi list, in the order of the grid
 };
 long long lean_items(int nx, int ny, int nz, int zb);  // tiles of one instance
+// two_columns: the two-column bodies may run; -1: grid too large
 template <typename real>
-int lean_classify(const InstDev<real>& I, int zb, std::vector<unsigned>* lists);  // -1: grid too large
+int lean_classify(const InstDev<real>& I, int zb, bool two_columns, std::vector<unsigned>* lists, bool& merged);
 // Correction passes after the tile kernels: E sources (one pass per source
 // slot), then polarisations; blk[b] = (instance, block of that instance).
 constexpr int LEAN_FIX_PASSES = SJ_MAX_SOURCES + 1;

@@ -25,7 +25,8 @@
 //           double-buffered shared plane (one barrier per plane).  Two
 //           columns per thread in FP32 where rows are whole (5 warps per
 //           tile: 4 of row pairs, 1 of halo), else one (10 warps: 8 rows,
-//           2 halo).
+//           2 halo).  In FP32 with whole rows and mostly slab tiles
+//           k_lean_all2 takes every class in one launch (lean_classify).
 //           Compiled per axis set, so the other axes' terms vanish.
 //   general (k_lean_general): an H source in the footprint; also runs the
 //           probe blocks, and its blocks (the only ones that read the step
@@ -1111,6 +1112,22 @@ __device__ __forceinline__ void tile_pair_halo_any(const InstDev<real>& I, int t
 
 
 
+// the body of the tile's slab mask
+template <typename real, int ZB>
+__device__ __forceinline__ void tile_pair_halo_mask(const InstDev<real>& I, int m, int tx, int ty, int tz, bool dry,
+                                                    HaloPlane<real>* sh, unsigned qf) {
+    switch (m) {
+        case 0: tile_pair_halo_any<real, ZB, 0>(I, tx, ty, tz, dry, sh, qf); break;
+        case 1: tile_pair_halo_any<real, ZB, 1>(I, tx, ty, tz, dry, sh, qf); break;
+        case 2: tile_pair_halo_any<real, ZB, 2>(I, tx, ty, tz, dry, sh, qf); break;
+        case 3: tile_pair_halo_any<real, ZB, 3>(I, tx, ty, tz, dry, sh, qf); break;
+        case 4: tile_pair_halo_any<real, ZB, 4>(I, tx, ty, tz, dry, sh, qf); break;
+        case 5: tile_pair_halo_any<real, ZB, 5>(I, tx, ty, tz, dry, sh, qf); break;
+        case 6: tile_pair_halo_any<real, ZB, 6>(I, tx, ty, tz, dry, sh, qf); break;
+        default: tile_pair_halo_any<real, ZB, 7>(I, tx, ty, tz, dry, sh, qf); break;
+    }
+}
+
 // Monitors (every save_span steps, before the step) and running DFT sums, read
 // from buffer `cur`, which no stepping block writes during the launch.
 template <typename real>
@@ -1297,6 +1314,17 @@ k_lean_multi2(const __grid_constant__ LeanTable<real> tab) {
         tile_pair_halo_any<real, ZB, 7>(tab.inst, tx, ty, tz, tab.dry != 0, sh, qf);
 }
 
+// Every tile of a group in the order of the grid (merged lists): one launch
+// for the classes that would read each other's halos from memory again.
+template <typename real, int ZB>
+__global__ void __launch_bounds__(HALO2_THREADS, multi2_minb<real>())
+k_lean_all2(const __grid_constant__ LeanTable<real> tab) {
+    __shared__ HaloPlane<real> sh[2];
+    int tx, ty, tz, m;
+    tile_decode(__ldg(tab.tiles + blockIdx.x), tx, ty, tz, m);
+    tile_pair_halo_mask<real, ZB>(tab.inst, m, tx, ty, tz, tab.dry != 0, sh, blockIdx.y * tab.qvol);
+}
+
 // Plain tiles with two columns per thread (instances whose nx is a multiple
 // of 32): the two-column shared-halo body with no CPML axis, 5 warps per tile.
 template <typename real, int ZB>
@@ -1335,16 +1363,7 @@ k_lean_queue(const __grid_constant__ LeanQueueParams<real> qp, const uint4* __re
         tile_decode(w.z, tx, ty, tz, m);
         const unsigned qf = w.y * st.qvol;
         const bool dry = st.dry != 0;
-        switch (m) {
-            case 0: tile_pair_halo_any<real, ZB, 0>(st.inst, tx, ty, tz, dry, sh, qf); break;
-            case 1: tile_pair_halo_any<real, ZB, 1>(st.inst, tx, ty, tz, dry, sh, qf); break;
-            case 2: tile_pair_halo_any<real, ZB, 2>(st.inst, tx, ty, tz, dry, sh, qf); break;
-            case 3: tile_pair_halo_any<real, ZB, 3>(st.inst, tx, ty, tz, dry, sh, qf); break;
-            case 4: tile_pair_halo_any<real, ZB, 4>(st.inst, tx, ty, tz, dry, sh, qf); break;
-            case 5: tile_pair_halo_any<real, ZB, 5>(st.inst, tx, ty, tz, dry, sh, qf); break;
-            case 6: tile_pair_halo_any<real, ZB, 6>(st.inst, tx, ty, tz, dry, sh, qf); break;
-            default: tile_pair_halo_any<real, ZB, 7>(st.inst, tx, ty, tz, dry, sh, qf); break;
-        }
+        tile_pair_halo_mask<real, ZB>(st.inst, m, tx, ty, tz, dry, sh, qf);
     }
 }
 
@@ -1547,7 +1566,7 @@ long long lean_items(int nx, int ny, int nz, int zb) {
 }
 
 template <typename real>
-int lean_classify(const InstDev<real>& I, int zb, std::vector<unsigned>* lists) {
+int lean_classify(const InstDev<real>& I, int zb, bool two_columns, std::vector<unsigned>* lists, bool& merged) {
     const int ntx = (I.nx + LX - 1) / LX, nty = (I.ny + LY - 1) / LY, ntz = (I.nz + zb - 1) / zb;
     if (ntx > 512 || nty > 1024 || ntz > 1024) return -1;
     for (int c = 0; c < LEAN_CLASSES; ++c) lists[c].clear();
@@ -1562,10 +1581,29 @@ int lean_classify(const InstDev<real>& I, int zb, std::vector<unsigned>* lists) 
                                                              : LEAN_MULTI;
                 lists[c].push_back((unsigned)tx | ((unsigned)ty << 9) | ((unsigned)tz << 19) | ((unsigned)m << 29));
             }
+    // Classes launched one after another read the rows, planes and sectors
+    // that a tile shares with neighbours of another class from memory again
+    // (1.2 times the algorithmic bytes on 192^3 sweep members).  Where most
+    // tiles touch a slab, one launch takes them all in the order of the grid:
+    // 32 x 96^3 597 -> 535 us per step, 32 x 128^3 1220 -> 1158, 32 x 192^3
+    // 3790 -> 3515 (5.1 TB/s of algorithmic bytes).  It holds every tile to the CPML bodies' registers, so
+    // grids of mostly plain tiles keep the classes (bowtie, 56% plain: 1320 us
+    // against 1349; 192^3 on quartz, 61%: 702 against 700).
+    const size_t n = lists[LEAN_PLAIN].size() + lists[LEAN_SLAB].size() + lists[LEAN_MULTI].size();
+    merged = sizeof(real) == 4 && two_columns && I.nx % LX == 0 && 2 * lists[LEAN_PLAIN].size() <= n &&
+             lists[LEAN_MULTI].size() < n;
+    if (merged) {
+        std::vector<unsigned>& all = lists[LEAN_MULTI];
+        for (int c : {LEAN_PLAIN, LEAN_SLAB}) {
+            all.insert(all.end(), lists[c].begin(), lists[c].end());
+            lists[c].clear();
+        }
+        std::sort(all.begin(), all.end(), [](unsigned a, unsigned b) { return (a & 0x1fffffffu) < (b & 0x1fffffffu); });
+    }
     return 0;
 }
-template int lean_classify<float>(const InstDev<float>&, int, std::vector<unsigned>*);
-template int lean_classify<double>(const InstDev<double>&, int, std::vector<unsigned>*);
+template int lean_classify<float>(const InstDev<float>&, int, bool, std::vector<unsigned>*, bool&);
+template int lean_classify<double>(const InstDev<double>&, int, bool, std::vector<unsigned>*, bool&);
 
 namespace {
 
@@ -1716,8 +1754,12 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
     case Z:                                                                                                  \
         t.tiles = T.list[LEAN_MULTI], t.n_tiles = T.count[LEAN_MULTI];                                       \
         if constexpr (sizeof(real) == 4)                                                                     \
-            if (t.n_tiles && pairs2)                                                                         \
-                k_lean_multi2<real, Z><<<dim3((unsigned)t.n_tiles, gn), halo2, 0, sc[LEAN_MULTI]>>>(t);      \
+            if (t.n_tiles && pairs2) {                                                                       \
+                if (T.merged)                                                                                \
+                    k_lean_all2<real, Z><<<dim3((unsigned)t.n_tiles, gn), halo2, 0, sc[LEAN_MULTI]>>>(t);    \
+                else                                                                                         \
+                    k_lean_multi2<real, Z><<<dim3((unsigned)t.n_tiles, gn), halo2, 0, sc[LEAN_MULTI]>>>(t);  \
+            }                                                                                                \
         if (t.n_tiles && !pairs2)                                                                            \
             k_lean_multi<real, Z><<<dim3((unsigned)t.n_tiles, gn), halo, 0, sc[LEAN_MULTI]>>>(t);            \
         t.tiles = T.list[LEAN_SLAB], t.n_tiles = T.count[LEAN_SLAB];                                         \

@@ -41,7 +41,19 @@ def batch():
             ((64, 20.0, 0.3, 2.0), (40, 12.5, 1.7, 0.5), (64, 20.0, 4.0, 1.0))]
 
 
-CASES = {"odd_box": odd_box, "whole_slab": whole_slab, "many_probes": many_probes, "batch": batch,
+def mostly_plain():
+    """Rows of whole tiles and mostly plain tiles: the tile launches keep their classes (elsewhere here they merge)."""
+    inst = junction_instance(n=96, res=30.0)
+    inst.grid = Grid(128, 24, 128, inst.grid.dx, inst.grid.dt)
+    inst.pml = PML([[0.1, 0.0], [0.0, 0.0], [0.1, 0.1]])
+    src = inst.sources[0]
+    src.start_time, src.end_time = -9.0, 11.0
+    src.lo, src.hi = (0.0, 0.0, 1.7), (4.3, 0.8, 1.7)
+    inst.probes = [Probe(c, (2.0, 0.4, z), dft=True) for c in (0, 4) for z in (0.05, 2.0)]
+    return [inst]
+
+
+CASES = {"mostly_plain": mostly_plain, "odd_box": odd_box, "whole_slab": whole_slab, "many_probes": many_probes, "batch": batch,
          "quartz": lambda: [inverse_design_case(0, n=72)[0]], "junction65": lambda: [junction_instance(n=65, res=20.0)]}
 
 
