@@ -987,6 +987,18 @@ void prepare_fused(sj_sim* sim) {
     sim->fused_ready = true;
 }
 
+// The instances of every launch group, in the groups' order (a packed group
+// may have split into runs).
+std::vector<std::vector<int>> launch_members(const sj_sim* sim) {
+    std::vector<std::vector<int>> out;
+    for (const LeanGroup& g : sim->lgroups)
+        for (const auto& mem : sim->lmembers) {
+            const auto it = std::find(mem.begin(), mem.end(), g.lead);
+            if (it != mem.end()) out.emplace_back(it, it + g.n);
+        }
+    return out;
+}
+
 // Tile lists of the fused schedule for the current z-segment length: every
 // instance's tiles by class, in one device buffer.
 template <typename real>
@@ -1052,12 +1064,11 @@ void prepare_lean(sj_sim* sim) {
     sim->lgen.blk = reinterpret_cast<const int4*>(sim->d_gen);
     // correction passes (independent of the tiling)
     std::vector<int2> passes[LEAN_FIX_PASSES];
-    lean_fix_blocks<real>(dv.data(), sim->n_inst, passes, sim->lfix.per);
+    lean_fix_blocks<real>(dv.data(), launch_members(sim), passes, sim->lfix);
     std::vector<int2> fall;
     long long foff[LEAN_FIX_PASSES];
     for (int p = 0; p < LEAN_FIX_PASSES; ++p) {
         foff[p] = (long long)fall.size();
-        sim->lfix.count[p] = (long long)passes[p].size();
         fall.insert(fall.end(), passes[p].begin(), passes[p].end());
     }
     sim->dfree(sim->d_fix);
@@ -2268,13 +2279,13 @@ int32_t sj_launches_per_step(const sj_sim* sim) {
                               ? lean_classify(sim->h64[q], sim->l_zb, !sim->l_one_column, lists, merged)
                               : lean_classify(sim->h32[q], sim->l_zb, !sim->l_one_column, lists, merged);
             if (r != 0) return -1;
+            lt[q].merged = merged;
             for (int c = 0; c < LEAN_CLASSES; ++c) lt[q].count[c] = (long long)lists[c].size();
         }
         if (sim->precision == SJ_F64)
-            lean_fix_blocks(sim->h64.data(), sim->n_inst, passes, fx.per);
+            lean_fix_blocks(sim->h64.data(), launch_members(sim), passes, fx);
         else
-            lean_fix_blocks(sim->h32.data(), sim->n_inst, passes, fx.per);
-        for (int p = 0; p < LEAN_FIX_PASSES; ++p) fx.count[p] = (long long)passes[p].size();
+            lean_fix_blocks(sim->h32.data(), launch_members(sim), passes, fx);
         const LeanGroup* lg = sim->lgroups.data();
         const int ng = (int)sim->lgroups.size();
         sj_sim* ms = const_cast<sj_sim*>(sim);
@@ -2282,7 +2293,7 @@ int32_t sj_launches_per_step(const sj_sim* sim) {
             ng <= LEAN_QUEUE_GROUPS) {
             // one queued launch for every group's plain, slab and multi tiles
             int total = 1;
-            for (int p = 0; p < LEAN_FIX_PASSES; ++p) total += fx.count[p] > 0;
+            for (int p = 0; p < LEAN_FIX_PASSES; ++p) total += fx.first[p].back() > 0;
             for (int q = 0; q < sim->n_inst; ++q)
                 if (lt[q].count[LEAN_PLAIN] + lt[q].count[LEAN_SLAB] + lt[q].count[LEAN_MULTI] > 0) return total + 1;
             return total;

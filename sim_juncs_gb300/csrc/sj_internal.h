@@ -179,11 +179,12 @@ int lean_classify(const InstDev<real>& I, int zb, bool two_columns, std::vector<
 constexpr int LEAN_FIX_PASSES = SJ_MAX_SOURCES + 1;
 struct LeanFix {
     const int2* blk[LEAN_FIX_PASSES];
-    long long count[LEAN_FIX_PASSES];
-    int per[LEAN_FIX_PASSES];  // cells per thread
+    std::vector<long long> first[LEAN_FIX_PASSES];  // [group] first block, groups in launch order; then the total
+    int per[LEAN_FIX_PASSES];                       // cells per thread
 };
 template <typename real>
-void lean_fix_blocks(const InstDev<real>* h_insts, int n_inst, std::vector<int2>* passes, int* per);
+void lean_fix_blocks(const InstDev<real>* h_insts, const std::vector<std::vector<int>>& groups,
+                     std::vector<int2>* passes, LeanFix& fix);
 // The general launch of a step: one block per H-source tile and per probe
 // block of every instance.  blk[b] = (instance, 0, tile code) or (instance,
 // 1, probe chunk); the tiles come first, so a dry launch takes the first

@@ -1404,8 +1404,8 @@ k_lean_general(const InstDev<real>* __restrict__ parity_tab, const int4* __restr
 }
 
 // ------------------------------------------------------------ corrections
-// After the tile kernels of a step, on the caller's stream and in this
-// order: one k_lean_esrc launch per source slot s (the instances whose
+// After the tile kernels of a step (of a merged group: of the group, on its
+// stream), in this order: one k_lean_esrc launch per source slot s (the instances whose
 // source s is an E source), then one k_lean_disp launch (the instances with
 // dispersive voxels).  Block b takes per * FIX_THREADS cells of one instance's
 // box: blk[b] = (instance, block of that instance).  Descriptors come from the
@@ -1620,9 +1620,30 @@ long long general_blocks(const LeanGen& gen, int dry) {
 
 }  // namespace
 
+// A merged group without general tiles has one tile launch, so its
+// corrections need nothing else: they follow it on its stream, under the
+// other groups' tiles, instead of after the join of all (four
+// members of each sweep size, graph replays: 692 -> 679 us per step; the
+// 96-member sweep 5095 -> 5064).
+static bool fixed_early(const LeanTiles& t) { return t.merged && t.count[LEAN_GENERAL] == 0; }
+
+// Runs of groups whose corrections go out together: f(first, last, early)
+template <typename F>
+static void fix_runs(const LeanTiles* tiles, const LeanGroup* groups, int n_groups, bool split, F f) {
+    for (int g = 0; g < n_groups;) {
+        const bool early = split && fixed_early(tiles[groups[g].lead]);
+        int e = g + 1;
+        while (!early && e < n_groups && !(split && fixed_early(tiles[groups[e].lead]))) ++e;
+        f(g, e, early);
+        g = e;
+    }
+}
+
 int lean_launches(const LeanTiles* tiles, const LeanGroup* groups, int n_groups, const LeanFix& fix) {
     int total = 1;  // the general launch
-    for (int p = 0; p < LEAN_FIX_PASSES; ++p) total += fix.count[p] > 0;
+    fix_runs(tiles, groups, n_groups, true, [&](int g, int e, bool) {
+        for (int p = 0; p < LEAN_FIX_PASSES; ++p) total += fix.first[p][e] > fix.first[p][g];
+    });
     for (int g = 0; g < n_groups; ++g)
         for (int c = 0; c < LEAN_CLASSES; ++c)
             if (c != LEAN_GENERAL && tiles[groups[g].lead].count[c] > 0) ++total;
@@ -1656,7 +1677,8 @@ int fix_per(long long cells, int most) {
 }
 
 template <typename real>
-void lean_fix_blocks(const InstDev<real>* h_insts, int n_inst, std::vector<int2>* passes, int* per) {
+void lean_fix_blocks(const InstDev<real>* h_insts, const std::vector<std::vector<int>>& groups,
+                     std::vector<int2>* passes, LeanFix& fix) {
     auto cells_of = [&](int q, int p) -> long long {  // cells of pass p in instance q
         const InstDev<real>& I = h_insts[q];
         if (p == SJ_MAX_SOURCES) return I.n_poles > 0 ? I.dvol : 0;
@@ -1666,18 +1688,25 @@ void lean_fix_blocks(const InstDev<real>* h_insts, int n_inst, std::vector<int2>
     for (int p = 0; p < LEAN_FIX_PASSES; ++p) {
         passes[p].clear();
         long long total = 0;
-        for (int q = 0; q < n_inst; ++q) total += cells_of(q, p);
-        per[p] = fix_per(total, p == SJ_MAX_SOURCES ? 16 : 8);
-        for (int q = 0; q < n_inst; ++q)
-            for (long long b = 0; b * per[p] * FIX_THREADS < cells_of(q, p); ++b) passes[p].push_back(make_int2(q, (int)b));
+        for (const auto& g : groups)
+            for (int q : g) total += cells_of(q, p);
+        const int per = fix.per[p] = fix_per(total, p == SJ_MAX_SOURCES ? 16 : 8);
+        fix.first[p].assign(1, 0);
+        for (const auto& g : groups) {
+            for (int q : g)
+                for (long long b = 0; b * per * FIX_THREADS < cells_of(q, p); ++b) passes[p].push_back(make_int2(q, (int)b));
+            fix.first[p].push_back((long long)passes[p].size());
+        }
     }
 }
-template void lean_fix_blocks<float>(const InstDev<float>*, int, std::vector<int2>*, int*);
-template void lean_fix_blocks<double>(const InstDev<double>*, int, std::vector<int2>*, int*);
+template void lean_fix_blocks<float>(const InstDev<float>*, const std::vector<std::vector<int>>&, std::vector<int2>*,
+                                     LeanFix&);
+template void lean_fix_blocks<double>(const InstDev<double>*, const std::vector<std::vector<int>>&, std::vector<int2>*,
+                                      LeanFix&);
 
-// Each class of instance q goes to its own stream of set q % LEAN_SETS: the
-// kernels of a step overlap and fill each other's tails.  Only as many sets
-// as there are instances are forked.
+// Each class of group g goes to its own stream of set g % LEAN_SETS: the
+// kernels of a step overlap and fill each other's tails.  Only streams that
+// get a launch are forked and joined.
 template <typename real>
 cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* d_insts,
                              const InstDev<real>* d_parity, const LeanTiles* tiles, const LeanGroup* groups,
@@ -1686,16 +1715,24 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
                              const LeanQueue<real>* queue) {
     cudaError_t e = cudaSuccess;
     const bool fork = ls.side[0] != nullptr;
-    const int nsets = fork ? (queue ? 1 : std::min(std::max(n_groups, 1), LEAN_SETS)) : 0;
     if (fork) {
         e = cudaEventRecord(ls.fork, ls.main);
-        for (int q = 0; q < nsets * LEAN_CLASSES && e == cudaSuccess; ++q)
-            e = cudaStreamWaitEvent(ls.side[q], ls.fork, 0);
         if (e != cudaSuccess) return e;
     }
+    // the stream of class c of set s, forked from main at its first use
+    bool used[LEAN_STREAMS] = {};
+    auto stream = [&](int s, int c) {
+        if (!fork) return ls.main;
+        const int q = (s % LEAN_SETS) * LEAN_CLASSES + c;
+        if (!used[q]) {
+            used[q] = true;
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(ls.side[q], ls.fork, 0);
+        }
+        return ls.side[q];
+    };
     const long long gb = general_blocks(gen, dry);
     long long gtotal = gb;
-    for (int p = 0; p < LEAN_FIX_PASSES; ++p) gtotal += fix.count[p];
+    for (int p = 0; p < LEAN_FIX_PASSES; ++p) gtotal += fix.first[p].back();
     const dim3 block(LX, LY), halo(LX, LY + HALO_WARPS), halo2(LX, LY / 2 + 1);
     // descriptor of instance q with the step's parity applied
     auto table = [&](int q) {
@@ -1710,26 +1747,37 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
         t.qvol = (unsigned)h_insts[q].vol;
         return t;
     };
-    auto set_streams = [&](int s, cudaStream_t* sc) {
-        for (int c = 0; c < LEAN_CLASSES; ++c) sc[c] = fork ? ls.side[(s % LEAN_SETS) * LEAN_CLASSES + c] : ls.main;
+    // groups [g, g2): every correction pass, on stream s
+    auto fixes = [&](int g, int g2, cudaStream_t s) {
+        for (int p = 0; p < LEAN_FIX_PASSES && e == cudaSuccess; ++p) {
+            const long long b = fix.first[p][g];
+            const unsigned nb = (unsigned)(fix.first[p][g2] - b);
+            if (!nb) continue;
+            if (p < SJ_MAX_SOURCES)
+                k_lean_esrc<real><<<nb, FIX_THREADS, 0, s>>>(d_insts, fix.blk[p] + b, fix.per[p], p, cur, (unsigned)gtotal,
+                                                             dry, st);
+            else
+                k_lean_disp<real><<<nb, FIX_THREADS, 0, s>>>(d_insts, fix.blk[p] + b, fix.per[p], cur, (unsigned)gtotal,
+                                                             dry, st);
+            e = cudaGetLastError();
+        }
     };
     // queued: every group's plain, slab and multi tiles in one launch
     if (queue && queue->n_items) {
-        cudaStream_t sc[LEAN_CLASSES];
-        set_streams(0, sc);
+        const cudaStream_t qs = stream(0, LEAN_MULTI);
         const LeanTable<real>* tabs = queue->tabs + (size_t)(dry ? 2 : 0) * queue->n_groups +
                                       (size_t)cur * queue->n_groups;
         LeanQueueParams<real> qp;
         memset(&qp, 0, sizeof(qp));
         for (int g = 0; g < queue->n_groups && g < LEAN_QUEUE_GROUPS; ++g) qp.t[g] = tabs[g];
-        e = cudaMemsetAsync(queue->ctr, 0, sizeof(unsigned), sc[LEAN_MULTI]);
+        if (e == cudaSuccess) e = cudaMemsetAsync(queue->ctr, 0, sizeof(unsigned), qs);
         const unsigned grid = (unsigned)std::min<long long>(queue->grid, queue->n_items);
         if (e == cudaSuccess) {
             if constexpr (sizeof(real) == 4) {
                 switch (zb) {
-                    case 8: k_lean_queue<real, 8><<<grid, halo2, 0, sc[LEAN_MULTI]>>>(qp, queue->items, queue->n_items, queue->ctr); break;
-                    case 16: k_lean_queue<real, 16><<<grid, halo2, 0, sc[LEAN_MULTI]>>>(qp, queue->items, queue->n_items, queue->ctr); break;
-                    case 32: k_lean_queue<real, 32><<<grid, halo2, 0, sc[LEAN_MULTI]>>>(qp, queue->items, queue->n_items, queue->ctr); break;
+                    case 8: k_lean_queue<real, 8><<<grid, halo2, 0, qs>>>(qp, queue->items, queue->n_items, queue->ctr); break;
+                    case 16: k_lean_queue<real, 16><<<grid, halo2, 0, qs>>>(qp, queue->items, queue->n_items, queue->ctr); break;
+                    case 32: k_lean_queue<real, 32><<<grid, halo2, 0, qs>>>(qp, queue->items, queue->n_items, queue->ctr); break;
                     default: return cudaErrorInvalidValue;
                 }
                 e = cudaGetLastError();
@@ -1749,7 +1797,7 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
         // two-column bodies need 152-168 registers: 2 blocks per SM, slower)
         const bool pairs2 = pairs && sizeof(real) == 4;
         cudaStream_t sc[LEAN_CLASSES];
-        set_streams(g, sc);
+        for (int c = 0; c < LEAN_CLASSES; ++c) sc[c] = c != LEAN_GENERAL && T.count[c] ? stream(g, c) : ls.main;
 #define SJ_ZB(Z)                                                                                             \
     case Z:                                                                                                  \
         t.tiles = T.list[LEAN_MULTI], t.n_tiles = T.count[LEAN_MULTI];                                       \
@@ -1785,13 +1833,12 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
     }
     // general tiles (H sources) and probe blocks of all instances: one launch
     if (e == cudaSuccess) {
-        cudaStream_t sc[LEAN_CLASSES];
-        set_streams(0, sc);
+        const cudaStream_t gs = stream(0, LEAN_GENERAL);
         const long long nb = dry ? gen.n_tiles : gen.n_all;
         switch (zb) {
 #define SJ_GEN(Z)                                                                                       \
     case Z:                                                                                             \
-        k_lean_general<real, Z><<<(unsigned)gb, block, 0, sc[LEAN_GENERAL]>>>(d_parity, gen.blk, nb, n_inst, \
+        k_lean_general<real, Z><<<(unsigned)gb, block, 0, gs>>>(d_parity, gen.blk, nb, n_inst, \
                                                                              cur, dry, (unsigned)gtotal, st); \
         break;
             SJ_GEN(8)
@@ -1802,22 +1849,18 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
         }
         e = cudaGetLastError();
     }
-    if (fork) {
-        for (int q = 0; q < nsets * LEAN_CLASSES && e == cudaSuccess; ++q) {
-            e = cudaEventRecord(ls.join[q], ls.side[q]);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(ls.main, ls.join[q], 0);
-        }
+    const bool split = fork && !queue;
+    fix_runs(tiles, groups, n_groups, split, [&](int g, int g2, bool early) {
+        if (early) fixes(g, g2, stream(g, LEAN_MULTI));
+    });
+    for (int q = 0; q < LEAN_STREAMS && e == cudaSuccess; ++q) {
+        if (!used[q]) continue;
+        e = cudaEventRecord(ls.join[q], ls.side[q]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ls.main, ls.join[q], 0);
     }
-    for (int p = 0; p < LEAN_FIX_PASSES && e == cudaSuccess; ++p) {
-        if (!fix.count[p]) continue;
-        const unsigned nb = (unsigned)fix.count[p];
-        if (p < SJ_MAX_SOURCES)
-            k_lean_esrc<real><<<nb, FIX_THREADS, 0, ls.main>>>(d_insts, fix.blk[p], fix.per[p], p, cur, (unsigned)gtotal,
-                                                               dry, st);
-        else
-            k_lean_disp<real><<<nb, FIX_THREADS, 0, ls.main>>>(d_insts, fix.blk[p], fix.per[p], cur, (unsigned)gtotal, dry, st);
-        e = cudaGetLastError();
-    }
+    fix_runs(tiles, groups, n_groups, split, [&](int g, int g2, bool early) {
+        if (!early) fixes(g, g2, ls.main);
+    });
     return e;
 }
 
