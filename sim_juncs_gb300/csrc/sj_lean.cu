@@ -1565,6 +1565,8 @@ long long lean_items(int nx, int ny, int nz, int zb) {
     return (long long)((nx + LX - 1) / LX) * ((ny + LY - 1) / LY) * ((nz + zb - 1) / zb);
 }
 
+constexpr int LEAN_MERGE_LAYER = 5 * 152;  // tiles of a merged launch that are resident at once
+
 template <typename real>
 int lean_classify(const InstDev<real>& I, int zb, bool two_columns, std::vector<unsigned>* lists, bool& merged) {
     const int ntx = (I.nx + LX - 1) / LX, nty = (I.ny + LY - 1) / LY, ntz = (I.nz + zb - 1) / zb;
@@ -1583,15 +1585,19 @@ int lean_classify(const InstDev<real>& I, int zb, bool two_columns, std::vector<
             }
     // Classes launched one after another read the rows, planes and sectors
     // that a tile shares with neighbours of another class from memory again
-    // (1.2 times the algorithmic bytes on 192^3 sweep members).  Where most
-    // tiles touch a slab, one launch takes them all in the order of the grid:
-    // 32 x 96^3 597 -> 535 us per step, 32 x 128^3 1220 -> 1158, 32 x 192^3
-    // 3790 -> 3515 (5.1 TB/s of algorithmic bytes).  It holds every tile to the CPML bodies' registers, so
-    // grids of mostly plain tiles keep the classes (bowtie, 56% plain: 1320 us
-    // against 1349; 192^3 on quartz, 61%: 702 against 700).
+    // (1.2 times the algorithmic bytes on 192^3 sweep members).  Where at least
+    // half of the tiles touch a slab, one launch takes them all in the order of
+    // the grid: 32 x 96^3 597 -> 535 us per step, 32 x 128^3 1220 -> 1158, 32 x
+    // 192^3 3790 -> 3515 (5.1 TB/s of algorithmic bytes); 4 x 192^3 with slabs
+    // of 15 cells (46% plain) 676 -> 669.  It holds every tile to the CPML
+    // bodies' registers (5 blocks per SM, plain tiles alone 8), so grids of
+    // mostly plain tiles keep the classes (384 x 384 x 288, 54%: 568 us against
+    // 575), and so do those whose layer of tiles is more than is resident at
+    // once, whose neighbours in z then follow late either way (512 x 512 x 384,
+    // 47%: 1298 against 1321).
     const size_t n = lists[LEAN_PLAIN].size() + lists[LEAN_SLAB].size() + lists[LEAN_MULTI].size();
     merged = sizeof(real) == 4 && two_columns && I.nx % LX == 0 && 2 * lists[LEAN_PLAIN].size() <= n &&
-             lists[LEAN_MULTI].size() < n;
+             ntx * nty <= LEAN_MERGE_LAYER && lists[LEAN_MULTI].size() < n;
     if (merged) {
         std::vector<unsigned>& all = lists[LEAN_MULTI];
         for (int c : {LEAN_PLAIN, LEAN_SLAB}) {
