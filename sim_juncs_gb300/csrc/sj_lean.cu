@@ -1725,10 +1725,13 @@ cudaError_t launch_lean_step(const InstDev<real>* h_insts, const InstDev<real>* 
         e = cudaEventRecord(ls.fork, ls.main);
         if (e != cudaSuccess) return e;
     }
-    // the stream of class c of set s, forked from main at its first use
+    // the stream of class c of set s, forked from main at its first use; the
+    // first group's multi-slab (or merged) tiles stay on main, which saves a
+    // step's longest chain the event at either end (512 x 512 x 384 bowtie as
+    // plain launches 1312 -> 1302 us, 256 x 256 x 192 replayed 226 -> 221)
     bool used[LEAN_STREAMS] = {};
     auto stream = [&](int s, int c) {
-        if (!fork) return ls.main;
+        if (!fork || (s == 0 && c == LEAN_MULTI)) return ls.main;
         const int q = (s % LEAN_SETS) * LEAN_CLASSES + c;
         if (!used[q]) {
             used[q] = true;
