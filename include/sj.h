@@ -284,7 +284,8 @@ int32_t sj_get_schedule(const sj_sim* sim);
 int sj_synchronize(sj_sim* sim);
 
 /* tiling of the single-pass schedules.  FUSED: blocks of 32 x 8 columns
-   march z segments of zseg in {8, 16, 32} planes (tile_y, ring ignored).
+   march z segments of zseg in {8, 16, 32} planes (tile_y, ring ignored; 8
+   until set where 16 would give fewer than 3200 tiles, else 16).
    TMA: tiles of 32 x tile_y cells, a TMA ring of `ring` planes
    ((tile_y, ring) in {(4,3), (8,3), (16,3), (4,4), (8,4)}), z segments of
    zseg planes.  Applies to the schedule selected when it is called.  FUSED
@@ -318,7 +319,7 @@ int sj_autotune(sj_sim* sim, int32_t steps, int32_t* tile_y, int32_t* ring, int3
 /* n_steps iterations of the loop body at src/disp.cpp:719-741: sample
    monitors when step % save_span == 0, accumulate DFTs, then fields.step().
    Asynchronous on the sim's stream.  FUSED with its default launch settings:
-   on small grids (all instances together at most 2^23 cells in FP32, 2^25 in
+   on small grids (all instances together at most 2^22 cells in FP32, 2^27 in
    FP64) a call of two or more steps is one cooperative launch per 256 steps,
    with the tile launches' bits; sj_adjoint_gradient and sj_objective run
    forward the same way. */

@@ -1349,13 +1349,14 @@ void take_snapshot_async(sj_sim* sim, int q) {
 }
 
 // Most cells (all instances) that run through the resident kernel.  Measured,
-// us per step, resident against tile launches (zseg 16): FP32 64^3 9.1 / 72,
-// 128^3 44 / 119, 192^3 157 / 184, 4 x 128^3 (2^23) 208 / 244, 256 x 256 x
-// 192 272 / 254 (the two-pass traffic leaves L2); FP64, whose bound is the
-// FP64 pipe and which gains from the missing halo work, 64^3 27 / 124, 192^3
-// 540 / 684, 256 x 256 x 192 879 / 1005, 384 x 384 x 288 (42M) 2936 / 2956.
+// us per step, resident against tile launches (graph replays at the default z
+// segment): FP32 64^3 9.1 / 49, 128^3 44 / 70, 160^3 (4.1M) 101 / 102, 2 x 128^3
+// (2^22) 107 / 105, 5 x 96^3 118 / 113, 192^3 165 / 144 (its two passes leave
+// L2).  FP64, whose bound is the FP64 pipe and which gains from the missing
+// halo work: 64^3 26 / 85, 192^3 512 / 680, 256 x 256 x 192 802 / 974, 320^3
+// 2322 / 2662, 512 x 512 x 384 (101M, two passes over HBM) 6501 / 6921.
 template <typename real>
-constexpr long long res_max_voxels() { return sizeof(real) == 4 ? 1LL << 23 : 1LL << 25; }
+constexpr long long res_max_voxels() { return sizeof(real) == 4 ? 1LL << 22 : 1LL << 27; }
 constexpr int RES_CHUNK = 256;                                // steps per launch
 constexpr unsigned long long RES_WAIT_NS = 4000000000ull;     // limit of a wait at the grid barrier
 
@@ -1372,7 +1373,7 @@ bool resident(sj_sim* sim) {
     }
     if (cells > res_max_voxels<real>()) return false;
     if (sim->r_blocks < 0) {
-        sim->r_blocks = resident_grid<real>(sim->n_inst);
+        sim->r_blocks = resident_grid<real>(devv<real>(sim).data(), sim->n_inst);
         if (sim->r_blocks > 0) sim->d_bar = (unsigned*)sim->dalloc(sizeof(unsigned));
     }
     return sim->r_blocks > 0;
@@ -1724,7 +1725,7 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
         o.D = (double2*)tmp((size_t)o.n_cells * 3 * sizeof(double2), true);
     }
     // small grids run forward through the resident kernel, the objective's sums in blocks of its own
-    const int obj_blocks = resident_objective_blocks<real>(O.data(), ni);
+    const int obj_blocks = resident_objective_blocks<real>(dv.data(), O.data(), ni);
     const bool res = resident<real>(sim) && obj_blocks <= sim->r_blocks / 4;
     ObjDev<real>* d_obj = nullptr;
     if (res) {
@@ -1958,6 +1959,13 @@ void create_t(sj_sim* sim, int n, const sj_instance_desc* insts) {
     }
     sim->snaps.assign(n, Snapshots{});
     group_instances<real>(sim);
+    // z segments of 8 planes where 16 would leave few waves of tiles, each a
+    // serial march (192^3, 1728 tiles of 16: 144 us per step against 161; 2 x
+    // 192^3, 3456: 264 / 276; 3 x 192^3, 5184: 374 / 382, but 24 x 96^3, as
+    // many, 431 / 417)
+    long long tiles16 = 0;
+    for (const InstDev<real>& I : dv) tiles16 += lean_items(I.nx, I.ny, I.nz, 16);
+    sim->l_zb = tiles16 < 3200 ? 8 : 16;
     upload_table<real>(sim);
 }
 

@@ -293,9 +293,9 @@ cudaError_t launch_objective(const ObjDev<real>* o, int n_inst, int cur, long lo
 // the launch.
 constexpr int RES_MAX_INST = 32;  // instances of one resident launch
 template <typename real>
-int resident_grid(int n_inst);
+int resident_grid(const InstDev<real>* h_insts, int n_inst);
 template <typename real>
-int resident_objective_blocks(const ObjDev<real>* o, int n_inst);
+int resident_objective_blocks(const InstDev<real>* h_insts, const ObjDev<real>* o, int n_inst);
 template <typename real>
 cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d_insts, int n_inst, int cur,
                             int n_steps, int max_blocks, const ObjDev<real>* d_obj, int obj_blocks, unsigned* d_bar,

@@ -10,11 +10,11 @@
 // The cell's arithmetic is the tile kernels', operation for operation, so
 // the bits are theirs (this file too is compiled with contraction off).
 //
-// FP32 is bound by latency up to about 64^3 (36^3 8.5 us per step, 64^3 9.1: two
+// FP32 is bound by latency up to about 64^3 (36^3 7.9 us per step, 64^3 9.1: two
 // L2 round trips and two barriers; 72 us as tile launches) and by L2 above.
 // FP64 is bound by the FP64 pipe (19 cycles per warp instruction and SM):
-// 64^3 27 us per step (124 as tile launches), of which 17 are its 35 FP64
-// operations per cell.
+// 64^3 26 us per step (124 as tile launches), of which 17 are its 35 FP64
+// operations per cell; 256 x 256 x 192 802 us, of which 720.
 //
 // Cells are dealt out by their linear index over nx*ny*nz, so odd rows leave
 // no idle lanes.  Probes have blocks of their own: E probes of step n are
@@ -30,27 +30,22 @@ namespace sj {
 namespace {
 
 constexpr int RES_MAXF = 256;
-#ifndef SJ_RES_THREADS32
-#define SJ_RES_THREADS32 1024
-#endif
-#ifndef SJ_RES_CHUNK32
-#define SJ_RES_CHUNK32 1024
-#endif
-#ifndef SJ_RES_CHUNK64
-#define SJ_RES_CHUNK64 32
-#endif
-
-// FP32: 1024 threads of 64 registers hide latency better than 512 of 96
-// (96^3 18.4 us per step against 23.7; 36^3 8.6 against 9.7 is the price)
+// Threads of a block, by the cells of the launch.  More warps hide more latency
+// and keep the FP64 pipe busier at a phase's ends, on few cells they only add
+// to the barrier: us per step of 36^3, 48^3, 64^3, 128^3, 192^3
+//   FP64  512 threads  13.2 15.0 27.4 168 537;  768  16.8 16.6 26.4 165 512
+//         (256 x 256 x 192 bowtie 875 and 802)
+//   FP32  512 threads  7.9 7.6 11.2 63.8 249;  1024  8.6 8.3 9.2 44.7 166
 template <typename real>
-constexpr int res_threads() { return sizeof(real) == 4 ? SJ_RES_THREADS32 : 512; }
+constexpr int res_threads(bool few) { return few ? 512 : (sizeof(real) == 4 ? 1024 : 768); }
+constexpr long long RES_FEW_CELLS = 1 << 18;  // fewer cells than this: the small blocks
 
 // A block takes its cells in chunks of this many consecutive ones, dealt out
 // over the blocks in turn.  FP64 is bound by the FP64 pipe of each SM, so its
 // chunks are one warp's (the SMs' shares differ by one: 64^3 27.3 us per step,
 // 29.9 with 256); FP32's are the block's, whose rows share L1 lines.
-template <typename real>
-constexpr int res_chunk() { return sizeof(real) == 4 ? SJ_RES_CHUNK32 : SJ_RES_CHUNK64; }
+template <typename real, int T>
+constexpr int res_chunk() { return sizeof(real) == 4 ? T : 32; }
 
 // What a block knows of one instance besides its descriptor.  FP64 deals the
 // columns between the x slabs first and the slabs' columns after them: a
@@ -550,14 +545,14 @@ __device__ __noinline__ void res_probe_block(const InstDev<real>* tab, int n_ins
 // ONE: a single instance, its descriptor in the parameter space; else the
 // descriptors are copied to shared memory.  The fields' buffer `cur` is
 // stepped in place.
-template <typename real, bool ONE, bool DES>
-__global__ void __launch_bounds__(res_threads<real>(), 1)
+template <typename real, int T, bool ONE, bool DES>
+__global__ void __launch_bounds__(T, 1)
 k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __restrict__ tab, int n_inst, int cur,
            int n_steps, int workers, int probe_blocks, int h_probes, int one_chunk, const ObjDev<real>* __restrict__ obj,
            unsigned* bar, unsigned long long limit, DevState* st) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ ResGrid grids[RES_MAX_INST];
-    constexpr unsigned CH = res_chunk<real>(), SLOTS = res_threads<real>() / CH;
+    constexpr unsigned CH = res_chunk<real, T>(), SLOTS = T / CH;
     const long long n0 = st->step;
     if ((int)blockIdx.x >= workers) {
         int b = (int)blockIdx.x - workers;
@@ -630,25 +625,38 @@ k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __res
 }  // namespace
 
 namespace {
+template <typename real, int T>
+const void* res_kernel_t(int n_inst, bool des) {
+    if (n_inst > 1)
+        return des ? (const void*)k_resident<real, T, false, true> : (const void*)k_resident<real, T, false, false>;
+    return des ? (const void*)k_resident<real, T, true, true> : (const void*)k_resident<real, T, true, false>;
+}
 template <typename real>
-const void* res_kernel(int n_inst, bool des) {
-    if (n_inst > 1) return des ? (const void*)k_resident<real, false, true> : (const void*)k_resident<real, false, false>;
-    return des ? (const void*)k_resident<real, true, true> : (const void*)k_resident<real, true, false>;
+const void* res_kernel(bool few, int n_inst, bool des) {
+    return few ? res_kernel_t<real, res_threads<real>(true)>(n_inst, des)
+               : res_kernel_t<real, res_threads<real>(false)>(n_inst, des);
+}
+template <typename real>
+bool res_few(const InstDev<real>* h_insts, int n_inst) {
+    long long cells = 0;
+    for (int q = 0; q < n_inst; ++q) cells += (long long)h_insts[q].nx * h_insts[q].ny * h_insts[q].nz;
+    return cells < RES_FEW_CELLS;
 }
 }  // namespace
 
 template <typename real>
-int resident_grid(int n_inst) {
+int resident_grid(const InstDev<real>* h_insts, int n_inst) {
     int dev = 0, sms = 0, coop = 0, least = INT_MAX;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (!coop) return 0;
+    const bool few = res_few(h_insts, n_inst);
     const size_t smem = n_inst > 1 ? (size_t)n_inst * sizeof(InstDev<real>) : 0;
     for (int des = 0; des < 2; ++des) {
         int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, res_kernel<real>(n_inst, des), res_threads<real>(), smem) !=
-            cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, res_kernel<real>(few, n_inst, des), res_threads<real>(few),
+                                                          smem) != cudaSuccess)
             return 0;
         least = std::min(least, nb);
     }
@@ -656,9 +664,10 @@ int resident_grid(int n_inst) {
 }
 
 template <typename real>
-int resident_objective_blocks(const ObjDev<real>* o, int n_inst) {
+int resident_objective_blocks(const InstDev<real>* h_insts, const ObjDev<real>* o, int n_inst) {
+    const int T = res_threads<real>(res_few(h_insts, n_inst));
     int b = 0;
-    for (int q = 0; q < n_inst; ++q) b += (3 * o[q].n_cells + res_threads<real>() - 1) / res_threads<real>();
+    for (int q = 0; q < n_inst; ++q) b += (3 * o[q].n_cells + T - 1) / T;
     return b;
 }
 
@@ -669,7 +678,8 @@ cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d
     long long cells = 0, chunks = 0;
     int h_probes = 0;
     bool des = d_obj != nullptr;
-    const int T = res_threads<real>();
+    const bool few = res_few(h_insts, n_inst);
+    const int T = res_threads<real>(few);
     for (int q = 0; q < n_inst; ++q) {
         const InstDev<real>& I = h_insts[q];
         cells += (long long)I.nx * I.ny * I.nz;
@@ -688,13 +698,14 @@ cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d
     void* args[] = {&one,      &d_insts,   &n_inst, &cur,   &n_steps,  &w, &probe,
                     &h_probes, &one_chunk, &d_obj,  &d_bar, &limit_ns, &st};
     const size_t smem = n_inst > 1 ? (size_t)n_inst * sizeof(InstDev<real>) : 0;
-    return cudaLaunchCooperativeKernel(res_kernel<real>(n_inst, des), dim3(w + probe + obj_blocks), dim3(T), args, smem, s);
+    return cudaLaunchCooperativeKernel(res_kernel<real>(few, n_inst, des), dim3(w + probe + obj_blocks), dim3(T), args,
+                                       smem, s);
 }
 
-template int resident_grid<float>(int);
-template int resident_grid<double>(int);
-template int resident_objective_blocks<float>(const ObjDev<float>*, int);
-template int resident_objective_blocks<double>(const ObjDev<double>*, int);
+template int resident_grid<float>(const InstDev<float>*, int);
+template int resident_grid<double>(const InstDev<double>*, int);
+template int resident_objective_blocks<float>(const InstDev<float>*, const ObjDev<float>*, int);
+template int resident_objective_blocks<double>(const InstDev<double>*, const ObjDev<double>*, int);
 template cudaError_t launch_resident<float>(const InstDev<float>*, const InstDev<float>*, int, int, int, int,
                                             const ObjDev<float>*, int, unsigned*, unsigned long long, DevState*,
                                             cudaStream_t);
