@@ -298,7 +298,8 @@ int sj_get_tiling(const sj_sim* sim, int32_t* tile_y, int32_t* ring, int32_t* zs
    the results do not change. */
 int sj_set_fused_columns(sj_sim* sim, int32_t columns);
 /* FUSED: how a step's tile kernels are launched.  GROUPED (default): one
-   launch per launch group and tile class (plain, single-slab, multi-slab),
+   launch per launch group and tile class (plain, single-slab, multi-slab), or
+   one per group (FP32, mostly CPML tiles),
    the launches of a step concurrent on forked streams.  QUEUE: one launch of
    resident blocks for every group's tiles, which claim (group, member, tile)
    items from a counter, multi-slab tiles first; FP32 with two columns per

@@ -32,8 +32,8 @@
 //           probe blocks, and its blocks (the only ones that read the step
 //           counter) count themselves: the last advances the step.
 // Instances with the same grid, CPML and coefficient table form a group
-// (LeanGroup) whose arrays sit at fixed strides: one launch per class covers
-// the group's tiles (blockIdx.y = member).  The launches of a step go to
+// (LeanGroup) whose arrays sit at fixed strides: one launch per class, or one
+// merged, covers the group's tiles (blockIdx.y = member).  The launches of a step go to
 // streams forked from the caller's, one per class and group set, so they
 // overlap; after they join, small correction kernels add the E sources and
 // the polarisation ADE on their cells only.  All evaluate one update

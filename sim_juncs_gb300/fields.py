@@ -84,8 +84,8 @@ class Fields:
         self._ck(self.lib.sj_set_fused_columns(self.handle, int(columns)))
 
     def set_fused_launch(self, mode):
-        """"grouped" (one launch per group and tile class) or "queue" (one
-        launch of resident blocks claiming every group's tiles)."""
+        """"grouped" (one launch per group, or per group and tile class) or
+        "queue" (one launch of resident blocks claiming every group's tiles)."""
         self._ck(self.lib.sj_set_fused_launch(self.handle, {"grouped": 0, "queue": 1}[mode]))
 
     def fused_launch(self):
