@@ -23,7 +23,8 @@ __device__ __forceinline__ void mat_vec(const double* __restrict__ m, double x, 
 // Which of a node's transforms are the identity: bit 0 the ancestors' (m),
 // bit 1 the primitive's own (t).  At a finite point the product with an
 // identity gives the point back, up to the sign of a zero, which no primitive
-// can tell; the flags are formed once per block.
+// can tell (t's point, r - c, is finite where neither number is near overflow);
+// the flags are formed once per block.
 constexpr int RASTER_MAX_NODES = SJ_MAX_CSG_NODES * SJ_MAX_REGIONS;
 __device__ __forceinline__ bool is_identity(const double* m) {
     bool id = true;
@@ -33,9 +34,13 @@ __device__ __forceinline__ bool is_identity(const double* m) {
     }
     return id;
 }
+constexpr double FAR = 1e307;
 __device__ void identity_flags(const sj_csg_node* __restrict__ nodes, int n, bool finite, uint8_t* flags) {
-    for (int q = threadIdx.x; q < n; q += blockDim.x)
-        flags[q] = finite ? (uint8_t)((is_identity(nodes[q].m) ? 1 : 0) | (is_identity(nodes[q].t) ? 2 : 0)) : 0;
+    for (int q = threadIdx.x; q < n; q += blockDim.x) {
+        const sj_csg_node& nd = nodes[q];
+        const bool centre = fabs(nd.c[0]) < FAR && fabs(nd.c[1]) < FAR && fabs(nd.c[2]) < FAR;
+        flags[q] = finite ? (uint8_t)((is_identity(nd.m) ? 1 : 0) | (centre && is_identity(nd.t) ? 2 : 0)) : 0;
+    }
     __syncthreads();
 }
 
@@ -106,10 +111,12 @@ __device__ int eval_program(const sj_csg_node* __restrict__ nodes, const uint8_t
     return (int)(stk & 1ull);
 }
 
-// every point of the grid has finite coordinates
+// every point of the grid has coordinates below FAR
 static bool finite_grid(int nx, int ny, int nz, double dx, const double* o) {
-    return std::isfinite(o[0]) && std::isfinite(o[1]) && std::isfinite(o[2]) && std::isfinite(o[0] + (nx + 1.0) * dx) &&
-           std::isfinite(o[1] + (ny + 1.0) * dx) && std::isfinite(o[2] + (nz + 1.0) * dx);
+    const int n[3] = {nx, ny, nz};
+    for (int a = 0; a < 3; ++a)
+        if (!(std::fabs(o[a]) < FAR && std::fabs(o[a] + (n[a] + 1.0) * dx) < FAR)) return false;
+    return true;
 }
 
 // Region start table carried by value in the kernel's parameters.
@@ -211,7 +218,7 @@ __global__ void k_rasterize_counts(const sj_csg_node* __restrict__ nodes, const 
                                    unsigned long long* __restrict__ set, unsigned cap, int* __restrict__ overflow) {
     __shared__ uint8_t flags[RASTER_MAX_NODES];
     bool all = finite != 0;
-    for (int q = threadIdx.x; q < 3 * n_offs; q += blockDim.x) all = all && isfinite(offs[q]);
+    for (int q = threadIdx.x; q < 3 * n_offs; q += blockDim.x) all = all && fabs(offs[q]) < FAR;
     identity_flags(nodes, rstart[n_regions], __syncthreads_and(all) != 0, flags);
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long total = (long long)nx * ny * nz;

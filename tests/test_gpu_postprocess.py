@@ -34,6 +34,18 @@ def test_rasteriser_matches_the_cpu_for_every_transform(lib, oracle_lib, trans):
     assert all(0 < np.count_nonzero(dev & (1 << r)) < dev.size for r in range(3))
 
 
+@pytest.mark.parametrize("origin", [(-1.0, -1.125, -0.9375), (1.2e308, 0.0, 0.0)], ids=["near", "overflow"])
+def test_rasteriser_with_infinite_numbers(lib, oracle_lib, origin):
+    """A centre that is not a number (a half-space given as a box) or so far that r - c overflows: then the product with
+    an identity is not the point."""
+    inf = float("inf")
+    roots = [Box((-0.5, -0.5, -inf), (0.25, 0.5, 0.0)), Sphere((inf, 0.0, 0.0), 0.5), Cylinder((0.0, 0.0, -0.5), inf, 0.25, 0.375),
+             Box((-0.5, -0.5, -0.5), (0.25, inf, 0.5)), Sphere((-1.5e308, 0.0, 0.0), inf)]
+    scene = Scene([Region(r) for r in roots])
+    g = Grid(17, 19, 15, 0.125, origin=origin)
+    np.testing.assert_array_equal(rasterize(g, scene), oracle_rasterize(g, scene))
+
+
 @pytest.mark.parametrize("monitors", [1, 3, 8, 9, 700])
 @pytest.mark.parametrize("samples", [1, 2, 3, 65, 300])
 def test_spectrum_matches_the_direct_sum(lib, monitors, samples):
