@@ -24,7 +24,10 @@ __device__ __forceinline__ void mat_vec(const double* __restrict__ m, double x, 
 // bit 1 the primitive's own (t).  At a finite point the product with an
 // identity gives the point back, up to the sign of a zero, which no primitive
 // can tell (t's point, r - c, is finite where neither number is near overflow);
-// the flags are formed once per block.
+// the flags are formed once per block.  Bit 2: the primitive's answer
+// over a row of points is decided by leaf_code at its ends: no transform, and
+// every number so far from overflow (`moderate` grids) that no infinity or NaN
+// can come up on the way.
 constexpr int RASTER_MAX_NODES = SJ_MAX_CSG_NODES * SJ_MAX_REGIONS;
 __device__ __forceinline__ bool is_identity(const double* m) {
     bool id = true;
@@ -34,14 +37,35 @@ __device__ __forceinline__ bool is_identity(const double* m) {
     }
     return id;
 }
-constexpr double FAR = 1e307;
-__device__ void identity_flags(const sj_csg_node* __restrict__ nodes, int n, bool finite, uint8_t* flags) {
+constexpr double MODERATE = 1e100, FAR = 1e307;
+__device__ void identity_flags(const sj_csg_node* __restrict__ nodes, int n, bool finite, bool moderate, uint8_t* flags) {
     for (int q = threadIdx.x; q < n; q += blockDim.x) {
         const sj_csg_node& nd = nodes[q];
         const bool centre = fabs(nd.c[0]) < FAR && fabs(nd.c[1]) < FAR && fabs(nd.c[2]) < FAR;
-        flags[q] = finite ? (uint8_t)((is_identity(nd.m) ? 1 : 0) | (centre && is_identity(nd.t) ? 2 : 0)) : 0;
+        int f = finite ? (is_identity(nd.m) ? 1 : 0) | (centre && is_identity(nd.t) ? 2 : 0) : 0;
+        bool ends = moderate && f == 3;
+        for (int a = 0; a < 4; ++a) ends = ends && fabs(nd.p[a]) < MODERATE;
+        for (int a = 0; a < 3; ++a) ends = ends && fabs(nd.c[a]) < MODERATE;
+        if (nd.op > SJ_CSG_PLANE) f = 4;
+        if (ends) f |= 4;
+        flags[q] = (uint8_t)f;
     }
     __syncthreads();
+}
+
+// The operand stack after one operator
+__device__ __forceinline__ unsigned long long combine(const sj_csg_node& nd, unsigned long long stk) {
+    const int op = nd.op;
+    if (op == SJ_CSG_UNION || op == SJ_CSG_INTERSECT) {
+        const int b = (int)(stk & 1ull);
+        stk >>= 1;
+        const int a = (int)(stk & 1ull);
+        stk >>= 1;
+        return (stk << 1) | (unsigned long long)(nd.invert ^ (op == SJ_CSG_UNION ? (a | b) : (a & b)));
+    }
+    if (op == SJ_CSG_PASS) return (stk & ~1ull) | (unsigned long long)(nd.invert ^ (int)(stk & 1ull));
+    if (op == SJ_CSG_CONST) return (stk << 1) | (unsigned long long)(nd.invert & 1);
+    return stk << 1;  // NOOP
 }
 
 // Evaluate one region's postfix program at r; returns in_root(r) in {0,1}.
@@ -49,7 +73,7 @@ __device__ void identity_flags(const sj_csg_node* __restrict__ nodes, int n, boo
 // Bound by the FP64 pipe (19 cycles per warp operation and SM): a box under
 // two identities costs three subtractions and three comparisons, z first (a
 // thin film's z decides most points of a row at once), instead of 36
-// operations.  256 x 256 x 192 bowtie scene: 16.3 ms before, 2.9 ms.
+// operations.  256 x 256 x 192 bowtie scene, every point: 16.3 ms before, 2.9 ms.
 __device__ int eval_program(const sj_csg_node* __restrict__ nodes, const uint8_t* flags, int n, double x, double y,
                             double z) {
     unsigned long long stk = 0;
@@ -92,31 +116,69 @@ __device__ int eval_program(const sj_csg_node* __restrict__ nodes, const uint8_t
                 v = out ? nd.invert : 1 - nd.invert;
             }
             stk = (stk << 1) | (unsigned long long)v;
-        } else if (op == SJ_CSG_UNION || op == SJ_CSG_INTERSECT) {
-            const int b = (int)(stk & 1ull);
-            stk >>= 1;
-            const int a = (int)(stk & 1ull);
-            stk >>= 1;
-            v = nd.invert ^ (op == SJ_CSG_UNION ? (a | b) : (a & b));
-            stk = (stk << 1) | (unsigned long long)v;
-        } else if (op == SJ_CSG_PASS) {
-            const int a = (int)(stk & 1ull);
-            stk = (stk & ~1ull) | (unsigned long long)(nd.invert ^ a);
-        } else if (op == SJ_CSG_CONST) {
-            stk = (stk << 1) | (unsigned long long)(nd.invert & 1);
-        } else {  // NOOP
-            stk = (stk << 1);
+        } else {
+            stk = combine(nd, stk);
         }
     }
     return (int)(stk & 1ull);
 }
 
-// every point of the grid has coordinates below FAR
-static bool finite_grid(int nx, int ny, int nz, double dx, const double* o) {
+// Where x stands to a primitive without transforms, at a fixed y and z: 0 in,
+// else out, by y or z alone (2) or on x's lower (-1) or upper (1) side; a plane
+// 0 or 1.  Rounded sums and products are monotone in each operand, so along
+// a row a plane's dot product and a box's distance are monotone and a sphere's
+// or cylinder's radius is on either side of its centre: two points with one
+// code have it all the way between them.
+__device__ __forceinline__ int leaf_code(const sj_csg_node& nd, double x, double y, double z) {
+    if (nd.op == SJ_CSG_PLANE) {
+        const double d = __dadd_rn(__dadd_rn(__dmul_rn(x, nd.p[0]), __dmul_rn(y, nd.p[1])), __dmul_rn(z, nd.p[2]));
+        return d > nd.p[3] ? 1 : 0;
+    }
+    const double qx = __dsub_rn(x, nd.c[0]), qy = __dsub_rn(y, nd.c[1]), qz = __dsub_rn(z, nd.c[2]);
+    const int side = qx < 0 ? -1 : 1;
+    if (nd.op == SJ_CSG_BOX) {
+        if (fabs(qz) > nd.p[2] || fabs(qy) > nd.p[1]) return 2;
+        return fabs(qx) > nd.p[0] ? side : 0;
+    }
+    if (nd.op == SJ_CSG_SPHERE) {
+        const double s2 = __dadd_rn(__dadd_rn(__dadd_rn(0.0, __dmul_rn(qx, qx)), __dmul_rn(qy, qy)), __dmul_rn(qz, qz));
+        return __dsqrt_rn(s2) > nd.p[0] ? side : 0;
+    }
+    const double h = nd.p[0], r1 = nd.p[1], r2 = nd.p[2];
+    if (qz < 0 || qz > h) return 2;
+    const double cr = __dadd_rn(__dmul_rn(qx, qx), __dmul_rn(qy, qy));
+    return __dmul_rn(cr, h) > __dadd_rn(__dmul_rn(__dsub_rn(r2, r1), qz), __dmul_rn(r1, h)) ? side : 0;
+}
+
+// eval_program on the row of points from (xa, y, z) to (xb, y, z): in_root
+// where it is one answer by every primitive's code at the ends, else -1.
+__device__ int eval_row(const sj_csg_node* __restrict__ nodes, int n, double xa, double xb, double y, double z) {
+    unsigned long long stk = 0;
+    for (int q = 0; q < n; ++q) {
+        const sj_csg_node& nd = nodes[q];
+        const int op = nd.op;
+        if (op <= SJ_CSG_PLANE) {
+            const int code = leaf_code(nd, xa, y, z);
+            if (code != 2 && leaf_code(nd, xb, y, z) != code) return -1;
+            const int out = code != 0;
+            stk = (stk << 1) | (unsigned long long)(op == SJ_CSG_PLANE ? 1 - out : out ? nd.invert : 1 - nd.invert);
+        } else {
+            stk = combine(nd, stk);
+        }
+    }
+    return (int)(stk & 1ull);
+}
+
+// every point of the grid has coordinates below FAR (1), of moderate size (3)
+static int finite_grid(int nx, int ny, int nz, double dx, const double* o) {
     const int n[3] = {nx, ny, nz};
-    for (int a = 0; a < 3; ++a)
-        if (!(std::fabs(o[a]) < FAR && std::fabs(o[a] + (n[a] + 1.0) * dx) < FAR)) return false;
-    return true;
+    int f = 3;
+    for (int a = 0; a < 3; ++a) {
+        const double end = o[a] + (n[a] + 1.0) * dx;
+        if (!(std::fabs(o[a]) < FAR && std::fabs(end) < FAR)) return 0;
+        if (std::fabs(o[a]) >= MODERATE || std::fabs(end) >= MODERATE) f = 1;
+    }
+    return f;
 }
 
 // Region start table carried by value in the kernel's parameters.
@@ -140,42 +202,126 @@ __device__ __forceinline__ void voxel_of(long long t, long long total, int nx, i
     }
 }
 
-// One thread per voxel: masks for the Ex, Ey and Ez points.  Starts is a
-// device pointer to the region start table or a RegionStarts value.
+// The mask of component c's point (i, j, k): bit g = in region g.
 template <typename Starts>
-__global__ void k_rasterize(const sj_csg_node* __restrict__ nodes, const Starts rstart,
-                            int n_regions, int nx, int ny, int nz, double dx, double ox, double oy,
-                            double oz, int finite, uint8_t* __restrict__ masks, long long cpitch, int px) {
+__device__ __forceinline__ unsigned point_mask(const sj_csg_node* __restrict__ nodes, const Starts& rstart,
+                                               const uint8_t* flags, int n_regions, int c, int i, int j, int k,
+                                               double dx, double ox, double oy, double oz) {
+    const double x = __dadd_rn(ox, __dmul_rn((double)i + (c == 0 ? 0.5 : 0.0), dx));
+    const double y = __dadd_rn(oy, __dmul_rn((double)j + (c == 1 ? 0.5 : 0.0), dx));
+    const double z = __dadd_rn(oz, __dmul_rn((double)k + (c == 2 ? 0.5 : 0.0), dx));
+    unsigned m = 0;
+    for (int g = 0; g < n_regions; ++g) {
+        const int s = rstart[g], e = rstart[g + 1];
+        if (eval_program(nodes + s, flags + s, e - s, x, y, z)) m |= 1u << g;
+    }
+    return m;
+}
+
+// Masks for the Ex, Ey and Ez points.  A thread takes a segment of SEG points
+// of a row: where every primitive's code is the same at its ends the segment
+// has one mask (eval_row), the others are listed and the block then goes over
+// their points one by one, as over all points of a scene with a transform.
+// SEG = 1: a point.  Starts is a device pointer to the region start table or a
+// RegionStarts value.  Ends decide 3 of 4 segments of the 256 x 256 x 192 bowtie:
+// 2.91 ms with every point evaluated, 0.62 with segments of 16 (8: 0.88); 192^3
+// on quartz 0.74 and 0.10.  A segment's two ends and then its block's list are
+// a serial chain, so grids of fewer than RASTER_FEW points take one per thread
+// (spheres and cylinders, 48^3: 43 us, 169 in segments; 80^3 171 and 172;
+// 96^3 283 and 171).
+constexpr int RASTER_SEG = 16, RASTER_THREADS = 128;
+constexpr long long RASTER_FEW = 1 << 19;
+template <typename Starts, int SEG>
+__global__ void __launch_bounds__(RASTER_THREADS, 10)
+k_rasterize(const sj_csg_node* __restrict__ nodes, const Starts rstart, int n_regions, int nx, int ny, int nz, double dx,
+            double ox, double oy, double oz, int finite, uint8_t* __restrict__ masks, long long cpitch, int px) {
     __shared__ uint8_t flags[RASTER_MAX_NODES];
-    identity_flags(nodes, rstart[n_regions], finite != 0, flags);
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long total = (long long)nx * ny * nz;
-    if (t >= total) return;
-    int i, j, k;
-    voxel_of(t, total, nx, ny, i, j, k);
-    const long long o = ((long long)k * ny + j) * px + i;
-    for (int c = 0; c < 3; ++c) {
-        const double x = __dadd_rn(ox, __dmul_rn((double)i + (c == 0 ? 0.5 : 0.0), dx));
+    __shared__ int3 seg[RASTER_THREADS];                 // first point of each thread's segment
+    __shared__ unsigned short list[3 * RASTER_THREADS];  // component * RASTER_THREADS + segment
+    __shared__ int n_list;
+    const int n_nodes = rstart[n_regions];
+    if (threadIdx.x == 0) n_list = 0;
+    identity_flags(nodes, n_nodes, finite & 1, finite & 2, flags);
+    bool ends = SEG > 1;
+    for (int q = threadIdx.x; q < n_nodes && ends; q += RASTER_THREADS) ends = flags[q] & 4;
+    if (SEG > 1) ends = __syncthreads_and(ends);
+    const int nseg = (nx + SEG - 1) / SEG;
+    const long long t = blockIdx.x * (long long)RASTER_THREADS + threadIdx.x;
+    const long long total = (long long)nseg * ny * nz;
+    int i = nx, j = 0, k = 0;
+    if (t < total) {
+        voxel_of(t, total, nseg, ny, i, j, k);
+        i *= SEG;
+    }
+    const int len = min(SEG, nx - i);
+    for (int c = 0; c < 3 && len > 0; ++c) {
+        if (SEG > 1 && !ends) break;
+        uint8_t* const out = masks + c * cpitch + ((long long)k * ny + j) * px + i;
+        if (SEG == 1) {
+            *out = (uint8_t)point_mask(nodes, rstart, flags, n_regions, c, i, j, k, dx, ox, oy, oz);
+            continue;
+        }
+        const double xa = __dadd_rn(ox, __dmul_rn((double)i + (c == 0 ? 0.5 : 0.0), dx));
+        const double xb = __dadd_rn(ox, __dmul_rn((double)(i + len - 1) + (c == 0 ? 0.5 : 0.0), dx));
         const double y = __dadd_rn(oy, __dmul_rn((double)j + (c == 1 ? 0.5 : 0.0), dx));
         const double z = __dadd_rn(oz, __dmul_rn((double)k + (c == 2 ? 0.5 : 0.0), dx));
         unsigned m = 0;
-        for (int g = 0; g < n_regions; ++g) {
-            const int s = rstart[g], e = rstart[g + 1];
-            if (eval_program(nodes + s, flags + s, e - s, x, y, z)) m |= 1u << g;
+        bool one = true;
+        for (int g = 0; g < n_regions && one; ++g) {
+            const int v = eval_row(nodes + rstart[g], rstart[g + 1] - rstart[g], xa, xb, y, z);
+            one = v >= 0;
+            if (v > 0) m |= 1u << g;
         }
-        masks[c * cpitch + o] = (uint8_t)m;
+        if (!one) {
+            list[atomicAdd(&n_list, 1)] = (unsigned short)(c * RASTER_THREADS + threadIdx.x);
+        } else if (len == 16 && (reinterpret_cast<size_t>(out) & 15) == 0) {
+            const unsigned w = m * 0x01010101u;
+            *reinterpret_cast<uint4*>(out) = make_uint4(w, w, w, w);
+        } else {
+            for (int q = 0; q < len; ++q) out[q] = (uint8_t)m;
+        }
     }
+    if (SEG == 1) return;
+    seg[threadIdx.x] = make_int3(i, j, k);
+    __syncthreads();
+    // the points of `comps` components from c of entry e's segment
+    auto points = [&](int e, int q, int c, int comps) {
+        const int3 f = seg[e];
+        if (f.x + q >= nx) return;
+        uint8_t* const out = masks + ((long long)f.z * ny + f.y) * px + f.x + q;
+        for (int d = c; d < c + comps; ++d)
+            out[d * cpitch] = (uint8_t)point_mask(nodes, rstart, flags, n_regions, d, f.x + q, f.y, f.z, dx, ox, oy, oz);
+    };
+    if (ends) {
+        for (int u = threadIdx.x; u < n_list * SEG; u += RASTER_THREADS) {
+            const int e = list[u / SEG];
+            points(e % RASTER_THREADS, u % SEG, e / RASTER_THREADS, 1);
+        }
+    } else {
+        for (int u = threadIdx.x; u < RASTER_THREADS * SEG; u += RASTER_THREADS) points(u / SEG, u % SEG, 0, 3);
+    }
+}
+
+template <typename Starts>
+static cudaError_t rasterize_with(const sj_csg_node* d_nodes, const Starts& starts, int n_regions, int nx, int ny, int nz,
+                                  double dx, const double* o, uint8_t* d_masks, long long cpitch, int px, cudaStream_t s) {
+    const bool few = (long long)nx * ny * nz < RASTER_FEW;
+    const long long threads = (long long)(few ? nx : (nx + RASTER_SEG - 1) / RASTER_SEG) * ny * nz;
+    const unsigned blocks = (unsigned)((threads + RASTER_THREADS - 1) / RASTER_THREADS);
+    const int finite = finite_grid(nx, ny, nz, dx, o);
+    if (few)
+        k_rasterize<Starts, 1><<<blocks, RASTER_THREADS, 0, s>>>(d_nodes, starts, n_regions, nx, ny, nz, dx, o[0], o[1], o[2],
+                                                                 finite, d_masks, cpitch, px);
+    else
+        k_rasterize<Starts, RASTER_SEG><<<blocks, RASTER_THREADS, 0, s>>>(d_nodes, starts, n_regions, nx, ny, nz, dx, o[0],
+                                                                          o[1], o[2], finite, d_masks, cpitch, px);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_rasterize(const sj_csg_node* d_nodes, const int* d_region_start, int n_regions,
                              int nx, int ny, int nz, double dx, const double* origin,
                              uint8_t* d_masks, long long mask_pitch_elems, int px, cudaStream_t s) {
-    const long long total = (long long)nx * ny * nz;
-    const unsigned blocks = (unsigned)((total + 255) / 256);
-    k_rasterize<const int*><<<blocks, 256, 0, s>>>(d_nodes, d_region_start, n_regions, nx, ny, nz, dx,
-                                                   origin[0], origin[1], origin[2],
-                                                   finite_grid(nx, ny, nz, dx, origin), d_masks, mask_pitch_elems, px);
-    return cudaGetLastError();
+    return rasterize_with(d_nodes, d_region_start, n_regions, nx, ny, nz, dx, origin, d_masks, mask_pitch_elems, px, s);
 }
 
 // ------------------------------------------------------------ smoothing
@@ -219,7 +365,7 @@ __global__ void k_rasterize_counts(const sj_csg_node* __restrict__ nodes, const 
     __shared__ uint8_t flags[RASTER_MAX_NODES];
     bool all = finite != 0;
     for (int q = threadIdx.x; q < 3 * n_offs; q += blockDim.x) all = all && fabs(offs[q]) < FAR;
-    identity_flags(nodes, rstart[n_regions], __syncthreads_and(all) != 0, flags);
+    identity_flags(nodes, rstart[n_regions], __syncthreads_and(all) != 0, false, flags);
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long total = (long long)nx * ny * nz;
     if (t >= total) return;
@@ -574,13 +720,7 @@ int rasterize_static(const sj_grid_desc* g, const sj_scene_desc* sc, uint8_t* d_
                             (size_t)sc->regions[r].n_nodes * sizeof(sj_csg_node), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
         const long long nv = (long long)g->nx * g->ny * g->nz;
-        const long long total = nv;
-        const unsigned blocks = (unsigned)((total + 255) / 256);
-        k_rasterize<RegionStarts><<<blocks, 256, 0, s>>>(d_nodes, start, sc->n_regions, g->nx, g->ny, g->nz,
-                                                         g->dx, g->origin[0], g->origin[1], g->origin[2],
-                                                         finite_grid(g->nx, g->ny, g->nz, g->dx, g->origin), d_out, nv,
-                                                         g->nx);
-        e = cudaGetLastError();
+        e = rasterize_with(d_nodes, start, sc->n_regions, g->nx, g->ny, g->nz, g->dx, g->origin, d_out, nv, g->nx, s);
     }
     if (e != cudaSuccess) {
         *msg = "CUDA call failed in sj_rasterize_static";

@@ -46,6 +46,34 @@ def test_rasteriser_with_infinite_numbers(lib, oracle_lib, origin):
     np.testing.assert_array_equal(rasterize(g, scene), oracle_rasterize(g, scene))
 
 
+@pytest.mark.parametrize("nx", [1, 15, 16, 17, 32, 75])
+@pytest.mark.parametrize("x0", [-1.0, 1e101], ids=["near", "far"])
+def test_rasteriser_rows_match_the_cpu(lib, oracle_lib, nx, x0):
+    """Whole segments of a row decided at their ends: primitives smaller than a segment, tangent to rows, of zero,
+    negative and infinite extent, around, left and right of each segment."""
+    rng = np.random.default_rng(nx)
+    inf = float("inf")
+
+    def leaf():
+        c = tuple(np.round(rng.uniform(-1, 1, 3) * [nx / 16 + 0.5, 1, 1], 2))
+        s = [float(x) for x in np.round(rng.uniform(0.05, 0.8, 3), 2)]
+        return [lambda: Box(tuple(np.subtract(c, s)), tuple(np.add(c, s)), invert=int(rng.integers(2))),
+                lambda: Sphere(c, s[0], invert=int(rng.integers(2))),
+                lambda: Cylinder(c, *s),
+                lambda: Plane(tuple(rng.normal(size=3)), float(rng.uniform(-1, 1)))][rng.integers(4)]()
+
+    roots = [Union(Intersect(leaf(), leaf()), Difference(leaf(), leaf())) for _ in range(3)]
+    roots += [Union(Sphere((0.0625, 0.0, 0.0), 0.0), Sphere((0.5, 0.0, 0.0), 0.0625)),   # one point, two points of a row
+              Intersect(Plane((1.0, 0.0, 0.0), 0.25), Plane((-1.0, 1.0, 0.0), -0.25)),
+              Union(Box((0.25, -0.5, -0.5), (-0.25, 0.5, 0.5)), Sphere((0.0, 0.0, 0.0), -0.25))]
+    endless = Union(Cylinder((0.0, 0.0, -0.5), inf, 0.25, 0.375), Box((-0.5, -0.5, -inf), (0.25, 0.5, 0.0)))
+    n = int(np.sqrt(2 ** 19 / nx)) + 1   # enough points for the segments
+    g = Grid(nx, n, n, 0.125, origin=(x0, -0.125 * (n // 2), -0.125 * (n // 3)))
+    for rs in (roots, roots + [endless]):   # the second: every point evaluated
+        scene = Scene([Region(r) for r in rs])
+        np.testing.assert_array_equal(rasterize(g, scene), oracle_rasterize(g, scene))
+
+
 @pytest.mark.parametrize("monitors", [1, 3, 8, 9, 700])
 @pytest.mark.parametrize("samples", [1, 2, 3, 65, 300])
 def test_spectrum_matches_the_direct_sum(lib, monitors, samples):
