@@ -443,8 +443,8 @@ std::vector<unsigned long long> smooth_rasterize(sj_sim* sim, const sj_scene_des
     unsigned long long* d_set = (unsigned long long*)sim->dalloc(SMOOTH_SET_CAP * sizeof(unsigned long long), false);
     int* d_over = (int*)sim->dalloc(sizeof(int));
     ck(cudaMemsetAsync(d_set, 0xff, SMOOTH_SET_CAP * sizeof(unsigned long long), st), "set clear");
-    ck(launch_rasterize_counts(d_nodes, d_start, sc->n_regions, g.nx, g.ny, g.nz, g.dx, g.origin, d_offs,
-                               (int)(offs.size() / 3), d_keys, cpitch, px, d_set, SMOOTH_SET_CAP, d_over, st),
+    ck(launch_rasterize_counts(d_nodes, d_start, sc->n_regions, raster_rows(sc, offs.data(), offs.size()), g.nx, g.ny, g.nz,
+                               g.dx, g.origin, d_offs, (int)(offs.size() / 3), d_keys, cpitch, px, d_set, SMOOTH_SET_CAP, d_over, st),
        "rasterize counts");
     std::vector<unsigned long long> set(SMOOTH_SET_CAP);
     int over = 0;
@@ -532,8 +532,8 @@ void build_instance(sj_sim* sim, const sj_instance_desc& d, HostInst<real>& H, I
             smooth_scene_classes(m.scene, keys, eps, poles, sigma, n_classes);
         } else {
             scene_classes(m.scene, eps, poles, sigma, n_classes);
-            ck(launch_rasterize(d_nodes, d_start, m.scene->n_regions, nx, ny, nz, H.dx, g.origin, d_cls,
-                                cpitch, px, st),
+            ck(launch_rasterize(d_nodes, d_start, m.scene->n_regions, raster_rows(m.scene), nx, ny, nz, H.dx, g.origin,
+                                d_cls, cpitch, px, st),
                "rasterize");
         }
     }
@@ -2576,8 +2576,8 @@ int sj_rasterize(const sj_grid_desc* grid, const sj_scene_desc* scene, uint8_t* 
         const int nx = grid->nx, ny = grid->ny, nz = grid->nz;
         const long long nv = (long long)nx * ny * nz;
         uint8_t* d = (uint8_t*)tmp.dalloc(3 * nv);
-        ck(launch_rasterize(d_nodes, d_start, scene->n_regions, nx, ny, nz, grid->dx, grid->origin, d, nv,
-                            nx, tmp.stream),
+        ck(launch_rasterize(d_nodes, d_start, scene->n_regions, raster_rows(scene), nx, ny, nz, grid->dx, grid->origin, d,
+                            nv, nx, tmp.stream),
            "rasterize");
         ck(cudaMemcpyAsync(out, d, 3 * nv, cudaMemcpyDeviceToHost, tmp.stream), "mask read");
         ck(cudaStreamSynchronize(tmp.stream), "sync");
@@ -2605,8 +2605,8 @@ int sj_rasterize_counts(const sj_grid_desc* grid, const sj_scene_desc* scene, ui
             scene->smooth_n > 0 ? smooth_points(scene->smooth_n, scene->smooth_rad) : std::vector<double>();
         double* d_offs = tmp.upload(offs);
         unsigned long long* d = (unsigned long long*)tmp.dalloc(3 * nv * sizeof(unsigned long long));
-        ck(launch_rasterize_counts(d_nodes, d_start, R, nx, ny, nz, grid->dx, grid->origin, d_offs,
-                                   (int)(offs.size() / 3), d, nv, nx, nullptr, 0, nullptr, tmp.stream),
+        ck(launch_rasterize_counts(d_nodes, d_start, R, raster_rows(scene, offs.data(), offs.size()), nx, ny, nz, grid->dx,
+                                   grid->origin, d_offs, (int)(offs.size() / 3), d, nv, nx, nullptr, 0, nullptr, tmp.stream),
            "rasterize counts");
         std::vector<unsigned long long> keys(3 * nv);
         ck(cudaMemcpyAsync(keys.data(), d, keys.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,

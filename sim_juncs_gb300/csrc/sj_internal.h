@@ -324,14 +324,16 @@ cudaError_t launch_spectrum(const double* d_mon, int n_mon, long long n, long lo
                             cudaStream_t s);
 
 // Launch helpers implemented in sj_raster.cu.
+// may the ends of a row of points decide them? (offs: smoothing offsets)
+bool raster_rows(const sj_scene_desc* sc, const double* offs = nullptr, size_t n_offs = 0);
 cudaError_t launch_rasterize(const sj_csg_node* d_nodes, const int* d_region_start,
-                             int n_regions, int nx, int ny, int nz, double dx,
+                             int n_regions, bool rows, int nx, int ny, int nz, double dx,
                              const double* origin, uint8_t* d_masks, long long mask_pitch_elems,
                              int px, cudaStream_t s);
 // smoothing: per-point region counts packed 8 bits per region (keys, pitched
 // [3][pitch]), distinct keys into a set of cap slots, then key -> class byte
 constexpr unsigned SMOOTH_SET_CAP = 4096;
-cudaError_t launch_rasterize_counts(const sj_csg_node* d_nodes, const int* d_region_start, int n_regions,
+cudaError_t launch_rasterize_counts(const sj_csg_node* d_nodes, const int* d_region_start, int n_regions, bool rows,
                                     int nx, int ny, int nz, double dx, const double* origin,
                                     const double* d_offs, int n_offs, unsigned long long* d_keys,
                                     long long key_pitch_elems, int px, unsigned long long* d_set,

@@ -24,10 +24,7 @@ __device__ __forceinline__ void mat_vec(const double* __restrict__ m, double x, 
 // bit 1 the primitive's own (t).  At a finite point the product with an
 // identity gives the point back, up to the sign of a zero, which no primitive
 // can tell (t's point, r - c, is finite where neither number is near overflow);
-// the flags are formed once per block.  Bit 2: the primitive's answer
-// over a row of points is decided by leaf_code at its ends: no transform, and
-// every number so far from overflow (`moderate` grids) that no infinity or NaN
-// can come up on the way.
+// the flags are formed once per block.
 constexpr int RASTER_MAX_NODES = SJ_MAX_CSG_NODES * SJ_MAX_REGIONS;
 __device__ __forceinline__ bool is_identity(const double* m) {
     bool id = true;
@@ -38,19 +35,37 @@ __device__ __forceinline__ bool is_identity(const double* m) {
     return id;
 }
 constexpr double MODERATE = 1e100, FAR = 1e307;
-__device__ void identity_flags(const sj_csg_node* __restrict__ nodes, int n, bool finite, bool moderate, uint8_t* flags) {
+__device__ void identity_flags(const sj_csg_node* __restrict__ nodes, int n, bool finite, uint8_t* flags) {
     for (int q = threadIdx.x; q < n; q += blockDim.x) {
         const sj_csg_node& nd = nodes[q];
         const bool centre = fabs(nd.c[0]) < FAR && fabs(nd.c[1]) < FAR && fabs(nd.c[2]) < FAR;
-        int f = finite ? (is_identity(nd.m) ? 1 : 0) | (centre && is_identity(nd.t) ? 2 : 0) : 0;
-        bool ends = moderate && f == 3;
-        for (int a = 0; a < 4; ++a) ends = ends && fabs(nd.p[a]) < MODERATE;
-        for (int a = 0; a < 3; ++a) ends = ends && fabs(nd.c[a]) < MODERATE;
-        if (nd.op > SJ_CSG_PLANE) f = 4;
-        if (ends) f |= 4;
-        flags[q] = (uint8_t)f;
+        flags[q] = finite ? (uint8_t)((is_identity(nd.m) ? 1 : 0) | (centre && is_identity(nd.t) ? 2 : 0)) : 0;
     }
     __syncthreads();
+}
+
+// Do a row's ends decide every primitive of the scene (leaf_code)?  No
+// transforms, and every number so far from overflow that no infinity or NaN can
+// come up on the way.
+bool raster_rows(const sj_scene_desc* sc, const double* offs, size_t n_offs) {
+    for (size_t q = 0; q < n_offs; ++q)
+        if (!(std::fabs(offs[q]) < MODERATE)) return false;
+    auto identity = [](const double* m) {
+        for (int q = 0; q < 9; ++q)
+            if (m[q] != (q % 4 == 0 ? 1.0 : 0.0)) return false;
+        return true;
+    };
+    for (int r = 0; r < sc->n_regions; ++r)
+        for (int q = 0; q < sc->regions[r].n_nodes; ++q) {
+            const sj_csg_node& nd = sc->regions[r].nodes[q];
+            if (nd.op > SJ_CSG_PLANE) continue;
+            if (!identity(nd.m) || !identity(nd.t)) return false;
+            for (int a = 0; a < 4; ++a)
+                if (!(std::fabs(nd.p[a]) < MODERATE)) return false;
+            for (int a = 0; a < 3; ++a)
+                if (!(std::fabs(nd.c[a]) < MODERATE)) return false;
+        }
+    return true;
 }
 
 // The operand stack after one operator
@@ -221,8 +236,8 @@ __device__ __forceinline__ unsigned point_mask(const sj_csg_node* __restrict__ n
 // Masks for the Ex, Ey and Ez points.  A thread takes a segment of SEG points
 // of a row: where every primitive's code is the same at its ends the segment
 // has one mask (eval_row), the others are listed and the block then goes over
-// their points one by one, as over all points of a scene with a transform.
-// SEG = 1: a point.  Starts is a device pointer to the region start table or a
+// their points one by one.  SEG = 1 (also for scenes with a transform): a
+// point.  Starts is a device pointer to the region start table or a
 // RegionStarts value.  Ends decide 3 of 4 segments of the 256 x 256 x 192 bowtie:
 // 2.91 ms with every point evaluated, 0.62 with segments of 16 (8: 0.88); 192^3
 // on quartz 0.74 and 0.10.  A segment's two ends and then its block's list are
@@ -239,12 +254,8 @@ k_rasterize(const sj_csg_node* __restrict__ nodes, const Starts rstart, int n_re
     __shared__ int3 seg[RASTER_THREADS];                 // first point of each thread's segment
     __shared__ unsigned short list[3 * RASTER_THREADS];  // component * RASTER_THREADS + segment
     __shared__ int n_list;
-    const int n_nodes = rstart[n_regions];
     if (threadIdx.x == 0) n_list = 0;
-    identity_flags(nodes, n_nodes, finite & 1, finite & 2, flags);
-    bool ends = SEG > 1;
-    for (int q = threadIdx.x; q < n_nodes && ends; q += RASTER_THREADS) ends = flags[q] & 4;
-    if (SEG > 1) ends = __syncthreads_and(ends);
+    identity_flags(nodes, rstart[n_regions], finite != 0, flags);
     const int nseg = (nx + SEG - 1) / SEG;
     const long long t = blockIdx.x * (long long)RASTER_THREADS + threadIdx.x;
     const long long total = (long long)nseg * ny * nz;
@@ -255,7 +266,6 @@ k_rasterize(const sj_csg_node* __restrict__ nodes, const Starts rstart, int n_re
     }
     const int len = min(SEG, nx - i);
     for (int c = 0; c < 3 && len > 0; ++c) {
-        if (SEG > 1 && !ends) break;
         uint8_t* const out = masks + c * cpitch + ((long long)k * ny + j) * px + i;
         if (SEG == 1) {
             *out = (uint8_t)point_mask(nodes, rstart, flags, n_regions, c, i, j, k, dx, ox, oy, oz);
@@ -284,44 +294,42 @@ k_rasterize(const sj_csg_node* __restrict__ nodes, const Starts rstart, int n_re
     if (SEG == 1) return;
     seg[threadIdx.x] = make_int3(i, j, k);
     __syncthreads();
-    // the points of `comps` components from c of entry e's segment
-    auto points = [&](int e, int q, int c, int comps) {
-        const int3 f = seg[e];
-        if (f.x + q >= nx) return;
-        uint8_t* const out = masks + ((long long)f.z * ny + f.y) * px + f.x + q;
-        for (int d = c; d < c + comps; ++d)
-            out[d * cpitch] = (uint8_t)point_mask(nodes, rstart, flags, n_regions, d, f.x + q, f.y, f.z, dx, ox, oy, oz);
-    };
-    if (ends) {
-        for (int u = threadIdx.x; u < n_list * SEG; u += RASTER_THREADS) {
-            const int e = list[u / SEG];
-            points(e % RASTER_THREADS, u % SEG, e / RASTER_THREADS, 1);
-        }
-    } else {
-        for (int u = threadIdx.x; u < RASTER_THREADS * SEG; u += RASTER_THREADS) points(u / SEG, u % SEG, 0, 3);
+    for (int u = threadIdx.x; u < n_list * SEG; u += RASTER_THREADS) {
+        const int e = list[u / SEG], c = e / RASTER_THREADS;
+        const int3 f = seg[e % RASTER_THREADS];
+        const int p = f.x + u % SEG;
+        if (p < nx)
+            masks[c * cpitch + ((long long)f.z * ny + f.y) * px + p] =
+                (uint8_t)point_mask(nodes, rstart, flags, n_regions, c, p, f.y, f.z, dx, ox, oy, oz);
     }
 }
 
+// A kernel's segment length by the grid, and its blocks
+static bool raster_segments(int nx, int ny, int nz, bool rows, int finite, unsigned& blocks) {
+    const bool seg = rows && finite == 3 && (long long)nx * ny * nz >= RASTER_FEW;
+    const long long threads = (long long)(seg ? (nx + RASTER_SEG - 1) / RASTER_SEG : nx) * ny * nz;
+    blocks = (unsigned)((threads + RASTER_THREADS - 1) / RASTER_THREADS);
+    return seg;
+}
 template <typename Starts>
-static cudaError_t rasterize_with(const sj_csg_node* d_nodes, const Starts& starts, int n_regions, int nx, int ny, int nz,
-                                  double dx, const double* o, uint8_t* d_masks, long long cpitch, int px, cudaStream_t s) {
-    const bool few = (long long)nx * ny * nz < RASTER_FEW;
-    const long long threads = (long long)(few ? nx : (nx + RASTER_SEG - 1) / RASTER_SEG) * ny * nz;
-    const unsigned blocks = (unsigned)((threads + RASTER_THREADS - 1) / RASTER_THREADS);
+static cudaError_t rasterize_with(const sj_csg_node* d_nodes, const Starts& starts, int n_regions, bool rows, int nx, int ny,
+                                  int nz, double dx, const double* o, uint8_t* d_masks, long long cpitch, int px,
+                                  cudaStream_t s) {
     const int finite = finite_grid(nx, ny, nz, dx, o);
-    if (few)
-        k_rasterize<Starts, 1><<<blocks, RASTER_THREADS, 0, s>>>(d_nodes, starts, n_regions, nx, ny, nz, dx, o[0], o[1], o[2],
-                                                                 finite, d_masks, cpitch, px);
-    else
+    unsigned blocks;
+    if (raster_segments(nx, ny, nz, rows, finite, blocks))
         k_rasterize<Starts, RASTER_SEG><<<blocks, RASTER_THREADS, 0, s>>>(d_nodes, starts, n_regions, nx, ny, nz, dx, o[0],
                                                                           o[1], o[2], finite, d_masks, cpitch, px);
+    else
+        k_rasterize<Starts, 1><<<blocks, RASTER_THREADS, 0, s>>>(d_nodes, starts, n_regions, nx, ny, nz, dx, o[0], o[1], o[2],
+                                                                 finite, d_masks, cpitch, px);
     return cudaGetLastError();
 }
 
-cudaError_t launch_rasterize(const sj_csg_node* d_nodes, const int* d_region_start, int n_regions,
+cudaError_t launch_rasterize(const sj_csg_node* d_nodes, const int* d_region_start, int n_regions, bool rows,
                              int nx, int ny, int nz, double dx, const double* origin,
                              uint8_t* d_masks, long long mask_pitch_elems, int px, cudaStream_t s) {
-    return rasterize_with(d_nodes, d_region_start, n_regions, nx, ny, nz, dx, origin, d_masks, mask_pitch_elems, px, s);
+    return rasterize_with(d_nodes, d_region_start, n_regions, rows, nx, ny, nz, dx, origin, d_masks, mask_pitch_elems, px, s);
 }
 
 // ------------------------------------------------------------ smoothing
@@ -355,54 +363,129 @@ __device__ void smooth_insert(unsigned long long* set, unsigned cap, unsigned lo
     atomicExch(overflow, 1);
 }
 
-// One thread per voxel: keys of the Ex, Ey and Ez points; with a set, every
-// distinct key also goes into it (one insert per distinct key of a warp).
-__global__ void k_rasterize_counts(const sj_csg_node* __restrict__ nodes, const int* __restrict__ rstart,
-                                   int n_regions, int nx, int ny, int nz, double dx, double ox, double oy,
-                                   double oz, int finite, const double* __restrict__ offs, int n_offs,
-                                   unsigned long long* __restrict__ keys, long long kpitch, int px,
-                                   unsigned long long* __restrict__ set, unsigned cap, int* __restrict__ overflow) {
+// The key of the row of points from (xa, y, z) to (xb, y, z) where every sample
+// of every region is decided by its ends, else SMOOTH_EMPTY.
+__device__ __forceinline__ unsigned long long row_key(const sj_csg_node* __restrict__ nodes, const int* __restrict__ rstart,
+                                                      int n_regions, const double* __restrict__ offs, int n_offs, double xa,
+                                                      double xb, double y, double z) {
+    unsigned long long key = 0;
+    for (int g = 0; g < n_regions; ++g) {
+        const sj_csg_node* p = nodes + rstart[g];
+        const int n = rstart[g + 1] - rstart[g];
+        const int in = eval_row(p, n, xa, xb, y, z);
+        if (in < 0) return SMOOTH_EMPTY;
+        unsigned cnt = (unsigned)in;
+        for (int q = 0; q < n_offs; ++q) {
+            const double dx = offs[3 * q];
+            const int v = eval_row(p, n, __dadd_rn(xa, dx), __dadd_rn(xb, dx), __dadd_rn(y, offs[3 * q + 1]),
+                                   __dadd_rn(z, offs[3 * q + 2]));
+            if (v < 0) return SMOOTH_EMPTY;
+            cnt += (unsigned)v;
+        }
+        key |= (unsigned long long)cnt << (8 * g);
+    }
+    return key;
+}
+
+// Keys of the Ex, Ey and Ez points; with a set, every distinct key also goes
+// into it (one insert per distinct key of a warp's points).  Segments of SEG
+// points of a row as in k_rasterize: one key where their ends decide every
+// sample (rounded offsets keep the order of x), else point by point.
+// smooth_n = 1, every point and in segments: 256 x 256 x 192 bowtie 23.8 and
+// 5.3 ms, 192^3 junction 2.9 and 0.5 (FP64 operations of what stays undecided).
+template <int SEG>
+__global__ void __launch_bounds__(RASTER_THREADS, 8)
+k_rasterize_counts(const sj_csg_node* __restrict__ nodes, const int* __restrict__ rstart, int n_regions, int nx, int ny,
+                   int nz, double dx, double ox, double oy, double oz, int finite, const double* __restrict__ offs,
+                   int n_offs, unsigned long long* __restrict__ keys, long long kpitch, int px,
+                   unsigned long long* __restrict__ set, unsigned cap, int* __restrict__ overflow) {
     __shared__ uint8_t flags[RASTER_MAX_NODES];
+    __shared__ int3 seg[RASTER_THREADS];                 // first point of each thread's segment
+    __shared__ unsigned short list[3 * RASTER_THREADS];  // component * RASTER_THREADS + segment
+    __shared__ unsigned long long row[3][RASTER_THREADS];  // its key
+    __shared__ int n_list;
+    if (threadIdx.x == 0) n_list = 0;
     bool all = finite != 0;
-    for (int q = threadIdx.x; q < 3 * n_offs; q += blockDim.x) all = all && fabs(offs[q]) < FAR;
-    identity_flags(nodes, rstart[n_regions], __syncthreads_and(all) != 0, false, flags);
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long total = (long long)nx * ny * nz;
-    if (t >= total) return;
-    int i, j, k;
-    voxel_of(t, total, nx, ny, i, j, k);
-    const long long o = ((long long)k * ny + j) * px + i;
-    for (int c = 0; c < 3; ++c) {
-        const double x = __dadd_rn(ox, __dmul_rn((double)i + (c == 0 ? 0.5 : 0.0), dx));
-        const double y = __dadd_rn(oy, __dmul_rn((double)j + (c == 1 ? 0.5 : 0.0), dx));
-        const double z = __dadd_rn(oz, __dmul_rn((double)k + (c == 2 ? 0.5 : 0.0), dx));
+    for (int q = threadIdx.x; q < 3 * n_offs; q += RASTER_THREADS) all = all && fabs(offs[q]) < FAR;
+    identity_flags(nodes, rstart[n_regions], __syncthreads_and(all) != 0, flags);
+    const int nseg = (nx + SEG - 1) / SEG;
+    const long long t = blockIdx.x * (long long)RASTER_THREADS + threadIdx.x;
+    const long long total = (long long)nseg * ny * nz;
+    int i = nx, j = 0, k = 0;
+    if (t < total) {
+        voxel_of(t, total, nseg, ny, i, j, k);
+        i *= SEG;
+    }
+    auto insert = [&](unsigned long long key) {
+        if (!set) return;
+        const unsigned peers = __match_any_sync(__activemask(), key);
+        if ((threadIdx.x & 31) == (unsigned)(__ffs(peers) - 1)) smooth_insert(set, cap, key, overflow);
+    };
+    // component c's key at point (p, q, r)
+    auto point = [&](int c, int p, int q, int r) {
+        const double x = __dadd_rn(ox, __dmul_rn((double)p + (c == 0 ? 0.5 : 0.0), dx));
+        const double y = __dadd_rn(oy, __dmul_rn((double)q + (c == 1 ? 0.5 : 0.0), dx));
+        const double z = __dadd_rn(oz, __dmul_rn((double)r + (c == 2 ? 0.5 : 0.0), dx));
         unsigned long long key = 0;
         for (int g = 0; g < n_regions; ++g) {
             const int s = rstart[g], e = rstart[g + 1];
             unsigned cnt = (unsigned)eval_program(nodes + s, flags + s, e - s, x, y, z);
-            for (int q = 0; q < n_offs; ++q)
-                cnt += (unsigned)eval_program(nodes + s, flags + s, e - s, __dadd_rn(x, offs[3 * q]),
-                                              __dadd_rn(y, offs[3 * q + 1]), __dadd_rn(z, offs[3 * q + 2]));
+            for (int m = 0; m < n_offs; ++m)
+                cnt += (unsigned)eval_program(nodes + s, flags + s, e - s, __dadd_rn(x, offs[3 * m]),
+                                              __dadd_rn(y, offs[3 * m + 1]), __dadd_rn(z, offs[3 * m + 2]));
             key |= (unsigned long long)cnt << (8 * g);
         }
-        keys[c * kpitch + o] = key;
-        if (set) {
-            const unsigned peers = __match_any_sync(__activemask(), key);
-            if ((threadIdx.x & 31) == (unsigned)(__ffs(peers) - 1)) smooth_insert(set, cap, key, overflow);
+        keys[c * kpitch + ((long long)r * ny + q) * px + p] = key;
+        insert(key);
+    };
+    const int len = min(SEG, nx - i);
+    for (int c = 0; c < 3 && len > 0; ++c) {
+        if (SEG == 1) {
+            point(c, i, j, k);
+            continue;
         }
+        const double xa = __dadd_rn(ox, __dmul_rn((double)i + (c == 0 ? 0.5 : 0.0), dx));
+        const double xb = __dadd_rn(ox, __dmul_rn((double)(i + len - 1) + (c == 0 ? 0.5 : 0.0), dx));
+        const double y = __dadd_rn(oy, __dmul_rn((double)j + (c == 1 ? 0.5 : 0.0), dx));
+        const double z = __dadd_rn(oz, __dmul_rn((double)k + (c == 2 ? 0.5 : 0.0), dx));
+        const unsigned long long key = row_key(nodes, rstart, n_regions, offs, n_offs, xa, xb, y, z);
+        row[c][threadIdx.x] = key;
+        if (key == SMOOTH_EMPTY)
+            list[atomicAdd(&n_list, 1)] = (unsigned short)(c * RASTER_THREADS + threadIdx.x);
+        else
+            insert(key);
+    }
+    if (SEG == 1) return;
+    seg[threadIdx.x] = make_int3(i, j, k);
+    __syncthreads();
+    for (int u = threadIdx.x; u < RASTER_THREADS * SEG; u += RASTER_THREADS) {
+        const int3 f = seg[u / SEG];
+        const int p = f.x + u % SEG;
+        if (p >= nx) continue;
+        for (int c = 0; c < 3; ++c) {
+            if (row[c][u / SEG] != SMOOTH_EMPTY)
+                keys[c * kpitch + ((long long)f.z * ny + f.y) * px + p] = row[c][u / SEG];
+        }
+    }
+    for (int u = threadIdx.x; u < n_list * SEG; u += RASTER_THREADS) {
+        const int e = list[u / SEG];
+        const int3 f = seg[e % RASTER_THREADS];
+        const int p = f.x + u % SEG;
+        if (p < nx) point(e / RASTER_THREADS, p, f.y, f.z);
     }
 }
 
-cudaError_t launch_rasterize_counts(const sj_csg_node* d_nodes, const int* d_region_start, int n_regions,
+cudaError_t launch_rasterize_counts(const sj_csg_node* d_nodes, const int* d_region_start, int n_regions, bool rows,
                                     int nx, int ny, int nz, double dx, const double* origin,
                                     const double* d_offs, int n_offs, unsigned long long* d_keys,
                                     long long key_pitch_elems, int px, unsigned long long* d_set,
                                     unsigned cap, int* d_overflow, cudaStream_t s) {
-    const long long total = (long long)nx * ny * nz;
-    const unsigned blocks = (unsigned)((total + 255) / 256);
-    k_rasterize_counts<<<blocks, 256, 0, s>>>(d_nodes, d_region_start, n_regions, nx, ny, nz, dx, origin[0],
-                                              origin[1], origin[2], finite_grid(nx, ny, nz, dx, origin), d_offs, n_offs,
-                                              d_keys, key_pitch_elems, px, d_set, cap, d_overflow);
+    const int finite = finite_grid(nx, ny, nz, dx, origin);
+    unsigned blocks;
+    const bool seg = raster_segments(nx, ny, nz, rows, finite, blocks);
+    (seg ? k_rasterize_counts<RASTER_SEG> : k_rasterize_counts<1>)<<<blocks, RASTER_THREADS, 0, s>>>(
+        d_nodes, d_region_start, n_regions, nx, ny, nz, dx, origin[0], origin[1], origin[2], finite, d_offs, n_offs, d_keys,
+        key_pitch_elems, px, d_set, cap, d_overflow);
     return cudaGetLastError();
 }
 
@@ -720,7 +803,8 @@ int rasterize_static(const sj_grid_desc* g, const sj_scene_desc* sc, uint8_t* d_
                             (size_t)sc->regions[r].n_nodes * sizeof(sj_csg_node), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
         const long long nv = (long long)g->nx * g->ny * g->nz;
-        e = rasterize_with(d_nodes, start, sc->n_regions, g->nx, g->ny, g->nz, g->dx, g->origin, d_out, nv, g->nx, s);
+        e = rasterize_with(d_nodes, start, sc->n_regions, raster_rows(sc), g->nx, g->ny, g->nz, g->dx, g->origin, d_out, nv,
+                           g->nx, s);
     }
     if (e != cudaSuccess) {
         *msg = "CUDA call failed in sj_rasterize_static";

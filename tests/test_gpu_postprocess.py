@@ -5,10 +5,10 @@ smallest and largest series."""
 import numpy as np
 import pytest
 
-from oracle.oracle import rasterize as oracle_rasterize
+from oracle.oracle import rasterize as oracle_rasterize, rasterize_counts as oracle_counts
 from sim_juncs_gb300 import _abi
 from sim_juncs_gb300.configs import junction_instance
-from sim_juncs_gb300.fields import Fields, rasterize
+from sim_juncs_gb300.fields import Fields, rasterize, rasterize_counts
 from sim_juncs_gb300.geometry import Box, Cylinder, Difference, Intersect, Plane, Sphere, Union, rotation
 from sim_juncs_gb300.phases import extract_phases
 from sim_juncs_gb300.spec import Grid, Probe, Region, Scene
@@ -72,6 +72,10 @@ def test_rasteriser_rows_match_the_cpu(lib, oracle_lib, nx, x0):
     for rs in (roots, roots + [endless]):   # the second: every point evaluated
         scene = Scene([Region(r) for r in rs])
         np.testing.assert_array_equal(rasterize(g, scene), oracle_rasterize(g, scene))
+        scene = Scene([Region(r) for r in rs], smooth_n=1, smooth_rad=0.1)
+        counts = rasterize_counts(g, scene)
+        np.testing.assert_array_equal(counts, oracle_counts(g, scene))
+        assert x0 > 0 or np.count_nonzero((counts > 0) & (counts < 9))
 
 
 @pytest.mark.parametrize("monitors", [1, 3, 8, 9, 700])
