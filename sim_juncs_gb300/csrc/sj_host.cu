@@ -1962,10 +1962,14 @@ void create_t(sj_sim* sim, int n, const sj_instance_desc* insts) {
     // z segments of 8 planes where 16 would leave few waves of tiles, each a
     // serial march (192^3, 1728 tiles of 16: 144 us per step against 161; 2 x
     // 192^3, 3456: 264 / 276; 3 x 192^3, 5184: 374 / 382, but 24 x 96^3, as
-    // many, 431 / 417)
+    // many, 431 / 417) and the tile codes have room for them (8192 planes)
     long long tiles16 = 0;
-    for (const InstDev<real>& I : dv) tiles16 += lean_items(I.nx, I.ny, I.nz, 16);
-    sim->l_zb = tiles16 < 3200 ? 8 : 16;
+    bool codes8 = true;
+    for (const InstDev<real>& I : dv) {
+        tiles16 += lean_items(I.nx, I.ny, I.nz, 16);
+        codes8 = codes8 && lean_codes(I.nx, I.ny, I.nz, 8);
+    }
+    sim->l_zb = tiles16 < 3200 && codes8 ? 8 : 16;
     upload_table<real>(sim);
 }
 

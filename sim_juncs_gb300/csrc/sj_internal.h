@@ -171,6 +171,7 @@ struct LeanTiles {
     bool merged;  // the plain and slab tiles are in the multi list, in the order of the grid
 };
 long long lean_items(int nx, int ny, int nz, int zb);  // tiles of one instance
+bool lean_codes(int nx, int ny, int nz, int zb);       // can a tile code name each of them?
 // two_columns: the two-column bodies may run; -1: grid too large
 template <typename real>
 int lean_classify(const InstDev<real>& I, int zb, bool two_columns, std::vector<unsigned>* lists, bool& merged);

@@ -1565,12 +1565,16 @@ long long lean_items(int nx, int ny, int nz, int zb) {
     return (long long)((nx + LX - 1) / LX) * ((ny + LY - 1) / LY) * ((nz + zb - 1) / zb);
 }
 
+bool lean_codes(int nx, int ny, int nz, int zb) {
+    return (nx + LX - 1) / LX <= 512 && (ny + LY - 1) / LY <= 1024 && (nz + zb - 1) / zb <= 1024;
+}
+
 constexpr int LEAN_MERGE_LAYER = 5 * 152;  // tiles of a merged launch that are resident at once
 
 template <typename real>
 int lean_classify(const InstDev<real>& I, int zb, bool two_columns, std::vector<unsigned>* lists, bool& merged) {
     const int ntx = (I.nx + LX - 1) / LX, nty = (I.ny + LY - 1) / LY, ntz = (I.nz + zb - 1) / zb;
-    if (ntx > 512 || nty > 1024 || ntz > 1024) return -1;
+    if (!lean_codes(I.nx, I.ny, I.nz, zb)) return -1;
     for (int c = 0; c < LEAN_CLASSES; ++c) lists[c].clear();
     for (int tz = 0; tz < ntz; ++tz)
         for (int ty = 0; ty < nty; ++ty)

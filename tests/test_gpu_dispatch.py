@@ -1,0 +1,54 @@
+"""Which launches a call takes must not change what it accepts or returns."""
+import numpy as np
+import pytest
+
+from sim_juncs_gb300 import _abi
+from sim_juncs_gb300.configs import junction_instance
+from sim_juncs_gb300.fields import Fields
+from sim_juncs_gb300.geometry import Box
+from sim_juncs_gb300.spec import PML, Grid, Probe, Region, Scene
+
+pytestmark = pytest.mark.gpu
+
+
+def equal_sims(a, b):
+    assert a.steps_done == b.steps_done
+    for q in range(a.n_instances):
+        for c in range(6):
+            np.testing.assert_array_equal(a.get_array(c, q), b.get_array(c, q), err_msg=f"instance {q} component {c}")
+        np.testing.assert_array_equal(a.monitors(q), b.monitors(q))
+        np.testing.assert_array_equal(a.dft(q), b.dft(q))
+
+
+def lit(f, inst=0):
+    return max(float(np.max(np.abs(f.get_array(c, inst)))) for c in range(6)) > 0
+
+
+def column(nz):
+    """A long thin cell: few tiles, many planes; a box and a sheet near one end."""
+    inst = junction_instance(n=32, res=20.0)
+    dx = inst.grid.dx
+    inst.grid = Grid(32, 8, nz, dx, inst.grid.dt)
+    inst.pml = PML([[0.0, 0.0], [0.0, 0.0], [0.2, 0.2]])
+    inst.material = Scene([Region(Box((0.4, 0.0, 1.0), (1.2, 0.4, 1.3)), eps=2.0)], ambient_eps=1.0)
+    src = inst.sources[0]
+    src.start_time, src.end_time = -9.0, 11.0
+    src.lo, src.hi = (0.0, 0.0, 0.8), (32 * dx, 8 * dx, 0.8)
+    inst.probes = [Probe(0, (0.8, 0.2, 0.9), dft=True)]
+    return inst
+
+
+@pytest.mark.parametrize("nz", [8192, 8193, 16384])
+def test_long_thin_grids_take_single_steps(lib, nz):
+    # more than 8192 planes do not fit the tile codes in segments of 8
+    a, b = Fields(column(nz), "f32"), Fields(column(nz), "f32")
+    b.set_tiling(8, 0, 16)
+    assert a.launches_per_step() > 0
+    for f in (a, b):
+        f.step(1)
+        f.step(20)
+        f.step_graph(1, chunk=1)
+    equal_sims(a, b)
+    assert lit(a)
+    a.close()
+    b.close()
