@@ -1405,9 +1405,22 @@ void run_steps(sj_sim* sim, long long n) {
     }
 }
 
+// What later steps would allocate, whichever launches they take, is there
+// after a sim's first: a caller may then capture runs and single steps alike.
+template <typename real>
+void prepare_steps(sj_sim* sim) {
+    bool codes = true;
+    if (sim->schedule == SJ_SCHED_FUSED)
+        for (const InstDev<real>& I : devv<real>(sim)) codes = codes && lean_codes(I.nx, I.ny, I.nz, sim->l_zb);
+    if (resident<real>(sim) && !codes) return;  // runs of steps need no tiles
+    prepare_schedule<real>(sim);
+    if (sim->schedule == SJ_SCHED_FUSED) lean_streams(sim);
+}
+
 template <typename real>
 void do_steps(sj_sim* sim, long long n) {
     ensure_capacity<real>(sim, sim->t + n);
+    prepare_steps<real>(sim);
     while (n > 0) {
         // up to the next save point, the counter current there
         long long m = n;

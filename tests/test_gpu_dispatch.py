@@ -52,3 +52,30 @@ def test_long_thin_grids_take_single_steps(lib, nz):
     assert lit(a)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("warm", [(1,) * 40, (30, 10)], ids=["single", "runs"])
+@pytest.mark.parametrize("captured", [(1, 1), (6,)], ids=["single", "run"])
+def test_warmed_up_sims_can_be_captured(lib, warm, captured):
+    # the warm-up's kind of call (single steps or runs) need not be the captured one
+    import torch
+    s = torch.cuda.Stream()
+    inst = junction_instance(n=40, res=12.5, dft=False, probe_components=())
+    a, b = Fields(inst, "f32", stream=s), Fields(inst, "f32")
+    for n in warm:
+        a.step(n)
+    a.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        for n in captured:
+            a.step(n)
+    with torch.cuda.stream(s):
+        for _ in range(3):
+            g.replay()
+    s.synchronize()
+    b.step(sum(warm) + 3 * sum(captured))
+    for c in range(6):
+        np.testing.assert_array_equal(a.get_array(c), b.get_array(c))
+    assert lit(a)
+    a.close()
+    b.close()
