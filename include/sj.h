@@ -463,18 +463,20 @@ int sj_divergence(const sj_sim* sim, int64_t* step, int32_t* inst, int32_t* moni
    runs N steps forward keeping the full state every checkpoint_every steps,
    then runs the discrete adjoint of the stepper backwards (the exact
    transpose of each sub-update: H and its CPML psi, E and its psi, the
-   polarisation ADE), re-running each segment forward from its checkpoint
-   to regenerate what the gradient needs.  d_obj_d_eps receives, instance
-   after instance, dF/d(eps) for every design voxel ([n2][n1][n0] order);
-   obj receives F per instance.  On return the instances hold the state
-   after N steps.  Memory: (N / checkpoint_every + 1) copies of the full
-   state (fields, CPML psi, polarisations) plus the E-update bracket at the
-   design points for checkpoint_every steps; the work does not depend on
-   the interval (each segment is re-run once).  checkpoint_every <= 0 or
-   >= N keeps one segment: two state copies and the bracket of all N steps,
-   the least memory whenever the design region is small.  An interval whose
-   copies do not fit the free device memory fails with SJ_E_NOMEM; an
-   instance of 2^31 voxels or more (row pitch included) with SJ_E_INVALID. */
+   polarisation ADE).  What the gradient needs of the forward pass is recorded
+   a segment at a time: of the last segment as the forward pass runs it, of
+   the others by running them forward once more from their checkpoints.
+   d_obj_d_eps receives, instance after instance, dF/d(eps) for every design
+   voxel ([n2][n1][n0] order); obj receives F per instance.  On return the
+   instances hold the state after N steps.  Memory: one copy of the full
+   state (fields, CPML psi, polarisations) per segment, N / checkpoint_every
+   rounded up, plus the E-update bracket at the design points for
+   checkpoint_every steps.  checkpoint_every <= 0 or >= N makes one segment,
+   which keeps no copy and re-runs nothing: the bracket of all N steps, the
+   least memory and work whenever the design region is small.  A call whose
+   arrays do not fit the free device memory fails with SJ_E_NOMEM before it
+   changes anything; an instance of 2^31 voxels or more (row pitch included)
+   with SJ_E_INVALID. */
 typedef struct {
     int32_t lo[3];              /* first voxel of the design box */
     int32_t n[3];               /* extent in voxels */

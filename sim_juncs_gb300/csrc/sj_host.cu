@@ -1688,21 +1688,29 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
     size_t sbytes = 0;
     for (const Arr& a : state_of(0)) sbytes += a.bytes;
     const long long nseg = (N + K - 1) / K;
-    {
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && (size_t)(nseg + 1) * sbytes > free_b) {
-            char buf[240];
-            snprintf(buf, sizeof buf,
-                     "the %lld checkpoints of %.2f GB each need %.1f GB, %.1f GB are free: use a larger "
-                     "checkpoint_every (<= 0: one segment)",
-                     nseg + 1, sbytes / 1e9, (nseg + 1) * (double)sbytes / 1e9, free_b / 1e9);
-            fail(SJ_E_NOMEM, buf);
-        }
-    }
     // the last segment is recorded as the forward pass reaches it and never
     // re-run; the segments before it need their first state, and the state
     // after N steps has to be kept only where they overwrite it
     const long long keep = backward && nseg > 1 ? nseg : 0;  // slots: segments 0 .. nseg-2, then the final state
+    if (backward) {
+        // refused before any state changes where what is allocated below cannot fit
+        size_t need = (size_t)keep * sbytes, free_b = 0, total_b = 0;
+        for (int q = 0; q < ni; ++q) {
+            const InstDev<real>& I = dv[q];
+            const size_t vb = (size_t)I.vol * sizeof(real), nd = hv[q].des_eps.size();
+            need += 9 * vb + (size_t)K * nd * 3 * sizeof(real) + nd * 3 * sizeof(double);
+            for (int ax = 0; ax < 3; ++ax) need += I.psiE[ax] ? 4 * vb : 0;
+            if (I.P) need += (size_t)I.n_poles * 6 * I.dvol * sizeof(real);
+        }
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need > free_b) {
+            char buf[240];
+            snprintf(buf, sizeof buf,
+                     "the adjoint needs %.2f GB, %.2f of them for %lld checkpoints, and %.2f GB are free: use another "
+                     "checkpoint_every (<= 0: one segment, no checkpoints)",
+                     need / 1e9, keep * (double)sbytes / 1e9, keep, free_b / 1e9);
+            fail(SJ_E_NOMEM, buf);
+        }
+    }
     char* arena = keep ? (char*)tmp((size_t)keep * sbytes, false) : nullptr;
     std::vector<int> slot_cur(keep, 0);  // the parity each checkpoint was taken at
     auto save = [&](long long slot) {

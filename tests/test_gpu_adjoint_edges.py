@@ -8,7 +8,8 @@ import numpy as np
 import pytest
 
 from oracle.oracle import OracleFields
-from sim_juncs_gb300.configs import AU, junction_instance
+from sim_juncs_gb300 import _abi
+from sim_juncs_gb300.configs import AU, adjoint_case, junction_instance
 from sim_juncs_gb300.fields import Fields
 from sim_juncs_gb300.geometry import Box
 from sim_juncs_gb300.spec import PML, Design, Grid, Objective, Region, Scene
@@ -73,3 +74,34 @@ def test_unequal_designs_in_one_sim(lib):
         F1, g1 = s.adjoint_gradient(obj, STEPS, checkpoint_every=STEPS)
         assert F1[0] == F[q]
         np.testing.assert_array_equal(g1[0], g[q])
+
+
+def test_memory_refused_is_what_would_not_fit(lib):
+    """With 30 arrays' worth of memory free, the objective (no copies of the state) and a gradient of one segment
+    (21 arrays) run; five checkpoints of 18 arrays each are refused, and the state is then as it was."""
+    import torch
+    inst, des, obj = adjoint_case(n=128, res=40.0, design_um=(0.2, 0.2, 0.1))
+    inst.material.regions[0].susceptibilities = []
+    src = inst.sources[0]
+    src.start_time, src.end_time = -9.0, 11.0
+    src.lo, src.hi = src.lo[:2] + (1.5,), src.hi[:2] + (1.5,)  # four cells below the patch
+    f = Fields(inst, "f64")
+    f.set_design(des)
+    f.step(4)
+    want = f.get_array(0)
+    array = 128 ** 3 * 8
+    free, _ = torch.cuda.mem_get_info()
+    hog = torch.empty(free - 30 * array, dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(_abi.SJError) as e:
+            f.adjoint_gradient([obj], 20, checkpoint_every=4)
+        assert e.value.code == _abi.SJ_E_NOMEM
+        assert f.steps_done == 4
+        np.testing.assert_array_equal(f.get_array(0), want)
+        F = f.objective([obj], 20)
+        Fg, g = f.adjoint_gradient([obj], 20, checkpoint_every=0)
+        assert Fg[0] == F[0] and np.max(np.abs(g[0])) > 0 and f.steps_done == 20
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    f.close()
