@@ -398,6 +398,9 @@ static size_t phase_smem(int N) {
     return (2 * (size_t)N + (L == N ? 0 : 2 * (size_t)L) + N + 2) * sizeof(double);
 }
 
+// phase_smem of the longest series (4096 samples at most, odd ones need more)
+constexpr int PH_MAX_SMEM = (2 * 4095 + 2 * 4094 + 4095 + 2) * (int)sizeof(double);
+
 long long phase_workspace(int N) { return PhaseLay(N).total; }
 
 // series q: v[q * s_series + k * s_sample], k < N; t[k] the sample times.
@@ -730,7 +733,9 @@ cudaError_t launch_phases(const double* d_v, long long s_series, long long s_sam
     if (n_series <= 0) return cudaSuccess;
     const size_t smem = phase_smem(N);
     if (smem > 32 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_phases, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the attribute is the process's: always the largest size, so that callers of
+        // several threads do not set each other's
+        cudaError_t e = cudaFuncSetAttribute(k_phases, cudaFuncAttributeMaxDynamicSharedMemorySize, PH_MAX_SMEM);
         if (e != cudaSuccess) return e;
     }
     k_phases<<<n_series, PH_THREADS, smem, s>>>(d_v, s_series, s_sample, N, d_t, lowpass_inc, d_work,

@@ -94,3 +94,25 @@ def test_sweep_sized_batch_equals_series_one_at_a_time(lib, golden):
     for q in range(8):
         one = extract_phases(t, v[q:q + 1], LOWPASS_INC)[0]
         assert allr[q] == one and allr[q + 8 * 47] == one
+
+
+def pulses(n, count):
+    t = np.arange(n) * 0.05
+    c = 0.025 * n
+    return t, np.stack([np.exp(-((t - c) / (0.2 * c)) ** 2) * np.cos(2 * np.pi * 1.4 * (t - c) + p)
+                        for p in np.linspace(0.1, 5.0, count)])
+
+
+def test_threads_with_series_of_different_lengths(lib):
+    # each length wants another size of shared memory; calls of other threads must not change it
+    from concurrent.futures import ThreadPoolExecutor
+    lengths = (1366, 1700, 2001, 3001)
+    want = {n: extract_phases(*pulses(n, 2)) for n in lengths}
+
+    def run(n):
+        t, v = pulses(n, 2)
+        return all(extract_phases(t, v) == want[n] for _ in range(400))
+
+    assert all(w[0]["status"] == _abi.PHASE_OK for w in want.values())
+    with ThreadPoolExecutor(len(lengths)) as ex:
+        assert all(f.result() for f in [ex.submit(run, n) for n in lengths])
