@@ -2688,7 +2688,8 @@ int sj_extract_phases(int32_t n_series, int32_t n_samples, const double* t_pts, 
     sj_phase_result* d_out = reinterpret_cast<sj_phase_result*>(d_w + nw);
     cudaStream_t s = nullptr;
     cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_v, v, nv * sizeof(double), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(d_v, v, (size_t)n_series * n_samples * sizeof(double), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_t, t_pts, n_samples * sizeof(double), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = launch_phases(d_v, n_samples, 1, n_series, n_samples, d_t, lowpass_inc, d_w, d_out, s);
     if (e == cudaSuccess)

@@ -116,3 +116,24 @@ def test_threads_with_series_of_different_lengths(lib):
     assert all(w[0]["status"] == _abi.PHASE_OK for w in want.values())
     with ThreadPoolExecutor(len(lengths)) as ex:
         assert all(f.result() for f in [ex.submit(run, n) for n in lengths])
+
+
+def test_series_are_read_to_their_end_only(lib):
+    # the last sample ends a page, and the next page may not be read
+    import ctypes as C
+    import mmap
+    libc = C.CDLL(None, use_errno=True)
+    libc.mprotect.argtypes = [C.c_void_p, C.c_size_t, C.c_int]
+    page = mmap.PAGESIZE
+    t, v = pulses(101, 3)
+    size = -(-v.nbytes // page) * page
+    m = mmap.mmap(-1, size + page)
+    base = C.addressof(C.c_char.from_buffer(m))
+    assert libc.mprotect(base + size, page, 0) == 0
+    try:
+        end = np.frombuffer(m, dtype=np.float64, count=v.size, offset=size - v.nbytes).reshape(v.shape)
+        end[:] = v
+        want = extract_phases(t, v)
+        assert extract_phases(t, end) == want
+    finally:
+        assert libc.mprotect(base + size, page, mmap.PROT_READ | mmap.PROT_WRITE) == 0
