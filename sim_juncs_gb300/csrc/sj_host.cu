@@ -158,7 +158,7 @@ struct sj_sim {
     // TMA schedule: tiling, tensor maps, block prefixes
     int f_ty = 8, f_zs = 64, f_ring = 3;
     bool fused_ready = false;
-    unsigned long long tma_wait_ns = 0;  // limit of a wait on a TMA copy (0 = the kernel's 100 ms)
+    unsigned long long wait_ns = 0;      // sj_set_wait_limit (0: 100 ms on a TMA copy, RES_WAIT_NS at the grid barrier)
     int test_stall = 0;                  // sj_set_test_stall
     FusedLaunch fl{};
     void* d_fpre = nullptr;
@@ -981,7 +981,7 @@ void prepare_fused(sj_sim* sim) {
     fl.d_item_pre = reinterpret_cast<const long long*>(sim->d_fpre);
     fl.d_probe_pre = reinterpret_cast<const long long*>(sim->d_fpre) + (n + 1);
     fl.dry = 0;
-    fl.wait_ns = sim->tma_wait_ns;
+    fl.wait_ns = sim->wait_ns;
     fl.stall = sim->test_stall;
     upload_table<real>(sim);
     sim->fused_ready = true;
@@ -1358,7 +1358,7 @@ void take_snapshot_async(sj_sim* sim, int q) {
 template <typename real>
 constexpr long long res_max_voxels() { return sizeof(real) == 4 ? 1LL << 22 : 1LL << 27; }
 constexpr int RES_CHUNK = 256;                                // steps per launch
-constexpr unsigned long long RES_WAIT_NS = 4000000000ull;     // limit of a wait at the grid barrier
+constexpr unsigned long long RES_WAIT_NS = 4000000000ull;     // default limit of a wait at the grid barrier
 
 // Do runs of steps go through the resident kernel?
 template <typename real>
@@ -1386,7 +1386,8 @@ void run_resident(sj_sim* sim, long long n, const ObjDev<real>* d_obj = nullptr,
     const InstDev<real>* d = reinterpret_cast<const InstDev<real>*>(sim->d_table);
     for (; n > 0; n -= RES_CHUNK)
         ck(launch_resident<real>(devv<real>(sim).data(), d, sim->n_inst, sim->cur, (int)std::min<long long>(n, RES_CHUNK),
-                                 sim->r_blocks, d_obj, obj_blocks, sim->d_bar, RES_WAIT_NS, sim->d_state, sim->stream),
+                                 sim->r_blocks, d_obj, obj_blocks, sim->d_bar, sim->wait_ns ? sim->wait_ns : RES_WAIT_NS,
+                                 sim->test_stall, sim->d_state, sim->stream),
            "resident launch");
 }
 
@@ -1534,12 +1535,17 @@ void set_guard_t(sj_sim* sim, double bound) {
     upload_table<real>(sim);
 }
 
-int check_status(sj_sim* sim) {
+// waits for the stream; fails with what its kernels reported
+DevState kernel_status(sj_sim* sim) {
     DevState st;
     ck(cudaStreamSynchronize(sim->stream), "sync");
     ck(cudaMemcpy(&st, sim->d_state, sizeof(st), cudaMemcpyDeviceToHost), "state");
     if (st.status != 0) fail(st.status, "a kernel reported status " + std::to_string(st.status));
-    if (st.step != sim->t) fail(SJ_E_CUDA, "device step counter disagrees with host");
+    return st;
+}
+
+int check_status(sj_sim* sim) {
+    if (kernel_status(sim).step != sim->t) fail(SJ_E_CUDA, "device step counter disagrees with host");
     return 0;
 }
 
@@ -1618,14 +1624,16 @@ void set_design_t(sj_sim* sim, int q, const sj_design_desc* d) {
     if (sim->schedule == SJ_SCHED_FUSED) prepare_lean<real>(sim);
 }
 
+// The device's step counter; the status kernels have left stays unless `clear`.
 template <typename real>
-void set_dev_step(sj_sim* sim, long long step) {
+void set_dev_step(sj_sim* sim, long long step, bool clear = false) {
     DevState st{};
     st.step = step;
     st.done = 0;
     st.cur = sim->cur;
     st.status = 0;
-    ck(cudaMemcpyAsync(sim->d_state, &st, sizeof(st), cudaMemcpyHostToDevice, sim->stream), "state");
+    ck(cudaMemcpyAsync(sim->d_state, &st, clear ? sizeof(st) : offsetof(DevState, status), cudaMemcpyHostToDevice, sim->stream),
+       "state");
     ck(cudaStreamSynchronize(sim->stream), "sync");
 }
 
@@ -1768,7 +1776,7 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
     for (int q = 0; q < ni; ++q)
         if (dv[q].dft) ck(cudaMemsetAsync(dv[q].dft, 0, (size_t)hv[q].n_dft * hv[q].n_freq * sizeof(double2), st), "reset");
     sim->t = 0;
-    set_dev_step<real>(sim, 0);
+    set_dev_step<real>(sim, 0, true);
     for (long long seg = 0; seg < nseg; ++seg) {
         const long long t0 = seg * K, t1 = std::min(N, t0 + K);
         if (seg < nseg - 1)
@@ -1787,7 +1795,7 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
     record(0, 0);
     if (keep) save(nseg - 1);
     std::vector<std::vector<double2>> dft_keep(ni);
-    ck(cudaStreamSynchronize(st), "sync");
+    kernel_status(sim);
     for (int q = 0; q < ni; ++q) {
         if (keep && dv[q].dft) {
             dft_keep[q].resize((size_t)hv[q].n_dft * hv[q].n_freq);
@@ -1861,7 +1869,7 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
                 ck(cudaMemcpy(dv[q].dft, dft_keep[q].data(), dft_keep[q].size() * sizeof(double2), cudaMemcpyHostToDevice),
                    "dft");
     }
-    ck(cudaStreamSynchronize(st), "sync");
+    kernel_status(sim);
     // ---- dF/d(eps) = -eps^{-2} sum_c dF/d(inverse eps at the voxel's E_c point)
     long long off = 0;
     for (int q = 0; q < ni; ++q) {
@@ -2214,8 +2222,8 @@ int sj_set_wait_limit(sj_sim* sim, int64_t ns) {
     if (ns < 0 || ns > 10000000000ll) return finish(sim, SJ_E_INVALID, "wait limit must be in [0, 10 s]");
     SJ_TRY(sim)
     ck(cudaStreamSynchronize(sim->stream), "sync");
-    sim->tma_wait_ns = (unsigned long long)ns;
-    sim->fl.wait_ns = sim->tma_wait_ns;
+    sim->wait_ns = (unsigned long long)ns;
+    sim->fl.wait_ns = sim->wait_ns;
     sim->drop_graphs();
     SJ_CATCH(sim)
 }

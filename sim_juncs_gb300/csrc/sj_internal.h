@@ -291,7 +291,7 @@ cudaError_t launch_objective(const ObjDev<real>* o, int n_inst, int cur, long lo
 // the blocks of the kernel that fit the device at once (0: it cannot run).
 // d_obj (or null): objectives whose DFT sums the launch keeps, obj_blocks =
 // resident_objective_blocks of them.  d_bar: the barrier's counter, zeroed by
-// the launch.
+// the launch.  limit_ns: of a wait at the barrier; stall: sj_set_test_stall.
 constexpr int RES_MAX_INST = 32;  // instances of one resident launch
 template <typename real>
 int resident_grid(const InstDev<real>* h_insts, int n_inst);
@@ -300,7 +300,7 @@ int resident_objective_blocks(const InstDev<real>* h_insts, const ObjDev<real>* 
 template <typename real>
 cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d_insts, int n_inst, int cur,
                             int n_steps, int max_blocks, const ObjDev<real>* d_obj, int obj_blocks, unsigned* d_bar,
-                            unsigned long long limit_ns, DevState* st, cudaStream_t s);
+                            unsigned long long limit_ns, int stall, DevState* st, cudaStream_t s);
 
 // Diagnostics (sj_diag.cu): the discrete energy (scale * sum, partial sums in
 // d_partial[energy_partials()]) and the flux spectrum of DFT-probe rows.

@@ -81,7 +81,8 @@ __device__ __forceinline__ Cell res_cell(const ResGrid& G, unsigned t) {
 
 // Grid barrier: every block arrives with release, waits for `target`
 // arrivals with acquire.  A wait that does not end within `limit` ns records
-// SJ_E_TIMEOUT and ends the launch (false, block-uniform).
+// SJ_E_TIMEOUT and ends the launch (false, block-uniform); launches queued
+// behind it return at once (k_resident).
 __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, unsigned long long limit, DevState* st) {
     __shared__ int ok;
     __syncthreads();
@@ -549,11 +550,17 @@ template <typename real, int T, bool ONE, bool DES>
 __global__ void __launch_bounds__(T, 1)
 k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __restrict__ tab, int n_inst, int cur,
            int n_steps, int workers, int probe_blocks, int h_probes, int one_chunk, const ObjDev<real>* __restrict__ obj,
-           unsigned* bar, unsigned long long limit, DevState* st) {
+           unsigned* bar, unsigned long long limit, int stall, DevState* st) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ ResGrid grids[RES_MAX_INST];
+    __shared__ int gone;
     constexpr unsigned CH = res_chunk<real, T>(), SLOTS = T / CH;
     const long long n0 = st->step;
+    // a launch before this one gave up: its state is not to be stepped on.
+    // stall (sj_set_test_stall): the first block never arrives at a barrier.
+    if (threadIdx.x == 0) gone = st->status == SJ_E_TIMEOUT || (stall && blockIdx.x == 0);
+    __syncthreads();
+    if (gone) return;
     if ((int)blockIdx.x >= workers) {
         int b = (int)blockIdx.x - workers;
         if (b < probe_blocks) {
@@ -674,7 +681,7 @@ int resident_objective_blocks(const InstDev<real>* h_insts, const ObjDev<real>* 
 template <typename real>
 cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d_insts, int n_inst, int cur,
                             int n_steps, int max_blocks, const ObjDev<real>* d_obj, int obj_blocks, unsigned* d_bar,
-                            unsigned long long limit_ns, DevState* st, cudaStream_t s) {
+                            unsigned long long limit_ns, int stall, DevState* st, cudaStream_t s) {
     long long cells = 0, chunks = 0;
     int h_probes = 0;
     bool des = d_obj != nullptr;
@@ -695,8 +702,8 @@ cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d
     if (e != cudaSuccess) return e;
     InstDev<real> one = h_insts[0];
     int one_chunk = chunks <= probe;
-    void* args[] = {&one,      &d_insts,   &n_inst, &cur,   &n_steps,  &w, &probe,
-                    &h_probes, &one_chunk, &d_obj,  &d_bar, &limit_ns, &st};
+    void* args[] = {&one,      &d_insts,   &n_inst, &cur,   &n_steps,  &w,     &probe,
+                    &h_probes, &one_chunk, &d_obj,  &d_bar, &limit_ns, &stall, &st};
     const size_t smem = n_inst > 1 ? (size_t)n_inst * sizeof(InstDev<real>) : 0;
     return cudaLaunchCooperativeKernel(res_kernel<real>(few, n_inst, des), dim3(w + probe + obj_blocks), dim3(T), args,
                                        smem, s);
@@ -707,10 +714,10 @@ template int resident_grid<double>(const InstDev<double>*, int);
 template int resident_objective_blocks<float>(const InstDev<float>*, const ObjDev<float>*, int);
 template int resident_objective_blocks<double>(const InstDev<double>*, const ObjDev<double>*, int);
 template cudaError_t launch_resident<float>(const InstDev<float>*, const InstDev<float>*, int, int, int, int,
-                                            const ObjDev<float>*, int, unsigned*, unsigned long long, DevState*,
-                                            cudaStream_t);
+                                            const ObjDev<float>*, int, unsigned*, unsigned long long, int,
+                                            DevState*, cudaStream_t);
 template cudaError_t launch_resident<double>(const InstDev<double>*, const InstDev<double>*, int, int, int, int,
-                                             const ObjDev<double>*, int, unsigned*, unsigned long long, DevState*,
-                                             cudaStream_t);
+                                             const ObjDev<double>*, int, unsigned*, unsigned long long, int,
+                                             DevState*, cudaStream_t);
 
 }  // namespace sj

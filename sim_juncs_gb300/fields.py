@@ -310,12 +310,14 @@ class Fields:
 
     # ------------------------------------------------------------ bounded waits
     def set_wait_limit(self, ns):
-        """Limit of a TMA-schedule wait on a tile copy (0 = the default 100 ms)."""
+        """Limit of a TMA-schedule wait on a tile copy (0 = the default 100 ms) and
+        of a small grid's run of steps at its grid barrier (0 = 4 s)."""
         self._ck(self.lib.sj_set_wait_limit(self.handle, int(ns)))
 
     def set_test_stall(self, on):
-        """Test hook: the TMA schedule's first tile block skips a plane's
-        copy, so its wait runs out and SJ_E_TIMEOUT is reported."""
+        """Test hook: the TMA schedule's first tile block skips a plane's copy,
+        and a resident run's first block never arrives at the grid barrier, so
+        the wait runs out and SJ_E_TIMEOUT is reported."""
         self._ck(self.lib.sj_set_test_stall(self.handle, 1 if on else 0))
 
     # ------------------------------------------------------------ divergence guard

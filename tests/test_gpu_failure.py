@@ -6,14 +6,16 @@ huge value or a NaN written into Ex through sj_write_field before a save
 point.  The bounded waits of the TMA schedule are exercised with the test
 hook that leaves one plane's copy unissued, so a wait on it runs out after a
 short limit; the kernel returns, SJ_E_TIMEOUT reaches the host, and the
-context stays usable for the next simulation.
+context stays usable for the next simulation.  The grid barrier of small
+grids' runs of steps likewise, with a block that does not arrive.
 """
 import numpy as np
 import pytest
 
 from sim_juncs_gb300 import _abi
-from sim_juncs_gb300.configs import junction_instance
+from sim_juncs_gb300.configs import inverse_design_case, junction_instance
 from sim_juncs_gb300.fields import Fields
+from sim_juncs_gb300.spec import Probe
 
 pytestmark = pytest.mark.gpu
 
@@ -102,3 +104,40 @@ def test_tma_wait_runs_out_and_context_stays_usable(lib):
     b.step(30)
     ea, eb = a.get_array(_abi.EX), b.get_array(_abi.EX)
     assert np.max(np.abs(ea - eb)) <= 1e-5 * np.max(np.abs(eb))
+
+
+@pytest.mark.parametrize("kind", ["cells", "probes", "objective"])
+def test_resident_wait_runs_out_and_context_stays_usable(lib, kind):
+    """The grid barrier of a run of steps: worker, probe and objective blocks all give up within the limit, the
+    launches queued behind do nothing, the error is reported once and the next simulation is sound."""
+    import time
+    inst, des, obj = inverse_design_case(0, n=72, design_um=(0.4, 0.3, 0.1), patch=5)
+    if kind == "cells":
+        inst.probes, inst.freqs = [], []
+    if kind == "probes":
+        inst.probes = [Probe(c, (1.2, 1.2, 1.2), dft=True) for c in (0, 4)]
+        inst.freqs = [1.4]
+    f = Fields(inst, "f32")
+    f.step(40)
+    f.synchronize()
+    f.set_wait_limit(50_000_000)               # 50 ms
+    f.set_test_stall(True)
+    t0 = time.perf_counter()
+    with pytest.raises(_abi.SJError) as e:
+        if kind == "objective":
+            f.objective([obj], 2000)           # eight launches
+        else:
+            f.step(2000)
+            f.synchronize()
+    assert e.value.code == _abi.SJ_E_TIMEOUT
+    assert time.perf_counter() - t0 < 0.3      # one wait, not one per launch
+    f.close()
+    a, b = Fields(inst, "f32"), Fields(inst, "f32")
+    b.set_tiling(8, 0, 8)
+    a.step(30)
+    b.step(30)
+    for c in range(6):
+        np.testing.assert_array_equal(a.get_array(c), b.get_array(c))
+    assert a.objective([obj], 40)[0] == b.objective([obj], 40)[0]
+    a.close()
+    b.close()
