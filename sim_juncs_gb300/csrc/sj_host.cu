@@ -1376,7 +1376,7 @@ bool resident(sj_sim* sim) {
         sim->r_blocks = resident_grid<real>(devv<real>(sim).data(), sim->n_inst);
         if (sim->r_blocks > 0) sim->d_bar = (unsigned*)sim->dalloc(sizeof(unsigned));
     }
-    return sim->r_blocks > 0;
+    return sim->r_blocks > 0 && resident_pays<real>(devv<real>(sim).data(), sim->n_inst, sim->r_blocks);
 }
 
 // n steps in cooperative launches of up to RES_CHUNK; the caller's step mirror

@@ -289,12 +289,15 @@ cudaError_t launch_objective(const ObjDev<real>* o, int n_inst, int cur, long lo
 // Small grids (sj_resident.cu): n_steps steps in one cooperative launch of at
 // most max_blocks resident blocks, in place in buffer `cur`.  resident_grid:
 // the blocks of the kernel that fit the device at once (0: it cannot run).
+// resident_pays: false where the probes outweigh what the steps gain.
 // d_obj (or null): objectives whose DFT sums the launch keeps, obj_blocks =
 // resident_objective_blocks of them.  d_bar: the barrier's counter, zeroed by
 // the launch.  limit_ns: of a wait at the barrier; stall: sj_set_test_stall.
 constexpr int RES_MAX_INST = 32;  // instances of one resident launch
 template <typename real>
 int resident_grid(const InstDev<real>* h_insts, int n_inst);
+template <typename real>
+bool resident_pays(const InstDev<real>* h_insts, int n_inst, int max_blocks);
 template <typename real>
 int resident_objective_blocks(const InstDev<real>* h_insts, const ObjDev<real>* o, int n_inst);
 template <typename real>

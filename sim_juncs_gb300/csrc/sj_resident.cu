@@ -22,6 +22,7 @@
 // (H^{n-1/2}) during the E phase of step n-1, which does not write H.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 
 #include "sj_physics.cuh"
 
@@ -416,15 +417,15 @@ __device__ __forceinline__ void res_sample(const InstDev<real>& I, const Probe<r
 }
 
 // The E or H probes (h) of every instance at step n.  Block b of nb takes
-// every nb-th chunk of blockDim.x probes.
+// every nb-th chunk of `per` probes.
 template <typename real>
 __device__ __forceinline__ void res_probes(const InstDev<real>* tab, int n_inst, int cur, long long n, int h, int b,
-                                           int nb, DevState* st, double2* ph) {
+                                           int nb, int per, DevState* st, double2* ph) {
     int item = 0;
     for (int q = 0; q < n_inst; ++q) {
         const InstDev<real>& I = tab[q];
         const bool save = n % I.save_span == 0;
-        const int chunks = (I.n_probe + (int)blockDim.x - 1) / (int)blockDim.x;
+        const int chunks = (I.n_probe + per - 1) / per;
         if (!chunks || (!save && !I.n_dft)) {
             item += chunks;
             continue;
@@ -438,8 +439,8 @@ __device__ __forceinline__ void res_probes(const InstDev<real>* tab, int n_inst,
                 __syncthreads();
             }
             have = true;
-            const int p = c * blockDim.x + threadIdx.x;
-            if (p >= I.n_probe || (I.probe_comp[p] >= 3) != (h != 0)) continue;
+            const int p = c * per + (int)threadIdx.x;
+            if ((int)threadIdx.x >= per || p >= I.n_probe || (I.probe_comp[p] >= 3) != (h != 0)) continue;
             res_sample(I, res_probe(I, cur, p), n, save, I.n_freq, st, ph);
         }
     }
@@ -487,36 +488,36 @@ __device__ __noinline__ void res_objective_block(const ObjDev<real>& O, int cur,
 // formed while the cells of the phase before are updated.
 template <typename real>
 __device__ __noinline__ void res_probe_block(const InstDev<real>* tab, int n_inst, int cur, long long n0, int n_steps,
-                                             int b, int nb, int h_probes, int one_chunk, unsigned* bar,
+                                             int b, int nb, int per, int h_probes, int one_chunk, unsigned* bar,
                                              unsigned long long limit, DevState* st) {
     __shared__ double2 ph[2][RES_MAXF];
     unsigned target = 0;
     if (!one_chunk) {
         if (h_probes) {
-            res_probes<real>(tab, n_inst, cur, n0, 1, b, nb, st, ph[1]);
+            res_probes<real>(tab, n_inst, cur, n0, 1, b, nb, per, st, ph[1]);
             if (!grid_barrier(bar, target += gridDim.x, limit, st)) return;
         }
         for (int s = 0; s < n_steps; ++s) {
             const bool more = s + 1 < n_steps;
-            res_probes<real>(tab, n_inst, cur, n0 + s, 0, b, nb, st, ph[0]);
+            res_probes<real>(tab, n_inst, cur, n0 + s, 0, b, nb, per, st, ph[0]);
             if (!grid_barrier(bar, target += gridDim.x, limit, st)) return;
-            if (h_probes && more) res_probes<real>(tab, n_inst, cur, n0 + s + 1, 1, b, nb, st, ph[1]);
+            if (h_probes && more) res_probes<real>(tab, n_inst, cur, n0 + s + 1, 1, b, nb, per, st, ph[1]);
             if (more && !grid_barrier(bar, target += gridDim.x, limit, st)) return;
         }
         return;
     }
     int item = 0, q = 0, chunk = 0;
     for (; q < n_inst; ++q) {
-        const int chunks = (tab[q].n_probe + (int)blockDim.x - 1) / (int)blockDim.x;
+        const int chunks = (tab[q].n_probe + per - 1) / per;
         chunk = b - item;
         item += chunks;
         if (b < item) break;
     }
     const InstDev<real>& I = tab[q];
-    const int p = chunk * (int)blockDim.x + (int)threadIdx.x, n_freq = I.n_freq;
+    const int p = chunk * per + (int)threadIdx.x, n_freq = I.n_freq;
     Probe<real> r;
     r.comp = -1;
-    if (p < I.n_probe) r = res_probe(I, cur, p);
+    if ((int)threadIdx.x < per && p < I.n_probe) r = res_probe(I, cur, p);
     const int kind = r.comp < 0 ? -1 : r.comp >= 3;  // 0: an E probe, 1: an H probe
     const bool dft = I.n_dft > 0;
     long long until = n0 % I.save_span;              // steps to the next save point
@@ -549,7 +550,7 @@ __device__ __noinline__ void res_probe_block(const InstDev<real>* tab, int n_ins
 template <typename real, int T, bool ONE, bool DES>
 __global__ void __launch_bounds__(T, 1)
 k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __restrict__ tab, int n_inst, int cur,
-           int n_steps, int workers, int probe_blocks, int h_probes, int one_chunk, const ObjDev<real>* __restrict__ obj,
+           int n_steps, int workers, int probe_blocks, int per, int h_probes, int one_chunk, const ObjDev<real>* __restrict__ obj,
            unsigned* bar, unsigned long long limit, int stall, DevState* st) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ ResGrid grids[RES_MAX_INST];
@@ -564,7 +565,8 @@ k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __res
     if ((int)blockIdx.x >= workers) {
         int b = (int)blockIdx.x - workers;
         if (b < probe_blocks) {
-            res_probe_block<real>(tab, n_inst, cur, n0, n_steps, b, probe_blocks, h_probes, one_chunk, bar, limit, st);
+            res_probe_block<real>(tab, n_inst, cur, n0, n_steps, b, probe_blocks, per, h_probes, one_chunk, bar, limit,
+                                  st);
             return;
         }
         if constexpr (DES) {
@@ -649,7 +651,79 @@ bool res_few(const InstDev<real>* h_insts, int n_inst) {
     for (int q = 0; q < n_inst; ++q) cells += (long long)h_insts[q].nx * h_insts[q].ny * h_insts[q].nz;
     return cells < RES_FEW_CELLS;
 }
+
+// How the probes of a launch are dealt out, and ns per step of the cells and
+// of the probes (E probes ride on the H phase, H probes on the E phase).
+// Fitted to runs with 1000 to 200000 probes of 5 to 256 frequencies on 64^3 and
+// 128^3: a block takes 18 ns for a probe (its stencil, indexes and weights from
+// L2) and 2.6 ns for each of its DFT sums (a row is its own thread's: 32-byte
+// sectors read and written by one SM), at least 250 ns per frequency (a
+// thread's sums go through L2 four at a time).  So the probes' blocks are as
+// many as keep them within half a step of the cells, at most an eighth of the
+// grid: every thread takes a probe where that gives as many, else fewer do
+// (64^3 FP32, 1000 probes of 50 frequencies: 141 us per step in one block, 33
+// in eleven; 10000 of 5: 34 and 22).
+struct ProbePlan {
+    int blocks, per;         // probe blocks, probes per chunk
+    long long chunks;
+    double cells, probes[2]; // ns
+};
+template <typename real>
+ProbePlan probe_plan(const InstDev<real>* h_insts, int n_inst, int max_blocks) {
+    const int T = res_threads<real>(res_few(h_insts, n_inst)), most = std::max(1, max_blocks / 8);
+    ProbePlan P = {};
+    double cells = 0, ns[2] = {0, 0}, chain = 0;
+    long long total = 0;
+    for (int q = 0; q < n_inst; ++q) {
+        const InstDev<real>& I = h_insts[q];
+        cells += (double)I.nx * I.ny * I.nz;
+        total += I.n_probe;
+        const double each = I.n_probe ? 18.0 / (I.n_dft ? 1 : I.save_span) + 2.6 * I.n_dft * I.n_freq / I.n_probe : 0.0;
+        ns[0] += each * (I.n_probe - I.n_hprobe);
+        ns[1] += each * I.n_hprobe;
+        if (I.n_dft) chain = std::max(chain, 250.0 * I.n_freq);
+    }
+    P.cells = sizeof(real) == 4 ? 5000 + 0.021 * cells : 9000 + 0.066 * cells;
+    const auto chunks = [&](int per) {
+        long long c = 0;
+        for (int q = 0; q < n_inst; ++q) c += (h_insts[q].n_probe + per - 1) / per;
+        return c;
+    };
+    P.per = T;
+    const double want = std::min<double>(most, std::ceil(2 * std::max(ns[0], ns[1]) / P.cells));
+    if (want > (double)chunks(T)) {
+        P.per = std::min(T, ((int)std::ceil(total / want) + 31) / 32 * 32);
+        while (P.per < T && chunks(P.per) > most) P.per += 32;
+        P.per = std::min(P.per, T);
+    }
+    P.chunks = chunks(P.per);
+    P.blocks = (int)std::min<long long>(P.chunks, most);
+    if (P.chunks) {
+        const double rounds = (double)((P.chunks + P.blocks - 1) / P.blocks);
+        for (int h = 0; h < 2; ++h)
+            P.probes[h] = std::max(ns[h] ? chain : 0.0, ns[h] / total * std::min<double>(rounds * P.per, (double)total));
+    }
+    return P;
+}
 }  // namespace
+
+// Does a run of steps with these probes take less time here than as tile
+// launches, whose probes are spread over the whole device?  us per step of the
+// tile launches, without probes: FP32 64^3 41, 128^3 77, 160^3 102; FP64 64^3
+// 71, 128^3 240, 256 x 256 x 192 974.  64^3 FP32 with 10000 probes of 50
+// frequencies: 142 us here, 45 there; 50000: 432 and 50; 128^3 FP64 with 200000:
+// 1441 and 370.
+template <typename real>
+bool resident_pays(const InstDev<real>* h_insts, int n_inst, int max_blocks) {
+    const ProbePlan P = probe_plan(h_insts, n_inst, max_blocks);
+    if (!P.chunks) return true;
+    double cells = 0;
+    for (int q = 0; q < n_inst; ++q) cells += (double)h_insts[q].nx * h_insts[q].ny * h_insts[q].nz;
+    const double tiles = sizeof(real) == 4 ? 35000 + 0.0165 * cells : 50000 + 0.075 * cells;
+    return std::max(P.cells / 2, P.probes[0]) + std::max(P.cells / 2, P.probes[1]) <= tiles;
+}
+template bool resident_pays<float>(const InstDev<float>*, int, int);
+template bool resident_pays<double>(const InstDev<double>*, int, int);
 
 template <typename real>
 int resident_grid(const InstDev<real>* h_insts, int n_inst) {
@@ -682,7 +756,7 @@ template <typename real>
 cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d_insts, int n_inst, int cur,
                             int n_steps, int max_blocks, const ObjDev<real>* d_obj, int obj_blocks, unsigned* d_bar,
                             unsigned long long limit_ns, int stall, DevState* st, cudaStream_t s) {
-    long long cells = 0, chunks = 0;
+    long long cells = 0;
     int h_probes = 0;
     bool des = d_obj != nullptr;
     const bool few = res_few(h_insts, n_inst);
@@ -690,19 +764,18 @@ cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d
     for (int q = 0; q < n_inst; ++q) {
         const InstDev<real>& I = h_insts[q];
         cells += (long long)I.nx * I.ny * I.nz;
-        chunks += (I.n_probe + T - 1) / T;
         h_probes |= I.n_hprobe > 0;
         des |= I.dinv != nullptr;
     }
-    // probe blocks: each takes one chunk a phase where that leaves most of the grid to the cells
-    int probe = (int)std::min<long long>(chunks, std::max(1, max_blocks / 8));
+    ProbePlan plan = probe_plan(h_insts, n_inst, max_blocks);
+    int probe = plan.blocks;
     int w = (int)std::min<long long>((cells + T - 1) / T, max_blocks - probe - obj_blocks);
     if (w < 1) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(d_bar, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     InstDev<real> one = h_insts[0];
-    int one_chunk = chunks <= probe;
-    void* args[] = {&one,      &d_insts,   &n_inst, &cur,   &n_steps,  &w,     &probe,
+    int one_chunk = plan.chunks <= probe;
+    void* args[] = {&one,      &d_insts,   &n_inst, &cur,   &n_steps,  &w,     &probe, &plan.per,
                     &h_probes, &one_chunk, &d_obj,  &d_bar, &limit_ns, &stall, &st};
     const size_t smem = n_inst > 1 ? (size_t)n_inst * sizeof(InstDev<real>) : 0;
     return cudaLaunchCooperativeKernel(res_kernel<real>(few, n_inst, des), dim3(w + probe + obj_blocks), dim3(T), args,

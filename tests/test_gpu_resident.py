@@ -106,3 +106,31 @@ def test_design_and_objective_through_both_paths(lib, precision):
             np.testing.assert_array_equal(x, y)
     for x, y in zip(out[0][2], out[1][2]):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("counts,freqs", [((1000,), 50), ((33,), 20), ((700, 31, 0, 400), 30), ((9000,), 40)],
+                         ids=["small chunks", "one over a warp", "several grids", "more than pays"])
+def test_probes_dealt_out_over_blocks(lib, precision, counts, freqs):
+    """Probe blocks with fewer probes than threads, chunks that end inside an instance, instances without probes, and
+    so many that the run goes to the tile launches: every sum as the tile launches form it."""
+    rng = np.random.default_rng(3)
+    insts = []
+    for n in counts:
+        inst = junction_instance(n=36, res=11.25, probe_components=(), save_span=2)
+        inst.sources[0].start_time, inst.sources[0].end_time = -9.0, 11.0
+        at = rng.uniform(0.3, 2.9, size=(n, 3))
+        inst.probes = [Probe((0, 4, 2, 3)[q % 4], tuple(at[q]), monitor=q % 5 == 0, dft=q % 7 != 0) for q in range(n)]
+        inst.freqs = list(np.linspace(0.8, 2.0, freqs))
+        insts.append(inst)
+    a, b = Fields(insts, precision), Fields(insts, precision)
+    b.set_tiling(8, 0, 8)
+    for n in (21, 1, 20):
+        a.step(n)
+    b.step(42)
+    for q in range(len(insts)):
+        np.testing.assert_array_equal(a.monitors(q), b.monitors(q))
+        np.testing.assert_array_equal(a.dft(q), b.dft(q))
+        assert not len(insts[q].probes) or np.max(np.abs(a.dft(q))) > 0
+    a.close()
+    b.close()
