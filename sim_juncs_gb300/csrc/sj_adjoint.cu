@@ -19,8 +19,8 @@
 // from k_adj_h to the next k_adj_e.  A psi adjoint is kept as T, the value
 // before its factor b: the difference's adjoint is cv + c T, and b T enters
 // the next T, so neighbours need no arrays of their own for either.
-// The objective's dF/dE^n source is added to eb between the steps, by one
-// block of k_adj_h (which does not touch eb).  The gradient with respect to a
+// The objective's dF/dE^n source is added to eb between the steps, by blocks
+// of k_adj_h's launch of their own (its cells do not touch eb).  The gradient with respect to a
 // design voxel's inverse eps is sum_n dF/dE^{n+1} * acc^n, acc^n being the E
 // update's bracket at step n, recorded while the segment is run forward.
 //
@@ -368,23 +368,22 @@ k_adj_e(const __grid_constant__ AdjDev<real> A, long long n, int zs) {
 
 // dF/dH^{n+1/2} += what the E update's differences read from H at this cell,
 // then the transpose of the H update's psi; hb itself carries over to
-// H^{n-1/2}.  The last block column adds the objective's dF/dE^n to eb.
+// H^{n-1/2}.  The block columns from cell_blocks on add the objective's
+// dF/dE^n to eb, a thread per cell and component.
 template <typename real, int W>
 __global__ void __launch_bounds__(ADJ_THREADS, adj_minb<real>())
-k_adj_h(const __grid_constant__ AdjDev<real> A, long long n, int zs) {
+k_adj_h(const __grid_constant__ AdjDev<real> A, long long n, int zs, unsigned cell_blocks) {
     const InstDev<real>& I = A.I;
-    if (blockIdx.x == gridDim.x - 1) {
-        if (blockIdx.y) return;
+    if (blockIdx.x >= cell_blocks) {
+        const unsigned t = ((blockIdx.x - cell_blocks) * gridDim.y + blockIdx.y) * ADJ_THREADS + threadIdx.x;
+        const unsigned q = t / 3, c = t % 3;
+        if (q >= (unsigned)A.n_cells || !((A.comp_mask >> c) & 1)) return;
         double sn, cs;
         sincospi(2.0 * A.freq * ((double)n * I.dt), &sn, &cs);
-        for (int t = threadIdx.x; t < 3 * A.n_cells; t += ADJ_THREADS) {
-            const int q = t / 3, c = t % 3;
-            if (!((A.comp_mask >> c) & 1)) continue;
-            const int* x = A.cells + 3 * q;
-            const double2 v = A.D[t];
-            A.eb[c][(long long)x[2] * I.plane + (long long)x[1] * I.px + x[0]] +=
-                (real)(2.0 * I.dt * (v.x * cs + v.y * sn));
-        }
+        const int* x = A.cells + 3 * q;
+        const double2 v = A.D[t];
+        A.eb[c][(long long)x[2] * I.plane + (long long)x[1] * I.px + x[0]] +=
+            (real)(2.0 * I.dt * (v.x * cs + v.y * sn));
         return;
     }
     Place<real, W> P;
@@ -529,7 +528,11 @@ cudaError_t launch_adjoint_step(const AdjDev<real>& a, long long n, cudaStream_t
     const int zs = adj_segment(blocks, I.nz);
     const unsigned segs = (unsigned)((I.nz + zs - 1) / zs);
     k_adj_e<real, W><<<dim3((unsigned)blocks, segs), ADJ_THREADS, 0, s>>>(a, n, zs);
-    k_adj_h<real, W><<<dim3((unsigned)blocks + 1, segs), ADJ_THREADS, 0, s>>>(a, n, zs);
+    // the objective's blocks: a patch of 25 cells fills two; a plane of 192^2 cells, in
+    // one block a loop longer than the step (40 steps of 192^3: 79.0 ms), 1728 (15.9)
+    const long long src = (3ll * a.n_cells + ADJ_THREADS - 1) / ADJ_THREADS;
+    const unsigned cols = (unsigned)blocks + (unsigned)((src + segs - 1) / segs);
+    k_adj_h<real, W><<<dim3(cols, segs), ADJ_THREADS, 0, s>>>(a, n, zs, (unsigned)blocks);
     return cudaGetLastError();
 }
 

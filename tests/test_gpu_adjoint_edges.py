@@ -105,3 +105,20 @@ def test_memory_refused_is_what_would_not_fit(lib):
         del hog
         torch.cuda.empty_cache()
     f.close()
+
+
+@pytest.mark.parametrize("cells,comps", [(21, (0, 1, 2)), (22, (0, 1, 2)), (627, (2,)), (33 * 19 * 17, (0, 2))])
+def test_objectives_of_many_cells(lib, oracle_lib, cells, comps):
+    """The objective's source over one block, a block and a remainder, more blocks than z segments, and every cell."""
+    inst, des, _ = case(*GRIDS["odd"], seed=7)
+    q = np.arange(cells)
+    obj = Objective(np.stack([q % 33, q // 33 % 19, (8 + q // 627) % 17], axis=1), frequency=1 / 0.7, comps=comps)
+    o = OracleFields(inst)
+    o.set_design(des)
+    F0, g0 = o.adjoint(obj, STEPS)
+    f = Fields(inst, "f64")
+    f.set_design(des)
+    F, g = f.adjoint_gradient(obj, STEPS, checkpoint_every=STEPS)
+    assert F[0] == pytest.approx(F0, rel=1e-10)
+    assert np.max(np.abs(g0)) > 0
+    assert np.max(np.abs(g[0] - g0)) <= 1e-8 * np.max(np.abs(g0))
