@@ -398,7 +398,7 @@ int sj_max_abs_e(sj_sim* sim, int32_t inst, double* out);
    runs of steps on small grids wait for one another at a grid barrier.  A
    wait that does not end within the limit gives up (a TMA block first waits,
    bounded by 100 ms, for the copies it still has in flight), the launch ends,
-   the runs queued behind it do nothing, and SJ_E_TIMEOUT is recorded:
+   so do the runs queued behind it, and SJ_E_TIMEOUT is recorded:
    sj_synchronize (and every call that synchronises) then returns it.  The
    fields of that step are not valid.  ns = 0 restores the defaults: 100 ms
    for a copy (a healthy one takes microseconds), 4 s at the grid barrier (a

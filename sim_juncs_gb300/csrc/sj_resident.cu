@@ -82,8 +82,11 @@ __device__ __forceinline__ Cell res_cell(const ResGrid& G, unsigned t) {
 
 // Grid barrier: every block arrives with release, waits for `target`
 // arrivals with acquire.  A wait that does not end within `limit` ns records
-// SJ_E_TIMEOUT and ends the launch (false, block-uniform); launches queued
-// behind it return at once (k_resident).
+// SJ_E_TIMEOUT and ends the launch (false, block-uniform): BAR_DEAD on the
+// counter lets every block's wait end, and those of the launches queued behind
+// (k_bar_reset), whose state is not to be stepped on.
+constexpr unsigned BAR_DEAD = 0x80000000u;
+__global__ void k_bar_reset(unsigned* bar, const DevState* st) { *bar = st->status == SJ_E_TIMEOUT ? BAR_DEAD : 0u; }
 __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, unsigned long long limit, DevState* st) {
     __shared__ int ok;
     __syncthreads();
@@ -94,13 +97,17 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, uns
         for (unsigned spin = 0;; ++spin) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-            if (v >= target) break;
+            if (v >= target) {
+                ok = v < BAR_DEAD;
+                break;
+            }
             if ((spin & 1023u) == 1023u) {
                 unsigned long long t;
                 asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
                 if (!t0) t0 = t;
                 if (t - t0 > limit) {
                     st->status = SJ_E_TIMEOUT;
+                    atomicOr(bar, BAR_DEAD);
                     ok = 0;
                     break;
                 }
@@ -554,14 +561,9 @@ k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __res
            unsigned* bar, unsigned long long limit, int stall, DevState* st) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ ResGrid grids[RES_MAX_INST];
-    __shared__ int gone;
     constexpr unsigned CH = res_chunk<real, T>(), SLOTS = T / CH;
     const long long n0 = st->step;
-    // a launch before this one gave up: its state is not to be stepped on.
-    // stall (sj_set_test_stall): the first block never arrives at a barrier.
-    if (threadIdx.x == 0) gone = st->status == SJ_E_TIMEOUT || (stall && blockIdx.x == 0);
-    __syncthreads();
-    if (gone) return;
+    if (stall && blockIdx.x == 0) return;  // sj_set_test_stall: never arrives at a barrier
     if ((int)blockIdx.x >= workers) {
         int b = (int)blockIdx.x - workers;
         if (b < probe_blocks) {
@@ -771,7 +773,8 @@ cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d
     int probe = plan.blocks;
     int w = (int)std::min<long long>((cells + T - 1) / T, max_blocks - probe - obj_blocks);
     if (w < 1) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(d_bar, 0, sizeof(unsigned), s);
+    k_bar_reset<<<1, 1, 0, s>>>(d_bar, st);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     InstDev<real> one = h_insts[0];
     int one_chunk = plan.chunks <= probe;
