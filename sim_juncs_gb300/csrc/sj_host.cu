@@ -1443,7 +1443,7 @@ template <typename real>
 void do_steps_graph(sj_sim* sim, long long n, int chunk) {
     if (chunk < 1) fail(SJ_E_INVALID, "chunk must be >= 1");
     if (sim->any_snapshots()) return do_steps<real>(sim, n);  // save points fall inside chunks
-    if (resident<real>(sim)) return do_steps<real>(sim, n);   // one launch per run of steps already
+    if (n >= 2 && resident<real>(sim)) return do_steps<real>(sim, n);  // one launch per run of steps already
     ensure_capacity<real>(sim, sim->t + n);
     // everything that allocates or copies happens before the capture
     prepare_schedule<real>(sim);

@@ -79,3 +79,26 @@ def test_warmed_up_sims_can_be_captured(lib, warm, captured):
     assert lit(a)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+def test_single_step_graphs_between_runs(lib, precision):
+    # single steps replay graphs of the tile launches, one per parity; runs step in place
+    insts = [junction_instance(n=n, res=r, phase=p) for n, r, p in ((40, 12.5, 0.3), (64, 20.0, 1.0), (40, 12.5, 2.0))]
+    for i in insts:
+        i.sources[0].start_time, i.sources[0].end_time = -9.0, 11.0
+    a, b = Fields(insts, precision), Fields(insts, precision)
+    b.set_tiling(8, 0, 8)
+    for _ in range(5):
+        a.step_graph(1, chunk=1)
+    a.step(7)
+    for _ in range(4):
+        a.step_graph(1, chunk=1)
+    a.step_graph(20, chunk=1)
+    a.step(1)
+    a.step_graph(1, chunk=1)
+    b.step(38)
+    equal_sims(a, b)
+    assert lit(a)
+    a.close()
+    b.close()
