@@ -151,18 +151,6 @@ def measured_peak():
         return 6800.0, "fallback"
 
 
-def run_launches(f, steps):
-    """Kernel launches of a run of `steps` steps.  Small grids (at most 32
-    instances, 2^22 cells together in FP32, 2^27 in FP64) run up to 256 steps
-    per launch in the fused schedule's default settings."""
-    from sim_juncs_gb300 import _abi
-    limit = 1 << (27 if f.precision == _abi.F64 else 22)
-    if (steps >= 2 and f.schedule_name() == "fused" and f.fused_launch() == "grouped"
-            and f.n_instances <= 32 and f.voxels() <= limit):
-        return -(-steps // 256)
-    return steps * f.launches_per_step()
-
-
 def time_steps(f, torch, steps, warmup, graph_chunk=0):
     """Device time of `steps` steps on f's stream (CUDA events), after warmup;
     graph_chunk > 0: the steps replay CUDA graphs of that many steps
@@ -181,7 +169,7 @@ def time_steps(f, torch, steps, warmup, graph_chunk=0):
     e1.record(stream)
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1)
-    return ms / 1000.0, run_launches(f, steps)
+    return ms / 1000.0, f.run_launches(steps)
 
 
 def tuned_fields(insts, schedule, torch):
@@ -229,6 +217,11 @@ def run_ours(args):
                    autotune_dry_ms_per_step=tune_ms)  # the tuner's launches load but do not store
         if schedule == "fused":
             cfg["launch_mode"] = f.fused_launch()  # grouped launches or one queued launch, as the tuner kept
+    # small grids (not the sweep): sj_step's runs are resident launches, and the tuned tiling only
+    # its single steps'; setting it would ask for the tile launches
+    resident = f.run_launches(256) < 256
+    if resident:
+        cfg["launch_mode"], til = "resident runs", None
     voxels = f.voxels()
     bytes_step = f.bytes_per_step()
 
@@ -248,7 +241,7 @@ def run_ours(args):
     value = job_value(voxels, args.steps, ws, secs)
     peak, peak_kind = measured_peak()
     achieved = bytes_step / (secs / args.steps) / 1e9
-    kernel = {"fused": "fused step: the tile launches of each instance group (one, or one per tile class) and one "
+    kernel = "k_resident: up to 256 steps per launch" if resident else {"fused": "fused step: the tile launches of each instance group (one, or one per tile class) and one "
                        "general launch, concurrent (one HBM pass)",
               "tma": "k_fused (TMA shared-memory tiles), one launch per step",
               "split": "k_split_h + k_split_e"}[schedule]
@@ -258,7 +251,8 @@ def run_ours(args):
         "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": dict(cfg, schedule=schedule, l2="state larger than L2 (no flush needed)",
                        voxels_per_step=voxels, parallelism=f"replicas{ws}",
-                       timed=f"CUDA graph replays of {max(chunk, 0)} step(s) (sj_step_graph)" if chunk > 0
+                       timed="resident runs (sj_step_graph)" if resident and chunk > 0
+                       else f"CUDA graph replays of {max(chunk, 0)} step(s) (sj_step_graph)" if chunk > 0
                        else "sj_step launches",
                        ms_per_step_plain_launches=secs_launch / args.steps * 1e3),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",

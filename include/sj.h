@@ -346,9 +346,12 @@ int sj_transfer_bytes(const sj_sim* sim, int64_t* h2d, int64_t* d2h);
 int64_t sj_voxels(const sj_sim* sim, int32_t inst);
 double sj_bytes_per_step(const sj_sim* sim, int32_t inst);
 /* kernel launches a single step issues under the current schedule (GB300
-   query; the reference has no counterpart; runs of steps on small grids issue
-   fewer) */
+   query; the reference has no counterpart) */
 int32_t sj_launches_per_step(const sj_sim* sim);
+/* kernel launches a call of sj_step(n_steps) issues as things stand: n_steps
+   single steps', or two per 256 steps where it runs small grids as resident
+   launches.  No snapshots counted in; -1 where sj_launches_per_step is. */
+int64_t sj_run_launches(const sj_sim* sim, int64_t n_steps);
 
 /* ---------------------------------------------------------------- read-back */
 /* field_times (src/disp.hpp:172): out[monitor][sample], monitor = order of

@@ -141,6 +141,7 @@ SIGNATURES = {
     "sj_voxels": (C.c_int64, [_P, C.c_int32]),
     "sj_bytes_per_step": (C.c_double, [_P, C.c_int32]),
     "sj_launches_per_step": (C.c_int32, [_P]),
+    "sj_run_launches": (C.c_int64, [_P, C.c_int64]),
     "sj_get_schedule": (C.c_int32, [_P]),
     "sj_set_design": (C.c_int, [_P, C.c_int32, C.POINTER(DesignDesc)]),
     "sj_adjoint_gradient": (C.c_int, [_P, C.POINTER(ObjectiveDesc), C.c_int64, C.c_int32, _D, C.c_size_t, _D]),

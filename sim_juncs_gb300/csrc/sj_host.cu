@@ -2347,6 +2347,18 @@ int32_t sj_launches_per_step(const sj_sim* sim) {
         maxp = std::max(maxp, sim->precision == SJ_F64 ? sim->h64[q].n_probe : sim->h32[q].n_probe);
     return maxp > 0 ? 3 : 2;  // probe, H pass, E pass
 }
+int64_t sj_run_launches(const sj_sim* sim, int64_t n) {
+    if (!sim || n < 0) return -1;
+    try {
+        sj_sim* ms = const_cast<sj_sim*>(sim);  // asks the device once what fits it
+        if (n >= 2 && (sim->precision == SJ_F64 ? resident<double>(ms) : resident<float>(ms)))
+            return 2 * ((n + RES_CHUNK - 1) / RES_CHUNK);
+    } catch (const Fail&) {
+        return -1;
+    }
+    const int32_t per = sj_launches_per_step(sim);
+    return per < 0 ? -1 : n * per;
+}
 int64_t sj_n_samples(const sj_sim* sim, int32_t inst) {
     if (!sim || inst < 0 || inst >= sim->n_inst) return -1;
     const int ss = sim->precision == SJ_F64 ? sim->hi64[inst].save_span : sim->hi32[inst].save_span;

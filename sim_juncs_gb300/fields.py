@@ -212,6 +212,11 @@ class Fields:
         """Kernel launches one step issues under the current schedule."""
         return int(self.lib.sj_launches_per_step(self.handle))
 
+    def run_launches(self, n):
+        """Kernel launches step(n) issues: n single steps', or a few where it
+        runs small grids as resident launches."""
+        return int(self.lib.sj_run_launches(self.handle, int(n)))
+
     def n_samples(self, inst=0):
         return self.lib.sj_n_samples(self.handle, inst)
 

@@ -102,3 +102,22 @@ def test_single_step_graphs_between_runs(lib, precision):
     assert lit(a)
     a.close()
     b.close()
+
+
+def test_launch_counts_follow_the_dispatch(lib):
+    inst = junction_instance(n=64, res=20.0)
+    f = Fields(inst, "f32")
+    one = f.launches_per_step()
+    assert f.run_launches(1) == one and f.run_launches(0) == 0
+    assert f.run_launches(2) == f.run_launches(256) == 2 and f.run_launches(257) == 4
+    f.set_tiling(*f.tiling())                       # asks for the tile launches
+    assert f.run_launches(256) == 256 * one
+    f.close()
+    big = Fields(junction_instance(n=192, res=60.0), "f32")
+    assert big.run_launches(10) == 10 * big.launches_per_step()
+    big.close()
+    inst.probes = [Probe(0, (1.6, 1.6, 1.6), dft=True)] * 60000
+    inst.freqs = list(np.linspace(1.0, 2.0, 50))    # the probes outweigh what a resident run gains
+    f = Fields(inst, "f32")
+    assert f.run_launches(10) == 10 * f.launches_per_step()
+    f.close()
