@@ -306,13 +306,16 @@ int sj_set_fused_columns(sj_sim* sim, int32_t columns);
    thread only (every instance's nx a multiple of 32), else the grouped
    launches run.  Both evaluate the same per-cell arithmetic: the results do
    not change.  sj_autotune tries both where QUEUE applies and keeps the
-   faster. */
+   faster.  Runs of steps on small grids (sj_step) are neither, in GROUPED
+   mode; set to QUEUE they are queued launches too. */
 enum { SJ_LAUNCH_GROUPED = 0, SJ_LAUNCH_QUEUE = 1 };
 int sj_set_fused_launch(sj_sim* sim, int32_t mode);
 /* the launch mode in use (SJ_LAUNCH_*), -1 for a null handle */
 int32_t sj_get_fused_launch(const sj_sim* sim);
 /* time every fused tiling with `steps` launches that leave the state
-   untouched, keep the fastest and report it (any output may be NULL) */
+   untouched, keep the fastest and report it (any output may be NULL).  Where
+   runs of steps are resident launches (sj_step, small grids), they stay so
+   and ms_per_step is theirs; the tiling is then that of single steps. */
 int sj_autotune(sj_sim* sim, int32_t steps, int32_t* tile_y, int32_t* ring, int32_t* zseg,
                 float* ms_per_step);
 

@@ -1208,6 +1208,13 @@ cudaError_t launch_one(sj_sim* sim) {
     return e;
 }
 
+template <typename real>
+void set_dev_step(sj_sim* sim, long long step, bool clear = false);
+template <typename real>
+bool resident(sj_sim* sim);
+template <typename real>
+float time_resident(sj_sim* sim, int steps, cudaEvent_t e0, cudaEvent_t e1);
+
 // Time `steps` dry launches (no state change) of every tiling candidate and
 // keep the fastest: the project's own autotuner for the fused schedule.
 // Lean-schedule autotuner: z-segment length by timing dry launches.
@@ -1216,8 +1223,17 @@ void autotune_lean(sj_sim* sim, int steps, int* best_zs, float* best_ms) {
     const int zbs[3] = {8, 16, 32};
     float best = 1e30f;
     int bzb = sim->l_zb;
-    // the queued launch is a candidate where it applies
-    const bool try_queue = queue_eligible<real>(sim);
+    // Grids whose runs of steps are resident launches stay with them: on all of
+    // those they are faster than either launch mode's real steps (us per step of 100,
+    // resident / queued / its graphs of 10: 64^3 9 / 45 / 42, 96^3 18 / 55 / 50, 128^3
+    // 44 / 87 / 84, 160^3 101 / 122 / 119; a dry launch's time says less, as it does
+    // not store).  The segment length is then tuned for the single steps.
+    const int asked = sim->l_launch;
+    sim->l_launch = SJ_LAUNCH_GROUPED;
+    const bool res = resident<real>(sim);
+    if (!res) sim->l_launch = asked;
+    // else the queued launch is a candidate where it applies
+    const bool try_queue = !res && queue_eligible<real>(sim);
     int blaunch = sim->l_launch;
     cudaEvent_t e0, e1;
     ck(cudaEventCreate(&e0), "event");
@@ -1253,6 +1269,8 @@ void autotune_lean(sj_sim* sim, int steps, int* best_zs, float* best_ms) {
             blaunch = sim->l_launch;
         }
     }
+    const float run = res ? time_resident<real>(sim, steps, e0, e1) : -1;
+    if (run >= 0) best = run;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     sim->l_zb = bzb;
@@ -1389,6 +1407,53 @@ void run_resident(sj_sim* sim, long long n, const ObjDev<real>* d_obj = nullptr,
                                  sim->r_blocks, d_obj, obj_blocks, sim->d_bar, sim->wait_ns ? sim->wait_ns : RES_WAIT_NS,
                                  sim->test_stall, sim->d_state, sim->stream),
            "resident launch");
+}
+
+// Time (ms, of `steps` steps) of a run of steps, the state as it was
+// afterwards: without probes, on the buffers that the next single step
+// overwrites, and with the in-place arrays put back; < 0: not timed.
+template <typename real>
+float time_resident(sj_sim* sim, int steps, cudaEvent_t e0, cudaEvent_t e1) {
+    const int n = std::min(std::max(steps, 16), RES_CHUNK);  // a launch's start and end over as many steps
+    ensure_capacity<real>(sim, sim->t + 2 * n);
+    std::vector<InstDev<real>> v = devv<real>(sim);
+    std::vector<std::pair<void*, size_t>> kept;
+    size_t total = 0;
+    for (InstDev<real>& I : v) {
+        for (int a = 0; a < 3; ++a)
+            if (I.psiE[a]) kept.push_back({I.psiE[a], 2 * (size_t)I.vol * sizeof(real)});
+        if (I.P) kept.push_back({I.P, (size_t)I.n_poles * 6 * I.dvol * sizeof(real)});
+        I.n_probe = I.n_hprobe = I.n_dft = 0;
+    }
+    for (const auto& k : kept) total += k.second;
+    char* copy = nullptr;
+    if (total && cudaMalloc((void**)&copy, total) != cudaSuccess) {
+        cudaGetLastError();
+        return -1;  // no room to time it in
+    }
+    size_t off = 0;
+    for (const auto& k : kept) {
+        ck(cudaMemcpyAsync(copy + off, k.first, k.second, cudaMemcpyDeviceToDevice, sim->stream), "autotune copy");
+        off += k.second;
+    }
+    const InstDev<real>* d = reinterpret_cast<const InstDev<real>*>(sim->d_table);
+    for (int pass = 0; pass < 2; ++pass) {  // the first to warm up
+        ck(cudaEventRecord(e0, sim->stream), "event");
+        ck(launch_resident<real>(v.data(), d, sim->n_inst, sim->cur ^ 1, n, sim->r_blocks, nullptr, 0, sim->d_bar,
+                                 sim->wait_ns ? sim->wait_ns : RES_WAIT_NS, sim->test_stall, sim->d_state, sim->stream),
+           "autotune");
+        ck(cudaEventRecord(e1, sim->stream), "event");
+    }
+    off = 0;
+    for (const auto& k : kept) {
+        ck(cudaMemcpyAsync(k.first, copy + off, k.second, cudaMemcpyDeviceToDevice, sim->stream), "autotune copy");
+        off += k.second;
+    }
+    set_dev_step<real>(sim, sim->t);  // waits for the stream
+    cudaFree(copy);
+    float ms = 0;
+    ck(cudaEventElapsedTime(&ms, e0, e1), "event");
+    return ms * steps / n;
 }
 
 // n steps with no save point inside: one cooperative launch per RES_CHUNK
@@ -1626,7 +1691,7 @@ void set_design_t(sj_sim* sim, int q, const sj_design_desc* d) {
 
 // The device's step counter; the status kernels have left stays unless `clear`.
 template <typename real>
-void set_dev_step(sj_sim* sim, long long step, bool clear = false) {
+void set_dev_step(sj_sim* sim, long long step, bool clear) {
     DevState st{};
     st.step = step;
     st.done = 0;

@@ -98,7 +98,8 @@ class Fields:
 
     def autotune(self, steps=3):
         """Pick the fused tiling by timing state-preserving launches.
-        Returns (tile_y, ring, zseg, ms_per_step)."""
+        Returns (tile_y, ring, zseg, ms_per_step); on small grids the time is
+        that of their resident runs, the tiling that of single steps."""
         a, b, c, ms = C.c_int32(), C.c_int32(), C.c_int32(), C.c_float()
         self._ck(self.lib.sj_autotune(self.handle, int(steps), C.byref(a), C.byref(b), C.byref(c),
                                       C.byref(ms)))

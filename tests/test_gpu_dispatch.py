@@ -121,3 +121,25 @@ def test_launch_counts_follow_the_dispatch(lib):
     f = Fields(inst, "f32")
     assert f.run_launches(10) == 10 * f.launches_per_step()
     f.close()
+
+
+@pytest.mark.parametrize("precision,mode", [("f32", "grouped"), ("f32", "queue"), ("f64", "grouped")])
+def test_autotune_keeps_resident_runs(lib, precision, mode):
+    # poles, psi and DFT sums are stepped in place: timing a run must leave them as they were
+    insts = [junction_instance(n=64, res=20.0, phase=p) for p in (0.4, 1.9)]
+    for i in insts:
+        i.sources[0].start_time, i.sources[0].end_time = -9.0, 11.0
+    a, b = Fields(insts, precision), Fields(insts, precision)
+    a.step(31)
+    b.step(31)
+    a.set_fused_launch(mode)
+    ms = a.autotune(2)[3]
+    assert ms > 0 and a.fused_launch() == "grouped" and a.run_launches(256) == 2
+    a.synchronize()
+    for n in (1, 40):
+        a.step(n)
+        b.step(n)
+    equal_sims(a, b)
+    assert lit(a)
+    a.close()
+    b.close()
