@@ -134,3 +134,26 @@ def test_probes_dealt_out_over_blocks(lib, precision, counts, freqs):
         assert not len(insts[q].probes) or np.max(np.abs(a.dft(q))) > 0
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+def test_every_column_in_a_slab(lib, precision):
+    """Grids of one plane and of a few whose every column lies in an x slab, the sheet inside them."""
+    insts = []
+    for nz in (1, 5):
+        inst = whole_slab()[0]
+        inst.grid = Grid(8, 20, nz, inst.grid.dx, inst.grid.dt)
+        src = inst.sources[0]
+        src.start_time, src.end_time = -9.0, 11.0
+        src.lo, src.hi = (0.0, 0.0, 0.0), (8 / 14.0, 20 / 14.0, 0.0)
+        insts.append(inst)
+    a, b = Fields(insts, precision), Fields(insts, precision)
+    b.set_tiling(8, 0, 8)
+    a.step(41)
+    b.step(41)
+    for q in (0, 1):
+        for c in range(6):
+            np.testing.assert_array_equal(a.get_array(c, q), b.get_array(c, q), err_msg=f"instance {q} component {c}")
+        assert all(np.max(np.abs(a.get_array(c, q))) > 0 for c in ((0, 5) if q == 0 else (0, 4, 5)))
+    a.close()
+    b.close()
