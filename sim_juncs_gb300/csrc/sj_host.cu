@@ -255,11 +255,22 @@ struct sj_sim {
         if (it != allocs.end()) allocs.erase(it);
         cudaFree(p);
     }
+    // Host arrays go up on the sim's stream: cudaMemcpy returns when a pageable
+    // array is staged, and its stream is not one that the sim's waits for, so a
+    // kernel launched next could read what was there before.
+    void put(void* dst, const void* src, size_t bytes, const char* what) {
+        ck(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream), what);
+        ck(cudaStreamSynchronize(stream), what);
+    }
+    void put_rows(void* dst, size_t dpitch, const void* src, size_t width, size_t rows, const char* what) {
+        ck(cudaMemcpy2DAsync(dst, dpitch, src, width, width, rows, cudaMemcpyHostToDevice, stream), what);
+        ck(cudaStreamSynchronize(stream), what);
+    }
     template <typename T>
     T* upload(const std::vector<T>& v) {
         if (v.empty()) return nullptr;
         T* p = (T*)dalloc(v.size() * sizeof(T), false);
-        ck(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "upload");
+        put(p, v.data(), v.size() * sizeof(T), "upload");
         h2d += (long long)(v.size() * sizeof(T));
         return p;
     }
@@ -517,9 +528,8 @@ void build_instance(sj_sim* sim, const sj_instance_desc& d, HostInst<real>& H, I
         poles.assign(m.poles, m.poles + m.n_poles);
         sigma.assign(m.sigma, m.sigma + (size_t)n_classes * m.n_poles);
         for (int c = 0; c < 3; ++c)
-            ck(cudaMemcpy2D(d_cls + c * cpitch, px, m.class_map + (size_t)c * nx * ny * nz, nx, nx,
-                            (size_t)ny * nz, cudaMemcpyHostToDevice),
-               "class map upload");
+            sim->put_rows(d_cls + c * cpitch, px, m.class_map + (size_t)c * nx * ny * nz, nx, (size_t)ny * nz,
+                          "class map upload");
         sim->h2d += 3ll * nx * ny * nz;
     } else {
         check_scene(m.scene);
@@ -834,7 +844,7 @@ void upload_table(sj_sim* sim) {
     for (int q = 0; q < n; ++q) pre[q + 1] = pre[q] + split_blocks(dv[q]);
     if (!sim->d_table) sim->d_table = sim->dalloc(buf.size(), false);
     ck(cudaStreamSynchronize(sim->stream), "sync before table upload");
-    ck(cudaMemcpy(sim->d_table, buf.data(), buf.size(), cudaMemcpyHostToDevice), "table upload");
+    sim->put(sim->d_table, buf.data(), buf.size(), "table upload");
     sim->h2d += (long long)buf.size();
     // by parity: entry cur * n + q has slot 0 = buffer cur (fields, H-side psi)
     std::vector<InstDev<real>> par(2 * (size_t)n);
@@ -846,8 +856,7 @@ void upload_table(sj_sim* sim) {
         for (int a = 0; a < 3; ++a) std::swap(t.psiH[0][a], t.psiH[1][a]);
     }
     if (!sim->d_parity) sim->d_parity = sim->dalloc(par.size() * sizeof(InstDev<real>), false);
-    ck(cudaMemcpy(sim->d_parity, par.data(), par.size() * sizeof(InstDev<real>), cudaMemcpyHostToDevice),
-       "parity table upload");
+    sim->put(sim->d_parity, par.data(), par.size() * sizeof(InstDev<real>), "parity table upload");
     sim->h2d += (long long)(par.size() * sizeof(InstDev<real>));
     sim->table_version += 1;
 }
@@ -885,11 +894,11 @@ void ensure_capacity(sj_sim* sim, long long t_end) {
             if (H.mon_cap < need) {
                 const long long cap = std::max(need, 2 * H.mon_cap);
                 double* nb = (double*)sim->dalloc((size_t)cap * H.n_mon * sizeof(double));
-                ck(cudaStreamSynchronize(sim->stream), "sync");
                 if (H.d_mon)
-                    ck(cudaMemcpy(nb, H.d_mon, (size_t)H.mon_cap * H.n_mon * sizeof(double),
-                                  cudaMemcpyDeviceToDevice),
+                    ck(cudaMemcpyAsync(nb, H.d_mon, (size_t)H.mon_cap * H.n_mon * sizeof(double),
+                                       cudaMemcpyDeviceToDevice, sim->stream),
                        "mon grow");
+                ck(cudaStreamSynchronize(sim->stream), "sync");
                 sim->dfree(H.d_mon);
                 H.d_mon = nb;
                 H.mon_cap = cap;
@@ -1594,7 +1603,7 @@ void set_guard_t(sj_sim* sim, double bound) {
     ck(cudaStreamSynchronize(sim->stream), "sync");
     sim->guard_bound = bound;
     for (auto& I : devv<real>(sim)) I.guard_bound = bound;
-    ck(cudaMemset(sim->d_guard_flag, 0, sizeof(int)), "guard reset");
+    ck(cudaMemsetAsync(sim->d_guard_flag, 0, sizeof(int), sim->stream), "guard reset");
     memset(sim->h_guard, 0, sizeof(GuardRecord));
     sim->drop_graphs();
     upload_table<real>(sim);
@@ -1637,9 +1646,8 @@ void write_field_t(sj_sim* sim, int inst, int comp, const double* in) {
     std::vector<real> tmp((size_t)H.nx * H.ny * H.nz);
     for (size_t q = 0; q < tmp.size(); ++q) tmp[q] = (real)in[q];
     ck(cudaStreamSynchronize(sim->stream), "sync");
-    ck(cudaMemcpy2D(I.F[sim->cur][comp], H.px * sizeof(real), tmp.data(), H.nx * sizeof(real),
-                    H.nx * sizeof(real), (size_t)H.ny * H.nz, cudaMemcpyHostToDevice),
-       "field write");
+    sim->put_rows(I.F[sim->cur][comp], H.px * sizeof(real), tmp.data(), H.nx * sizeof(real), (size_t)H.ny * H.nz,
+                  "field write");
 }
 
 // ------------------------------------------------------------------ adjoint
@@ -1931,8 +1939,7 @@ void adjoint_t(sj_sim* sim, const sj_objective_desc* objs, long long N, long lon
         set_dev_step<real>(sim, N);
         for (int q = 0; q < ni; ++q)
             if (dv[q].dft)
-                ck(cudaMemcpy(dv[q].dft, dft_keep[q].data(), dft_keep[q].size() * sizeof(double2), cudaMemcpyHostToDevice),
-                   "dft");
+                sim->put(dv[q].dft, dft_keep[q].data(), dft_keep[q].size() * sizeof(double2), "dft");
     }
     kernel_status(sim);
     // ---- dF/d(eps) = -eps^{-2} sum_c dF/d(inverse eps at the voxel's E_c point)

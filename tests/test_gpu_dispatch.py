@@ -143,3 +143,30 @@ def test_autotune_keeps_resident_runs(lib, precision, mode):
     assert lit(a)
     a.close()
     b.close()
+
+
+def test_threads_step_their_own_sims(lib):
+    # tables and buffers that grow while other threads copy and step: each sim's kernels see its own
+    from concurrent.futures import ThreadPoolExecutor
+    jobs = [(junction_instance(n=n, res=r, phase=0.3 * q), p, tiles)
+            for q, (n, r, p, tiles) in enumerate([(36, 11.25, "f32", False), (64, 20.0, "f64", False), (48, 15.0, "f32", True),
+                                                  (64, 20.0, "f64", False), (36, 11.25, "f64", True), (64, 20.0, "f32", False)])]
+
+    def run(job):
+        inst, precision, tiles = job
+        f = Fields(inst, precision)
+        if tiles:
+            f.set_tiling(8, 0, 8)
+        for n in (1, 2, 5, 12, 30, 70, 160, 300):
+            f.step(n)
+        out = [f.get_array(c) for c in range(6)] + [f.monitors(), f.dft()]
+        f.close()
+        return out
+
+    want = [run(j) for j in jobs]
+    assert all(max(np.max(np.abs(a)) for a in w[:6]) > 0 for w in want)
+    for _ in range(5):
+        with ThreadPoolExecutor(len(jobs)) as ex:
+            for w, g in zip(want, ex.map(run, jobs)):
+                for x, y in zip(w, g):
+                    np.testing.assert_array_equal(x, y)
