@@ -352,7 +352,7 @@ double sj_bytes_per_step(const sj_sim* sim, int32_t inst);
    query; the reference has no counterpart) */
 int32_t sj_launches_per_step(const sj_sim* sim);
 /* kernel launches a call of sj_step(n_steps) issues as things stand: n_steps
-   single steps', or two per 256 steps where it runs small grids as resident
+   single steps', or one per 256 steps where it runs small grids as resident
    launches.  No snapshots counted in; -1 where sj_launches_per_step is. */
 int64_t sj_run_launches(const sj_sim* sim, int64_t n_steps);
 

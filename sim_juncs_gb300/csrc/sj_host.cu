@@ -2424,7 +2424,7 @@ int64_t sj_run_launches(const sj_sim* sim, int64_t n) {
     try {
         sj_sim* ms = const_cast<sj_sim*>(sim);  // asks the device once what fits it
         if (n >= 2 && (sim->precision == SJ_F64 ? resident<double>(ms) : resident<float>(ms)))
-            return 2 * ((n + RES_CHUNK - 1) / RES_CHUNK);
+            return (n + RES_CHUNK - 1) / RES_CHUNK;
     } catch (const Fail&) {
         return -1;
     }
