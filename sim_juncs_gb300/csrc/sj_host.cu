@@ -843,8 +843,7 @@ void upload_table(sj_sim* sim) {
     pre[0] = 0;
     for (int q = 0; q < n; ++q) pre[q + 1] = pre[q] + split_blocks(dv[q]);
     if (!sim->d_table) sim->d_table = sim->dalloc(buf.size(), false);
-    ck(cudaStreamSynchronize(sim->stream), "sync before table upload");
-    sim->put(sim->d_table, buf.data(), buf.size(), "table upload");
+    ck(cudaMemcpyAsync(sim->d_table, buf.data(), buf.size(), cudaMemcpyHostToDevice, sim->stream), "table upload");
     sim->h2d += (long long)buf.size();
     // by parity: entry cur * n + q has slot 0 = buffer cur (fields, H-side psi)
     std::vector<InstDev<real>> par(2 * (size_t)n);
@@ -1489,7 +1488,6 @@ void prepare_steps(sj_sim* sim) {
         for (const InstDev<real>& I : devv<real>(sim)) codes = codes && lean_codes(I.nx, I.ny, I.nz, sim->l_zb);
     if (resident<real>(sim) && !codes) return;  // runs of steps need no tiles
     prepare_schedule<real>(sim);
-    if (sim->schedule == SJ_SCHED_FUSED) lean_streams(sim);
 }
 
 template <typename real>
