@@ -462,6 +462,8 @@ k_phases(const double* __restrict__ vin, long long s_series, long long s_sample,
             }
         C.t0_ind = tm <= 0.0 ? 0 : (int)(at / tm);
         C.status = 0;
+        C.f0 = 0.0;
+        C.f0_ind = 0;
         C.low_stren = 0.0;
         C.last_cent = 0.0;
         C.lowpass_steps = 0;

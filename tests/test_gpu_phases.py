@@ -137,3 +137,11 @@ def test_series_are_read_to_their_end_only(lib):
         assert extract_phases(t, end) == want
     finally:
         assert libc.mprotect(base + size, page, mmap.PROT_READ | mmap.PROT_WRITE) == 0
+
+
+def test_series_without_a_frequency_report_none(lib):
+    # a block that ran before must not leave its frequency in the result
+    t, v = pulses(120, 400)
+    assert all(r["status"] == _abi.PHASE_OK for r in extract_phases(t, v))
+    for r in extract_phases(t, np.zeros((400, 120))):
+        assert r["status"] == _abi.PHASE_BAD_F0 and r["f0"] == 0.0 and r["f0_ind"] == 0
