@@ -404,15 +404,15 @@ int sj_max_abs_e(sj_sim* sim, int32_t inst, double* out);
    runs of steps on small grids wait for one another at a grid barrier.  A
    wait that does not end within the limit gives up (a TMA block first waits,
    bounded by 100 ms, for the copies it still has in flight), the launch ends,
-   so do the runs queued behind it, and SJ_E_TIMEOUT is recorded:
+   the runs queued behind it do not wait, and SJ_E_TIMEOUT is recorded:
    sj_synchronize (and every call that synchronises) then returns it.  The
    fields of that step are not valid.  ns = 0 restores the defaults: 100 ms
    for a copy (a healthy one takes microseconds), 4 s at the grid barrier (a
    healthy wait is shorter than a step); at most 10 s. */
 int sj_set_wait_limit(sj_sim* sim, int64_t ns);
 /* Test hook for the bounded waits: while on, the first tile block of every
-   TMA-schedule launch never fetches its second plane, and the first block of
-   a run of steps on a small grid never arrives at the grid barrier, so the
+   TMA-schedule launch never fetches its second plane, and a block more in a
+   run of steps on a small grid never arrives at the grid barrier, so the
    wait on it runs out after the limit and the launch records SJ_E_TIMEOUT.
    Nothing else is affected.  Off by default; for tests of a host's error
    handling only. */

@@ -109,7 +109,7 @@ struct InstDev {
 struct DevState {
     long long step;     // absolute step index n of the next step
     unsigned int done;  // blocks finished in the current launch
-    int cur;            // ping-pong buffer holding E^n, H^{n-1/2}
+    int cur;            // ping-pong buffer holding E^n, H^{n-1/2}: 0 or 1
     int status;         // sticky error code set by kernels (0 = fine)
     int _pad;
 };
@@ -291,7 +291,7 @@ cudaError_t launch_objective(const ObjDev<real>* o, int n_inst, int cur, long lo
 // the blocks of the kernel that fit the device at once (0: it cannot run).
 // resident_pays: false where the probes outweigh what the steps gain.
 // d_obj (or null): objectives whose DFT sums the launch keeps, obj_blocks =
-// resident_objective_blocks of them.  d_bar: the barrier's counter, zeroed by
+// resident_objective_blocks of them.  d_bar: the barrier's counter, set by
 // the launch.  limit_ns: of a wait at the barrier; stall: sj_set_test_stall.
 constexpr int RES_MAX_INST = 32;  // instances of one resident launch
 template <typename real>

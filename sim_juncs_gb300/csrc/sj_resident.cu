@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstddef>
 
 #include "sj_physics.cuh"
 
@@ -82,11 +83,7 @@ __device__ __forceinline__ Cell res_cell(const ResGrid& G, unsigned t) {
 
 // Grid barrier: every block arrives with release, waits for `target`
 // arrivals with acquire.  A wait that does not end within `limit` ns records
-// SJ_E_TIMEOUT and ends the launch (false, block-uniform), other blocks' waits
-// with it.  A launch queued behind ends at its first barrier, its state not
-// being one to step on.  (The step loop's time moves by up to 2% with the form
-// of this code, registers and spills the same; this one is within 1% of a
-// barrier without the status, 36^3 to 128^3 and both precisions.)
+// SJ_E_TIMEOUT and ends the launch (false, block-uniform).
 __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, unsigned long long limit, DevState* st) {
     __shared__ int ok;
     __syncthreads();
@@ -97,15 +94,12 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, uns
         for (unsigned spin = 0;; ++spin) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-            if (v >= target) {
-                if (target == gridDim.x) ok = *(volatile int*)&st->status != SJ_E_TIMEOUT;
-                break;
-            }
+            if (v >= target) break;
             if ((spin & 1023u) == 1023u) {
                 unsigned long long t;
                 asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
                 if (!t0) t0 = t;
-                if (t - t0 > (*(volatile int*)&st->status == SJ_E_TIMEOUT ? 0 : limit)) {
+                if (t - t0 > limit) {
                     st->status = SJ_E_TIMEOUT;
                     ok = 0;
                     break;
@@ -562,8 +556,8 @@ k_resident(const __grid_constant__ InstDev<real> one, const InstDev<real>* __res
     __shared__ ResGrid grids[RES_MAX_INST];
     constexpr unsigned CH = res_chunk<real, T>(), SLOTS = T / CH;
     const long long n0 = st->step;
-    if (stall && blockIdx.x == 0) return;  // sj_set_test_stall: never arrives at a barrier
     if ((int)blockIdx.x >= workers) {
+        if (stall && blockIdx.x == gridDim.x - 1) return;  // sj_set_test_stall: never arrives at a barrier
         int b = (int)blockIdx.x - workers;
         if (b < probe_blocks) {
             res_probe_block<real>(tab, n_inst, cur, n0, n_steps, b, probe_blocks, per, h_probes, one_chunk, bar, limit,
@@ -770,16 +764,24 @@ cudaError_t launch_resident(const InstDev<real>* h_insts, const InstDev<real>* d
     }
     ProbePlan plan = probe_plan(h_insts, n_inst, max_blocks);
     int probe = plan.blocks;
-    int w = (int)std::min<long long>((cells + T - 1) / T, max_blocks - probe - obj_blocks);
+    stall = stall ? 1 : 0;  // one block more
+    int w = (int)std::min<long long>((cells + T - 1) / T, max_blocks - probe - obj_blocks - stall);
     if (w < 1) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(d_bar, 0, sizeof(unsigned), s);
+    // The barrier's counter starts at 0.  After a time-out it starts above any target:
+    // the status's low byte over three zero bytes (cur is 0 or 1), so that launches
+    // queued behind, which have no state to step on, do not wait either.  (1.2 us more
+    // than a memset per launch; the status read in the kernel instead moved the step
+    // loop's time by 1-2%, registers and spills the same.)
+    static_assert(offsetof(DevState, status) == offsetof(DevState, cur) + sizeof(int) && SJ_E_TIMEOUT < 0, "layout");
+    cudaError_t e = cudaMemcpyAsync(d_bar, reinterpret_cast<const char*>(st) + offsetof(DevState, status) - 3,
+                                    sizeof(unsigned), cudaMemcpyDeviceToDevice, s);
     if (e != cudaSuccess) return e;
     InstDev<real> one = h_insts[0];
     int one_chunk = plan.chunks <= probe;
     void* args[] = {&one,      &d_insts,   &n_inst, &cur,   &n_steps,  &w,     &probe, &plan.per,
                     &h_probes, &one_chunk, &d_obj,  &d_bar, &limit_ns, &stall, &st};
     const size_t smem = n_inst > 1 ? (size_t)n_inst * sizeof(InstDev<real>) : 0;
-    return cudaLaunchCooperativeKernel(res_kernel<real>(few, n_inst, des), dim3(w + probe + obj_blocks), dim3(T), args,
+    return cudaLaunchCooperativeKernel(res_kernel<real>(few, n_inst, des), dim3(w + probe + obj_blocks + stall), dim3(T), args,
                                        smem, s);
 }
 

@@ -322,7 +322,7 @@ class Fields:
 
     def set_test_stall(self, on):
         """Test hook: the TMA schedule's first tile block skips a plane's copy,
-        and a resident run's first block never arrives at the grid barrier, so
+        and a block more in a resident run never arrives at its grid barrier, so
         the wait runs out and SJ_E_TIMEOUT is reported."""
         self._ck(self.lib.sj_set_test_stall(self.handle, 1 if on else 0))
 
