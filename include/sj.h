@@ -302,10 +302,10 @@ int sj_set_fused_columns(sj_sim* sim, int32_t columns);
    one per group (FP32, mostly CPML tiles),
    the launches of a step concurrent on forked streams.  QUEUE: one launch of
    resident blocks for every group's tiles, which claim (group, member, tile)
-   items from a counter, multi-slab tiles first; FP32 with two columns per
-   thread only (every instance's nx a multiple of 32), else the grouped
-   launches run.  Both evaluate the same per-cell arithmetic: the results do
-   not change.  sj_autotune tries both where QUEUE applies and keeps the
+   items from a counter, multi-slab tiles first (groups that GROUPED launches
+   as one: in the order of the grid); FP32 with two columns per thread only
+   (every instance's nx a multiple of 32), else the grouped launches run.
+   Both evaluate the same per-cell arithmetic: the results do not change.  sj_autotune tries both where QUEUE applies and keeps the
    faster.  Runs of steps on small grids (sj_step) are neither, in GROUPED
    mode; set to QUEUE they are queued launches too. */
 enum { SJ_LAUNCH_GROUPED = 0, SJ_LAUNCH_QUEUE = 1 };
@@ -323,14 +323,15 @@ int sj_autotune(sj_sim* sim, int32_t steps, int32_t* tile_y, int32_t* ring, int3
 /* n_steps iterations of the loop body at src/disp.cpp:719-741: sample
    monitors when step % save_span == 0, accumulate DFTs, then fields.step().
    Asynchronous on the sim's stream.  FUSED with its default launch settings:
-   on small grids (all instances together at most 2^22 cells in FP32, 2^27 in
-   FP64) a call of two or more steps is one cooperative launch per 256 steps,
-   with the tile launches' bits; sj_adjoint_gradient and sj_objective run
-   forward the same way. */
+   on small grids (at most 32 instances, all together at most 2^22 cells in
+   FP32, 2^27 in FP64) a call of two or more steps is one cooperative launch
+   per 256 steps, with the tile launches' bits, unless the probes (their
+   number times their DFT frequencies) outweigh what that gains;
+   sj_adjoint_gradient and sj_objective run forward the same way. */
 int sj_step(sj_sim* sim, int64_t n_steps);
 
 /* same, recorded once into a CUDA graph of `chunk` steps and replayed (small
-   grids: as sj_step) */
+   grids: two or more steps as sj_step) */
 int sj_step_graph(sj_sim* sim, int64_t n_steps, int32_t chunk);
 
 /* ---------------------------------------------------------------- queries */

@@ -214,7 +214,7 @@ struct LeanStreams {
 // Queued launch of the fused schedule (FP32, every instance with whole
 // 32-column rows): the plain, slab and multi-slab tiles of every group in one
 // launch of resident blocks that claim tiles from a counter, multi-slab tiles
-// first, then single-slab, then plain.
+// (of merged groups, every tile) first, then single-slab, then plain.
 constexpr int LEAN_QUEUE_GROUPS = 16;  // most launch groups one queued launch takes
 template <typename real>
 struct LeanQueueParams {          // kernel parameter: every group's descriptor

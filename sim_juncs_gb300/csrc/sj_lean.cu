@@ -29,15 +29,16 @@
 //           k_lean_all2 takes every class in one launch (lean_classify).
 //           Compiled per axis set, so the other axes' terms vanish.
 //   general (k_lean_general): an H source in the footprint; also runs the
-//           probe blocks, and its blocks (the only ones that read the step
-//           counter) count themselves: the last advances the step.
+//           probe blocks.  Its blocks and the corrections' (the only ones
+//           that read the step counter) count themselves: the last advances
+//           the step.
 // Instances with the same grid, CPML and coefficient table form a group
 // (LeanGroup) whose arrays sit at fixed strides: one launch per class, or one
 // merged, covers the group's tiles (blockIdx.y = member).  The launches of a step go to
 // streams forked from the caller's, one per class and group set, so they
-// overlap; after they join, small correction kernels add the E sources and
-// the polarisation ADE on their cells only.  All evaluate one update
-// formula, so a voxel's result does not depend on which kernel (or which
+// overlap; small correction kernels then add the E sources and the
+// polarisation ADE on their cells only, a merged group's behind its tiles,
+// the others' after the join.  All evaluate one update formula, so a voxel's result does not depend on which kernel (or which
 // tiling) updated it:
 //   H^{n+1/2} = fma(-S, curl E, H^{n-1/2}) [- dt J_H]
 //   E^{n+1}   = fma(S ε∞⁻¹, curl H, E^n)
@@ -1337,8 +1338,9 @@ k_lean_plain2(const __grid_constant__ LeanTable<real> tab) {
 }
 
 // Queued tiles (LeanQueue): resident blocks claim (group, member, tile)
-// items from a counter, multi-slab tiles first; every group's descriptor
-// travels in the parameter space (as the grouped launches' one does), and the
+// items from a counter, multi-slab tiles first (of merged groups, all tiles in
+// the order of the grid: 96-member sweep 5.92 ms per step, 5.07 as grouped
+// launches); every group's descriptor travels in the parameter space (as the grouped launches' one does), and the
 // tile runs the two-column body of its slab mask.  One register budget covers
 // every mask.
 #ifndef SJ_LEAN_QUEUE_MINB
