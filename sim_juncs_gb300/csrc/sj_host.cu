@@ -1474,8 +1474,8 @@ float time_resident(sj_sim* sim, int steps, cudaEvent_t e0, cudaEvent_t e1) {
 
 // n steps with no save point inside: one cooperative launch per RES_CHUNK
 // steps on small grids, else a step's launches n times.  A single step keeps the
-// tile launches: 39 us a call at 64^3 FP32, 35 replayed, where a resident run of
-// two takes 26; runs are what was measured and moved.
+// tile launches (64^3 FP32: 39 us a call, 35 replayed; a resident run of two
+// takes 26, one of one step has not been tried).
 template <typename real>
 void run_steps(sj_sim* sim, long long n) {
     if (n >= 2 && resident<real>(sim)) {
@@ -1503,7 +1503,7 @@ void prepare_steps(sj_sim* sim) {
 template <typename real>
 void do_steps(sj_sim* sim, long long n) {
     ensure_capacity<real>(sim, sim->t + n);
-    prepare_steps<real>(sim);
+    if (n > 0) prepare_steps<real>(sim);
     while (n > 0) {
         // up to the next save point, the counter current there
         long long m = n;
@@ -2433,7 +2433,7 @@ int64_t sj_run_launches(const sj_sim* sim, int64_t n) {
         sj_sim* ms = const_cast<sj_sim*>(sim);  // asks the device once what fits it
         if (n >= 2 && (sim->precision == SJ_F64 ? resident<double>(ms) : resident<float>(ms)))
             return (n + RES_CHUNK - 1) / RES_CHUNK;
-    } catch (const Fail&) {
+    } catch (...) {
         return -1;
     }
     const int32_t per = sj_launches_per_step(sim);

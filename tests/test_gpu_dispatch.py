@@ -54,6 +54,22 @@ def test_long_thin_grids_take_single_steps(lib, nz):
     b.close()
 
 
+def test_no_steps_ask_for_nothing(lib):
+    # more planes than any tile code names: runs need no tiles, single steps are refused, no steps are nothing
+    f = Fields(column(16385), "f64")
+    f.set_tiling(8, 0, 16)
+    f.step(0)
+    with pytest.raises(_abi.SJError) as e:
+        f.step(1)
+    assert e.value.code == _abi.SJ_E_INVALID and f.steps_done == 0
+    f.close()
+    f = Fields(column(16385), "f64")   # (in FP32 it has more cells than resident runs take)
+    f.step(0)
+    f.step(3)
+    assert f.steps_done == 3 and lit(f)
+    f.close()
+
+
 @pytest.mark.parametrize("warm", [(1,) * 40, (30, 10)], ids=["single", "runs"])
 @pytest.mark.parametrize("captured", [(1, 1), (6,)], ids=["single", "run"])
 def test_warmed_up_sims_can_be_captured(lib, warm, captured):
